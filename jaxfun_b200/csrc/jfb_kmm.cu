@@ -143,60 +143,95 @@ __global__ void pack_factor_inv_kernel(const double* __restrict__ band, int n_mo
   }
 }
 
-// Reference layout (n, Ny, Nz) complex -> half layout [i][ky][kz < Kz],
-// zeroing the y Nyquist row.
-__global__ void to_half_kernel(const c64* __restrict__ full, int n, int Ny, int Nz,
-                               c64* __restrict__ half) {
-  const int Kz = Nz / 2;
-  const int64_t total = (int64_t)n * Ny * Kz;
-  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    const int kz = (int)(idx % Kz);
-    const int ky = (int)((idx / Kz) % Ny);
-    const int i = (int)(idx / ((int64_t)Kz * Ny));
-    half[idx] = (ky == Ny / 2) ? cmk(0.0, 0.0) : full[((size_t)i * Ny + ky) * Nz + kz];
-  }
-}
+// Conversions between the reference layout (n, Ny, Nz) complex and the half
+// layout [i][ky][kz < Kz], all arrays of a state in ONE launch (blockIdx.y =
+// array).  Bound by memory: at 65x64x64 a state is 12 arrays, 49 MB full, L2
+// resident between calls.  One launch per array left every launch too short
+// to fill the chip (12 x 3.4 us in, 12 x 4.1 us out, 1.9 and 2.1 us each on a
+// 17x16x16 grid); one launch takes 9.3 us in and 12.0 us out at 65x64x64,
+// 2.3 and 2.6 us at 17x16x16.  Four elements per thread, their loads first.
+constexpr int kMaxLayoutJobs = 28;  // 12 flow arrays + 15 of A
+constexpr int kLayoutPer = 4;       // elements per thread, all loads before the stores
+struct LayoutJob {
+  const c64* src;  // null (to half): zero fill
+  c64* dst;
+  int n;
+};
+// vw[i] = (a[i stride], b[i stride]) or back; null pointers read as zero / are skipped
+struct PairJob {
+  double *a, *b;
+  int64_t stride;
+  c64* vw;
+};
+struct LayoutJobs {
+  LayoutJob job[kMaxLayoutJobs];
+  PairJob pair[5];
+  int nj, np, Ny, Nz, nD;
+  int conj;  // to full: conjugate the values
+};
 
-// Half layout -> full reference layout using c(-ky, -kz) = conj(c(ky, kz));
-// the kz = Nz/2 column is zero.
-__global__ void to_full_kernel(const c64* __restrict__ half, int n, int Ny, int Nz,
-                               c64* __restrict__ full) {
-  const int Kz = Nz / 2;
-  const int64_t total = (int64_t)n * Ny * Nz;
-  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    const int kz = (int)(idx % Nz);
-    const int ky = (int)((idx / Nz) % Ny);
-    const int i = (int)(idx / ((int64_t)Nz * Ny));
-    c64 v = cmk(0.0, 0.0);
-    if (kz < Kz) {
-      v = half[((size_t)i * Ny + ky) * Kz + kz];
-    } else if (kz > Kz) {
-      const int my = (Ny - ky) % Ny;
-      v = conjc(half[((size_t)i * Ny + my) * Kz + (Nz - kz)]);
+// Full -> half: the kz < Kz columns, the y Nyquist row zeroed.
+__global__ void __launch_bounds__(256) to_half_kernel(const __grid_constant__ LayoutJobs J) {
+  if ((int)blockIdx.y == J.nj) {
+    for (int k = blockIdx.x; k < J.np; k += gridDim.x) {
+      const PairJob& q = J.pair[k];
+      for (int i = threadIdx.x; i < J.nD; i += blockDim.x)
+        q.vw[i] = cmk(q.a ? q.a[i * q.stride] : 0.0, q.b ? q.b[i * q.stride] : 0.0);
     }
-    full[idx] = v;
+    return;
   }
+  const LayoutJob& j = J.job[blockIdx.y];
+  const unsigned Kz = J.Nz / 2, Ny = J.Ny, total = (unsigned)j.n * Ny * Kz;
+  const unsigned base = blockIdx.x * (256u * kLayoutPer) + threadIdx.x;
+  if (base >= total) return;
+  c64 v[kLayoutPer];
+#pragma unroll
+  for (int t = 0; t < kLayoutPer; ++t) {
+    const unsigned idx = base + 256u * t, r = idx / Kz, kz = idx - r * Kz;
+    v[t] = (j.src && idx < total && r % Ny != Ny / 2) ? j.src[(size_t)r * J.Nz + kz] : cmk(0.0, 0.0);
+  }
+#pragma unroll
+  for (int t = 0; t < kLayoutPer; ++t)
+    if (base + 256u * t < total) j.dst[base + 256u * t] = v[t];
 }
 
-// Pack / unpack the two real mean-flow vectors into one complex vector.
-__global__ void means_in_kernel(const c64* __restrict__ u1, const c64* __restrict__ u2,
-                                int n, int Ny, int Nz, c64* __restrict__ vw) {
-  for (int i = threadIdx.x; i < n; i += blockDim.x)
-    vw[i] = cmk(u1[(size_t)i * Ny * Nz].re, u2[(size_t)i * Ny * Nz].re);
-}
-__global__ void real_pair_in_kernel(const double* __restrict__ a,
-                                    const double* __restrict__ b, int n,
-                                    c64* __restrict__ vw) {
-  for (int i = threadIdx.x; i < n; i += blockDim.x)
-    vw[i] = cmk(a ? a[i] : 0.0, b ? b[i] : 0.0);
-}
-__global__ void real_pair_out_kernel(const c64* __restrict__ vw, int n, double* a,
-                                     double* b) {
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    if (a) a[i] = vw[i].re;
-    if (b) b[i] = vw[i].im;
+// Half -> full using c(-ky, -kz) = conj(c(ky, kz)); the kz = Nz/2 column is
+// zero.  Every half value is read once and written to its two places.
+__global__ void __launch_bounds__(256) to_full_kernel(const __grid_constant__ LayoutJobs J) {
+  if ((int)blockIdx.y == J.nj) {
+    for (int k = blockIdx.x; k < J.np; k += gridDim.x) {
+      const PairJob& q = J.pair[k];
+      for (int i = threadIdx.x; i < J.nD; i += blockDim.x) {
+        if (q.a) q.a[i * q.stride] = q.vw[i].re;
+        if (q.b) q.b[i * q.stride] = q.vw[i].im;
+      }
+    }
+    return;
+  }
+  const LayoutJob& j = J.job[blockIdx.y];
+  const unsigned Kz = J.Nz / 2, Ny = J.Ny, total = (unsigned)j.n * Ny * Kz;
+  const unsigned base = blockIdx.x * (256u * kLayoutPer) + threadIdx.x;
+  if (base >= total) return;
+  c64 v[kLayoutPer];
+#pragma unroll
+  for (int t = 0; t < kLayoutPer; ++t) {
+    const unsigned idx = base + 256u * t;
+    v[t] = idx < total ? j.src[idx] : cmk(0.0, 0.0);
+    if (J.conj) v[t].im = -v[t].im;
+  }
+#pragma unroll
+  for (int t = 0; t < kLayoutPer; ++t) {
+    const unsigned idx = base + 256u * t;
+    if (idx >= total) break;
+    const unsigned r = idx / Kz, kz = idx - r * Kz;
+    c64* row = j.dst + (size_t)r * J.Nz;
+    row[kz] = v[t];
+    if (kz == 0) {
+      row[Kz] = cmk(0.0, 0.0);
+    } else {
+      const unsigned ky = r % Ny;
+      j.dst[(size_t)(ky ? r - ky + (Ny - ky) : r) * J.Nz + (J.Nz - kz)] = conjc(v[t]);
+    }
   }
 }
 
@@ -513,6 +548,31 @@ static PackedFactors packed(const jfb_kmm_plan* pl, const FactorSet& fs) {
   f.su_rec = pl->su_rec;
   f.sg_rec = pl->sg_rec;
   return f;
+}
+
+static LayoutJobs layout_jobs(const Dims& d) {
+  LayoutJobs J;
+  std::memset(&J, 0, sizeof(J));
+  J.Ny = d.Ny;
+  J.Nz = d.Nz;
+  J.nD = d.nD;
+  return J;
+}
+static void add_job(LayoutJobs& J, const void* src, int n, void* dst) {
+  J.job[J.nj++] = LayoutJob{(const c64*)src, (c64*)dst, n};
+}
+static void add_pair(LayoutJobs& J, const void* a, const void* b, int64_t stride, c64* vw) {
+  J.pair[J.np++] = PairJob{(double*)a, (double*)b, stride, vw};
+}
+static int run_layout(const LayoutJobs& J, bool to_half, cudaStream_t s) {
+  size_t most = 1;
+  for (int k = 0; k < J.nj; ++k)
+    most = std::max(most, (size_t)J.job[k].n * J.Ny * (J.Nz / 2));
+  const dim3 g((unsigned)ceil_div((int64_t)most, 256 * kLayoutPer), J.nj + (J.np ? 1 : 0));
+  if (to_half) to_half_kernel<<<g, 256, 0, s>>>(J);
+  else to_full_kernel<<<g, 256, 0, s>>>(J);
+  JFB_CHECK_LAUNCH();
+  return JFB_OK;
 }
 
 static StageArgs blank_args() {
@@ -1730,38 +1790,38 @@ extern "C" int jfb_kmm_get_info(const jfb_kmm_plan* pl, jfb_kmm_info* info) {
   return JFB_OK;
 }
 
-extern "C" int jfb_kmm_set_state(jfb_kmm_plan* pl, const jfb_kmm_state* s, void* stream) {
+// The flow part of a state into / out of the plan's rings, as layout jobs
+// (the MHD entry points append the potential's arrays to the same launch).
+static int flow_state_in(jfb_kmm_plan* pl, const jfb_kmm_state* s, LayoutJobs& J) {
   JFB_REQUIRE(pl && s && s->u0 && s->u1 && s->u2 && s->g, "null pointer");
   JFB_REQUIRE(s->history_steps >= 0 && s->history_steps <= 2, "history_steps in [0, 2]");
-  cudaStream_t st = (cudaStream_t)stream;
   const Dims& d = pl->d;
-  pl->n = 0;
-  const int c = slot(0), o1 = slot(-1), o2 = slot(-2);
-  const int blocks = 512;
-  auto half = [&](const void* full, int n, c64* dst) {
-    if (full) to_half_kernel<<<blocks, 256, 0, st>>>((const c64*)full, n, d.Ny, d.Nz, dst);
-    else cudaMemsetAsync(dst, 0, (size_t)n * d.P * sizeof(c64), st);
-  };
-  half(s->u0, d.nB, pl->U0[c]);
-  half(s->g, d.nD, pl->G[c]);
-  half(s->u1, d.nD, pl->U1S);
-  half(s->u2, d.nD, pl->U2S);
-  means_in_kernel<<<1, 128, 0, st>>>((const c64*)s->u1, (const c64*)s->u2, d.nD, d.Ny, d.Nz,
-                                     pl->VW[c]);
-  const int lv[2] = {o1, o2};
+  J = layout_jobs(d);
+  const int c = slot(0);
+  add_job(J, s->u0, d.nB, pl->U0[c]);
+  add_job(J, s->g, d.nD, pl->G[c]);
+  add_job(J, s->u1, d.nD, pl->U1S);
+  add_job(J, s->u2, d.nD, pl->U2S);
+  add_pair(J, s->u1, s->u2, (int64_t)2 * d.Ny * d.Nz, pl->VW[c]);
+  const int lv[2] = {slot(-1), slot(-2)};
   void* const* sol[2] = {s->solution_old, s->solution_older};
   void* const* nl[2] = {s->nonlinear_old, s->nonlinear_older};
   for (int k = 0; k < 2; ++k) {
-    half(sol[k][0], d.nB, pl->U0[lv[k]]);
-    half(sol[k][1], d.nD, pl->G[lv[k]]);
-    real_pair_in_kernel<<<1, 128, 0, st>>>((const double*)sol[k][2],
-                                           (const double*)sol[k][3], d.nD, pl->VW[lv[k]]);
-    half(nl[k][0], d.nB, pl->NU[lv[k]]);
-    half(nl[k][1], d.nD, pl->NG[lv[k]]);
-    real_pair_in_kernel<<<1, 128, 0, st>>>((const double*)nl[k][2], (const double*)nl[k][3],
-                                           d.nD, pl->NVW[lv[k]]);
+    add_job(J, sol[k][0], d.nB, pl->U0[lv[k]]);
+    add_job(J, sol[k][1], d.nD, pl->G[lv[k]]);
+    add_pair(J, sol[k][2], sol[k][3], 1, pl->VW[lv[k]]);
+    add_job(J, nl[k][0], d.nB, pl->NU[lv[k]]);
+    add_job(J, nl[k][1], d.nD, pl->NG[lv[k]]);
+    add_pair(J, nl[k][2], nl[k][3], 1, pl->NVW[lv[k]]);
   }
-  JFB_CHECK_LAUNCH();
+  return JFB_OK;
+}
+
+static int finish_state_in(jfb_kmm_plan* pl, const jfb_kmm_state* s, const LayoutJobs& J,
+                           cudaStream_t st) {
+  int rc = run_layout(J, true, st);
+  if (rc) return rc;
+  pl->n = 0;
   pl->hist = (int)s->history_steps;
   pl->have_state = true;
   pl->have_H = false;
@@ -1769,40 +1829,49 @@ extern "C" int jfb_kmm_set_state(jfb_kmm_plan* pl, const jfb_kmm_state* s, void*
   return JFB_OK;
 }
 
-extern "C" int jfb_kmm_get_state(jfb_kmm_plan* pl, const jfb_kmm_state* s, void* stream) {
+static int flow_state_out(jfb_kmm_plan* pl, const jfb_kmm_state* s, LayoutJobs& J,
+                          cudaStream_t st) {
   JFB_REQUIRE(pl && s, "null pointer");
   if (!pl->have_state) {
     set_error("no state loaded");
     return JFB_ERR_STATE;
   }
-  cudaStream_t st = (cudaStream_t)stream;
   const Dims& d = pl->d;
   int rc = ensure_explicit(pl, st);
   if (rc) return rc;
-  const int c = slot(pl->n), o1 = slot(pl->n - 1), o2 = slot(pl->n - 2);
-  const int blocks = 512;
+  J = layout_jobs(d);
   auto full = [&](const c64* src, int n, void* dst) {
-    if (dst) to_full_kernel<<<blocks, 256, 0, st>>>(src, n, d.Ny, d.Nz, (c64*)dst);
+    if (dst) add_job(J, src, n, dst);
   };
+  const int c = slot(pl->n);
   full(pl->U0[c], d.nB, s->u0);
   full(pl->G[c], d.nD, s->g);
   full(pl->U1S, d.nD, s->u1);
   full(pl->U2S, d.nD, s->u2);
-  const int lv[2] = {o1, o2};
+  const int lv[2] = {slot(pl->n - 1), slot(pl->n - 2)};
   void* const* sol[2] = {s->solution_old, s->solution_older};
   void* const* nl[2] = {s->nonlinear_old, s->nonlinear_older};
   for (int k = 0; k < 2; ++k) {
     full(pl->U0[lv[k]], d.nB, sol[k][0]);
     full(pl->G[lv[k]], d.nD, sol[k][1]);
-    real_pair_out_kernel<<<1, 128, 0, st>>>(pl->VW[lv[k]], d.nD, (double*)sol[k][2],
-                                            (double*)sol[k][3]);
+    add_pair(J, sol[k][2], sol[k][3], 1, pl->VW[lv[k]]);
     full(pl->NU[lv[k]], d.nB, nl[k][0]);
     full(pl->NG[lv[k]], d.nD, nl[k][1]);
-    real_pair_out_kernel<<<1, 128, 0, st>>>(pl->NVW[lv[k]], d.nD, (double*)nl[k][2],
-                                            (double*)nl[k][3]);
+    add_pair(J, nl[k][2], nl[k][3], 1, pl->NVW[lv[k]]);
   }
-  JFB_CHECK_LAUNCH();
   return JFB_OK;
+}
+
+extern "C" int jfb_kmm_set_state(jfb_kmm_plan* pl, const jfb_kmm_state* s, void* stream) {
+  LayoutJobs J;
+  int st = flow_state_in(pl, s, J);
+  return st ? st : finish_state_in(pl, s, J, (cudaStream_t)stream);
+}
+
+extern "C" int jfb_kmm_get_state(jfb_kmm_plan* pl, const jfb_kmm_state* s, void* stream) {
+  LayoutJobs J;
+  int st = flow_state_out(pl, s, J, (cudaStream_t)stream);
+  return st ? st : run_layout(J, false, (cudaStream_t)stream);
 }
 
 extern "C" int jfb_kmm_advance(jfb_kmm_plan* pl, int64_t steps, void* stream) {
@@ -1879,11 +1948,9 @@ extern "C" int jfb_kmm_convection(jfb_kmm_plan* pl, void* h0, void* h1, void* h2
   if (st) return st;
   const Dims& d = pl->d;
   void* outs[3] = {h0, h1, h2};
-  for (int f = 0; f < 3; ++f)
-    to_full_kernel<<<512, 256, 0, s>>>(pl->HD + (size_t)f * d.nD * d.P, d.nD, d.Ny, d.Nz,
-                                       (c64*)outs[f]);
-  JFB_CHECK_LAUNCH();
-  return JFB_OK;
+  LayoutJobs J = layout_jobs(d);
+  for (int f = 0; f < 3; ++f) add_job(J, pl->HD + (size_t)f * d.nD * d.P, d.nD, outs[f]);
+  return run_layout(J, false, s);
 }
 
 extern "C" int jfb_kmm_state_from_physical(jfb_kmm_plan* pl, const double* u0,
@@ -2044,48 +2111,40 @@ extern "C" int jfb_mhd_set_state(jfb_kmm_plan* pl, const jfb_mhd_state* s, void*
   JFB_REQUIRE(pl && s, "null pointer");
   JFB_REQUIRE(pl->mhd, "not an MHD plan");
   JFB_REQUIRE(s->A[0] && s->A[1] && s->A[2], "null pointer");
-  int st = jfb_kmm_set_state(pl, &s->flow, stream);
+  LayoutJobs J;
+  int st = flow_state_in(pl, &s->flow, J);
   if (st) return st;
-  cudaStream_t cs = (cudaStream_t)stream;
   const Dims& d = pl->d;
   const size_t comp = (size_t)d.nD * d.P;
   auto half3 = [&](void* const* full, c64* dst) {
-    for (int k = 0; k < 3; ++k) {
-      if (full && full[k])
-        to_half_kernel<<<512, 256, 0, cs>>>((const c64*)full[k], d.nD, d.Ny, d.Nz, dst + k * comp);
-      else
-        cudaMemsetAsync(dst + k * comp, 0, comp * sizeof(c64), cs);
-    }
+    for (int k = 0; k < 3; ++k) add_job(J, full[k], d.nD, dst + k * comp);
   };
   half3(s->A, pl->AR[slot(0)]);
   half3(s->A_old, pl->AR[slot(-1)]);
   half3(s->A_older, pl->AR[slot(-2)]);
   half3(s->nonlinear_A_old, pl->NA[slot(-1)]);
   half3(s->nonlinear_A_older, pl->NA[slot(-2)]);
-  JFB_CHECK_LAUNCH();
-  return JFB_OK;
+  return finish_state_in(pl, &s->flow, J, (cudaStream_t)stream);
 }
 
 extern "C" int jfb_mhd_get_state(jfb_kmm_plan* pl, const jfb_mhd_state* s, void* stream) {
   JFB_REQUIRE(pl && s, "null pointer");
   JFB_REQUIRE(pl->mhd, "not an MHD plan");
-  int st = jfb_kmm_get_state(pl, &s->flow, stream);
+  LayoutJobs J;
+  int st = flow_state_out(pl, &s->flow, J, (cudaStream_t)stream);
   if (st) return st;
-  cudaStream_t cs = (cudaStream_t)stream;
   const Dims& d = pl->d;
   const size_t comp = (size_t)d.nD * d.P;
   auto full3 = [&](const c64* src, void* const* dst) {
     for (int k = 0; k < 3; ++k)
-      if (dst[k])
-        to_full_kernel<<<512, 256, 0, cs>>>(src + k * comp, d.nD, d.Ny, d.Nz, (c64*)dst[k]);
+      if (dst[k]) add_job(J, src + k * comp, d.nD, dst[k]);
   };
   full3(pl->AR[slot(pl->n)], s->A);
   full3(pl->AR[slot(pl->n - 1)], s->A_old);
   full3(pl->AR[slot(pl->n - 2)], s->A_older);
   full3(pl->NA[slot(pl->n - 1)], s->nonlinear_A_old);
   full3(pl->NA[slot(pl->n - 2)], s->nonlinear_A_older);
-  JFB_CHECK_LAUNCH();
-  return JFB_OK;
+  return run_layout(J, false, (cudaStream_t)stream);
 }
 
 extern "C" int jfb_mhd_potential_from_physical(jfb_kmm_plan* pl, const double* ax,
@@ -2125,11 +2184,9 @@ extern "C" int jfb_mhd_potential_from_physical(jfb_kmm_plan* pl, const double* a
   int st = launch_mhd(pl, m, s);
   if (st) return st;
   void* outs[3] = {a0, a1, a2};
-  for (int k = 0; k < 3; ++k)
-    to_full_kernel<<<512, 256, 0, s>>>(pl->HD + (size_t)k * d.nD * d.P, d.nD, d.Ny, d.Nz,
-                                       (c64*)outs[k]);
-  JFB_CHECK_LAUNCH();
-  return JFB_OK;
+  LayoutJobs J = layout_jobs(d);
+  for (int k = 0; k < 3; ++k) add_job(J, pl->HD + (size_t)k * d.nD * d.P, d.nD, outs[k]);
+  return run_layout(J, false, s);
 }
 
 extern "C" int jfb_mhd_convection(jfb_kmm_plan* pl, void* h0, void* h1, void* h2, void* ha0,
@@ -2159,10 +2216,10 @@ extern "C" int jfb_mhd_convection(jfb_kmm_plan* pl, void* h0, void* h1, void* h2
       a.emf_b0x = pl->mphys.uw_emf * pl->mphys.b0x;
     }
     if ((st = launch_pencil(pl, a, s))) return st;
+    LayoutJobs J = layout_jobs(d);
     for (int f = 0; f < 3; ++f)
-      to_full_kernel<<<512, 256, 0, s>>>(pl->HD + (size_t)f * d.nD * d.P, d.nD, d.Ny, d.Nz,
-                                         (c64*)outs[3 * half + f]);
-    JFB_CHECK_LAUNCH();
+      add_job(J, pl->HD + (size_t)f * d.nD * d.P, d.nD, outs[3 * half + f]);
+    if ((st = run_layout(J, false, s))) return st;
   }
   return JFB_OK;
 }
@@ -2772,11 +2829,11 @@ extern "C" int jfb_kmm_gain_gradient(jfb_kmm_plan* pl, const jfb_kmm_state* init
   const c64* outs_half[4] = {R.EU[0], R.EU[1], R.EU[2], S0.g};
   void* outs[4] = {grad->u0, grad->u1, grad->u2, grad->g};
   const int rows[4] = {d.nB, d.nD, d.nD, d.nD};
-  for (int k = 0; k < 4; ++k) {
-    if (!outs[k]) continue;
-    to_full_kernel<<<512, 256, 0, s>>>(outs_half[k], rows[k], d.Ny, d.Nz, (c64*)outs[k]);
-    conj_kernel<<<512, 256, 0, s>>>((c64*)outs[k], (size_t)rows[k] * d.Ny * d.Nz);
-  }
+  LayoutJobs J = layout_jobs(d);
+  J.conj = 1;
+  for (int k = 0; k < 4; ++k)
+    if (outs[k]) add_job(J, outs_half[k], rows[k], outs[k]);
+  if ((st = run_layout(J, false, s))) return st;
   for (int k = 0; k < 4; ++k) {
     void* const lv[4] = {grad->nonlinear_old[k], grad->nonlinear_older[k], grad->solution_old[k],
                          grad->solution_older[k]};
@@ -2813,10 +2870,10 @@ extern "C" int jfb_kmm_energy_gradient(jfb_kmm_plan* pl, const jfb_kmm_state* st
   if ((st = adj_energy(pl, R, pl->U0[slot(0)], pl->U1S, pl->U2S, 2.0 * area, false, s))) return st;
   void* outs[3] = {grad->u0, grad->u1, grad->u2};
   const int rows[3] = {d.nB, d.nD, d.nD};
-  for (int k = 0; k < 3; ++k) {
-    to_full_kernel<<<512, 256, 0, s>>>(R.EU[k], rows[k], d.Ny, d.Nz, (c64*)outs[k]);
-    conj_kernel<<<512, 256, 0, s>>>((c64*)outs[k], (size_t)rows[k] * d.Ny * d.Nz);
-  }
+  LayoutJobs J = layout_jobs(d);
+  J.conj = 1;
+  for (int k = 0; k < 3; ++k) add_job(J, R.EU[k], rows[k], outs[k]);
+  if ((st = run_layout(J, false, s))) return st;
   if (grad->g) JFB_CHECK_CUDA(cudaMemsetAsync(grad->g, 0, (size_t)d.nD * d.Ny * d.Nz * sizeof(c64), s));
   JFB_CHECK_LAUNCH();
   JFB_CHECK_CUDA(cudaStreamSynchronize(s));

@@ -340,10 +340,4 @@ __global__ void axpy_kernel(c64* __restrict__ y, const c64* __restrict__ x, doub
     y[i] = y[i] + a * x[i];
 }
 
-__global__ void conj_kernel(c64* __restrict__ y, size_t n) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x)
-    y[i].im = -y[i].im;
-}
-
 }  // namespace jfb
