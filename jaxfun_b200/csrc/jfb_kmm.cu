@@ -1414,6 +1414,12 @@ static int create_plan(const jfb_kmm_config* cfg, const jfb_mhd_params* mhd,
   UP(Q, op.Q);
   UP(V, op.V);
   {
+    std::vector<double> VT(op.V.size());
+    for (int j = 0; j < d.Nx; ++j)
+      for (int n = 0; n < d.Nx; ++n) VT[(size_t)n * d.Nx + j] = op.V[(size_t)j * d.Nx + n];
+    UP(VT, VT);
+  }
+  {
     const int N = d.Nx, Jh = (N + 1) / 2, Jl = N / 2, Ne = (N + 1) / 2, No = N / 2;
     std::vector<double> VE((size_t)Jh * Ne), VO((size_t)Jh * std::max(1, No)),
         QE((size_t)Ne * Jh), QO((size_t)std::max(1, No) * std::max(1, Jl));
@@ -1660,6 +1666,14 @@ static int create_plan(const jfb_kmm_config* cfg, const jfb_mhd_params* mhd,
     UPM(B2, gh.B2);
     UPM(C1, gh.C1);
     UPM(C2, gh.C2);
+    auto transposed = [&](const std::vector<double>& a) {  // N x nD -> nD x N
+      std::vector<double> t(a.size());
+      for (int j = 0; j < d.Nx; ++j)
+        for (int k = 0; k < d.nD; ++k) t[(size_t)k * d.Nx + j] = a[(size_t)j * d.nD + k];
+      return t;
+    };
+    UPM(B1T, transposed(gh.B1));
+    UPM(B2T, transposed(gh.B2));
 #undef UPM
     M.Jh = (d.Nx + 1) / 2;
     M.Jl = d.Nx / 2;
@@ -2030,7 +2044,7 @@ extern "C" int jfb_kmm_diagnostics(jfb_kmm_plan* pl, double* out, void* stream) 
   diag_kernel<<<pl->diag_blocks, kNW * 32, pl->smem_diag, s>>>(
       pl->ops, d, pl->U0[c], pl->U1S, pl->U2S, pl->diag_partial, pl->diag_mean);
   JFB_CHECK_LAUNCH();
-  diag_finish_kernel<<<1, 32, 0, s>>>(d, pl->diag_partial, pl->diag_blocks, pl->diag_mean,
+  diag_finish_kernel<<<1, kDiagFinish, 0, s>>>(d, pl->diag_partial, pl->diag_blocks, pl->diag_mean,
                                       pl->cfg.ly, pl->cfg.lz, pl->cfg.x_lo, pl->cfg.x_hi,
                                       out, pl->status);
   JFB_CHECK_LAUNCH();
@@ -2231,10 +2245,10 @@ extern "C" int jfb_mhd_diagnostics(jfb_kmm_plan* pl, double* out, void* stream) 
   if (st) return st;
   cudaStream_t s = (cudaStream_t)stream;
   const Dims& d = pl->d;
-  mhd_diag_kernel<<<pl->diag_blocks, kNW * 32, 0, s>>>(pl->ops, d, pl->mops, pl->AR[slot(pl->n)],
+  mhd_diag_kernel<<<pl->diag_blocks, kNW * 32, (size_t)kNW * 3 * d.nD * sizeof(c64), s>>>(pl->ops, d, pl->mops, pl->AR[slot(pl->n)],
                                                        pl->mdiag_partial);
   JFB_CHECK_LAUNCH();
-  mhd_diag_finish_kernel<<<1, 32, 0, s>>>(pl->mdiag_partial, pl->diag_blocks, pl->cfg.ly,
+  mhd_diag_finish_kernel<<<1, kDiagFinish, 0, s>>>(pl->mdiag_partial, pl->diag_blocks, pl->cfg.ly,
                                           pl->cfg.lz, out + 8, pl->status);
   JFB_CHECK_LAUNCH();
   return JFB_OK;

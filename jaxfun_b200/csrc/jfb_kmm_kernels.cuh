@@ -37,6 +37,7 @@ constexpr int kLoadBatch = 4;    // staged loads per thread in flight
 struct DevOps {
   const double* Q;   // [n][j] scalar-product quadrature (Nx x Nx)
   const double* V;   // [j][n] Chebyshev Vandermonde (Nx x Nx)
+  const double* VT;  // [n][j] its transpose (lanes over the nodes j read consecutively)
   const double* VE;  // [j][m] = V[j][2m],   j < ceil(Nx/2)
   const double* VO;  // [j][m] = V[j][2m+1], j < ceil(Nx/2)
   const double* QE;  // [m][j] = Q[2m][j],   j < ceil(Nx/2)
@@ -1500,8 +1501,16 @@ __global__ void __launch_bounds__(256) z_forward_real_kernel(Dims d, FFTPlan pla
 // reference's uniform quadrature); x uses the Fejer-I weights of the Gauss
 // nodes.  Per block: partial sums of |u|^2 and |div u|^2; the mean pencil
 // writes its wall / base-flow terms.  diag_finish_kernel reduces in a fixed
-// order (deterministic).
+// order (deterministic).  Bound by the latency of its dependent passes at
+// 65x64x64 and by FP64 multiply-adds at 129x128x128 (4 fields x Nx^2 / 2 per
+// pencil: mirror nodes share their half sums).  Lanes run over the nodes and
+// read the transposed Vandermonde matrix, so its loads are consecutive, and
+// the mean pencil's sums are spread over its warp (on one lane they were the
+// kernel's critical path): 87 -> 31 us at 65x64x64, 652 -> 154 us at
+// 129x128x128; the finish over all partial sums on 256 threads instead of
+// one 18 -> 2.7 us and 48 -> 2.9 us.
 // ---------------------------------------------------------------------------
+constexpr int kDiagRows = 2;  // node pairs per lane
 __global__ void __launch_bounds__(256) diag_kernel(DevOps o, Dims d, const c64* __restrict__ u0,
                                                    const c64* __restrict__ u1,
                                                    const c64* __restrict__ u2,
@@ -1531,67 +1540,122 @@ __global__ void __launch_bounds__(256) diag_kernel(DevOps o, Dims d, const c64* 
     }
     __syncwarp();
     apply_SBT(o, d, B3, B0, lane);
-    if (lane == 0) {
-      for (int n = d.Nx - 1; n >= 0; --n) {
-        c64 v = (n < d.nD) ? B1[n] : cmk(0.0, 0.0);
-        if (n >= 2) v = v - B1[n - 2];
-        B1[n] = v;
-      }
-    } else if (lane == 1) {
-      for (int n = d.Nx - 1; n >= 0; --n) {
-        c64 v = (n < d.nD) ? B2[n] : cmk(0.0, 0.0);
-        if (n >= 2) v = v - B2[n - 2];
-        B2[n] = v;
-      }
+    // S_D^T in place, highest rows first (row n reads rows n and n - 2)
+    for (int n0 = (d.Nx - 1) & ~31; n0 >= 0; n0 -= 32) {
+      const int n = n0 + lane;
+      c64 v1 = cmk(0.0, 0.0), v2 = v1;
+      if (n < d.nD) v1 = B1[n], v2 = B2[n];
+      if (n >= 2 && n < d.Nx) v1 = v1 - B1[n - 2], v2 = v2 - B2[n - 2];
+      __syncwarp();
+      if (n < d.Nx) B1[n] = v1, B2[n] = v2;
+      __syncwarp();
     }
-    __syncwarp();
     chebder_warp(B0, B3, d.Nx, d.dfx, lane, d.family);
     for (int n = lane; n < d.Nx; n += 32) B3[n] = B3[n] + mul_i(kyp * B1[n] + kzp * B2[n]);
     __syncwarp();
     const double mult = (kz == 0) ? 1.0 : 2.0;
-    for (int j = lane; j < d.Nx; j += 32) {
-      c64 v0 = cmk(0.0, 0.0), v1 = v0, v2 = v0, v3 = v0;
-      for (int n = 0; n < d.Nx; ++n) {
-        const double t = __ldg(o.V + (size_t)j * d.Nx + n);
-        v0 = v0 + t * B0[n];
-        v1 = v1 + t * B1[n];
-        v2 = v2 + t * B2[n];
-        v3 = v3 + t * B3[n];
-      }
+    auto node = [&](int j, const c64 (&v)[4]) {
       const double w = o.fejer[j] * mult;
-      e_u += w * (v0.re * v0.re + v0.im * v0.im + v1.re * v1.re + v1.im * v1.im +
-                  v2.re * v2.re + v2.im * v2.im);
-      e_div += w * (v3.re * v3.re + v3.im * v3.im);
+      e_u += w * (v[0].re * v[0].re + v[0].im * v[0].im + v[1].re * v[1].re + v[1].im * v[1].im +
+                  v[2].re * v[2].re + v[2].im * v[2].im);
+      e_div += w * (v[3].re * v[3].re + v[3].im * v[3].im);
       if (ky == 0 && kz == 0) {
         // base-flow cross term 2 Ub Re(u1_00) + Ub^2 and the mean shear dv/dx
         const double ub = d.uwall * o.xphys[j];
-        meanterms[8 + j] = o.fejer[j] * (2.0 * ub * v1.re + ub * ub);
+        meanterms[8 + j] = o.fejer[j] * (2.0 * ub * v[1].re + ub * ub);
+      }
+    };
+    // mirror nodes x_j, x_{N-1-j} = -x_j share the even and odd half sums
+    const int Jl = d.Nx / 2;
+    for (int j0 = 0; j0 < Jl; j0 += 32 * kDiagRows) {
+      const bool two = j0 + 32 < Jl;  // whole warp
+      const int ja = min(j0 + lane, Jl - 1), jb = min(j0 + 32 + lane, Jl - 1);
+      c64 ea[4], oa[4], eb[4], ob[4];
+#pragma unroll
+      for (int f = 0; f < 4; ++f) ea[f] = oa[f] = eb[f] = ob[f] = cmk(0.0, 0.0);
+      // rows n, n + 1 of VT for both node pairs, loaded one step ahead
+      auto load = [&](int n, double (&t)[4]) {
+        const double* r = o.VT + (size_t)n * d.Nx;
+        const bool even = n < d.Nx, odd = n + 1 < d.Nx;
+        t[0] = even ? __ldg(r + ja) : 0.0;
+        t[1] = odd ? __ldg(r + d.Nx + ja) : 0.0;
+        t[2] = two && even ? __ldg(r + jb) : 0.0;
+        t[3] = two && odd ? __ldg(r + d.Nx + jb) : 0.0;
+      };
+      double tn[4];
+      load(0, tn);
+#pragma unroll 1
+      for (int n = 0; n < d.Nx; n += 2) {
+        const double ta0 = tn[0], ta1 = tn[1], tb0 = tn[2], tb1 = tn[3];
+        load(n + 2, tn);
+        const int n1 = min(n + 1, d.Nx - 1);
+#pragma unroll
+        for (int f = 0; f < 4; ++f) {
+          const c64* B = B0 + f * d.Nx;
+          const c64 x0 = B[n], x1 = B[n1];
+          ea[f] = ea[f] + ta0 * x0;
+          oa[f] = oa[f] + ta1 * x1;
+          if (two) {
+            eb[f] = eb[f] + tb0 * x0;
+            ob[f] = ob[f] + tb1 * x1;
+          }
+        }
+      }
+      c64 vp[4], vm[4];
+      if (j0 + lane < Jl) {
+#pragma unroll
+        for (int f = 0; f < 4; ++f) vp[f] = ea[f] + oa[f], vm[f] = ea[f] - oa[f];
+        node(ja, vp);
+        node(d.Nx - 1 - ja, vm);
+      }
+      if (j0 + 32 + lane < Jl) {
+#pragma unroll
+        for (int f = 0; f < 4; ++f) vp[f] = eb[f] + ob[f], vm[f] = eb[f] - ob[f];
+        node(jb, vp);
+        node(d.Nx - 1 - jb, vm);
       }
     }
+    if (d.Nx & 1) {  // the middle node: lanes over the coefficients
+      c64 v[4];
+#pragma unroll
+      for (int f = 0; f < 4; ++f) v[f] = cmk(0.0, 0.0);
+      for (int n = 2 * lane; n < d.Nx; n += 64) {
+        const double t = __ldg(o.V + (size_t)Jl * d.Nx + n);
+#pragma unroll
+        for (int f = 0; f < 4; ++f) v[f] = v[f] + t * B0[f * d.Nx + n];
+      }
+#pragma unroll
+      for (int f = 0; f < 4; ++f)
+        for (int off = 16; off > 0; off >>= 1) {
+          v[f].re += __shfl_down_sync(0xffffffffu, v[f].re, off);
+          v[f].im += __shfl_down_sync(0xffffffffu, v[f].im, off);
+        }
+      if (lane == 0) node(Jl, v);
+    }
     if (ky == 0 && kz == 0) {
-      // wall values and wall derivatives of the mean streamwise velocity
+      // wall values and wall derivatives of the mean streamwise velocity, and
+      // the integral of its shear, lanes over the coefficients / nodes
       chebder_warp(B1, B3, d.Nx, d.dfx, lane, d.family);
-      if (lane == 0) {
-        double top = 0.0, bot = 0.0, stop = 0.0, sbot = 0.0, shear = 0.0;
-        for (int n = 0; n < d.Nx; ++n) {
-          const double sgn = (n & 1) ? -1.0 : 1.0;
-          top += B1[n].re;
-          bot += sgn * B1[n].re;
-          // d/dX P_n at X = 1: n^2 (Chebyshev), n (n + 1) / 2 (Legendre)
-          const double n2 = d.family ? 0.5 * n * (n + 1.0) : (double)n * n;
-          stop += n2 * B1[n].re * d.dfx;
-          sbot += -sgn * n2 * B1[n].re * d.dfx;
-        }
-        for (int j = 0; j < d.Nx; ++j) {
-          double dv = 0.0;
-          for (int n = 0; n < d.Nx; ++n) dv += __ldg(o.V + (size_t)j * d.Nx + n) * B3[n].re;
-          shear += o.fejer[j] * dv;
-        }
-        meanterms[0] = top;
-        meanterms[1] = bot;
-        meanterms[2] = stop;
-        meanterms[3] = sbot;
-        meanterms[4] = shear;
+      double m[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+      for (int n = lane; n < d.Nx; n += 32) {
+        const double sgn = (n & 1) ? -1.0 : 1.0;
+        // d/dX P_n at X = 1: n^2 (Chebyshev), n (n + 1) / 2 (Legendre)
+        const double n2 = d.family ? 0.5 * n * (n + 1.0) : (double)n * n;
+        m[0] += B1[n].re;
+        m[1] += sgn * B1[n].re;
+        m[2] += n2 * B1[n].re * d.dfx;
+        m[3] += -sgn * n2 * B1[n].re * d.dfx;
+      }
+      for (int j = lane; j < d.Nx; j += 32) {
+        double dv = 0.0;
+#pragma unroll 16
+        for (int n = 0; n < d.Nx; ++n) dv += __ldg(o.VT + (size_t)n * d.Nx + j) * B3[n].re;
+        m[4] += o.fejer[j] * dv;
+      }
+#pragma unroll
+      for (int k = 0; k < 5; ++k) {
+        for (int off = 16; off > 0; off >>= 1) m[k] += __shfl_down_sync(0xffffffffu, m[k], off);
+        if (lane == 0) meanterms[k] = m[k];
       }
     }
   }
@@ -1616,19 +1680,40 @@ __global__ void __launch_bounds__(256) diag_kernel(DevOps o, Dims d, const c64* 
   }
 }
 
+// Sums of K values over a block of kDiagFinish threads in a fixed order; the
+// totals on thread 0.
+constexpr int kDiagFinish = 256;
+template <int K>
+__device__ __forceinline__ void block_sum(double (&v)[K]) {
+  __shared__ double red[kDiagFinish / 32][K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    for (int off = 16; off > 0; off >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], off);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][k] = v[k];
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      for (int w = 1; w < kDiagFinish / 32; ++w) v[k] += red[w][k];
+  }
+}
+
 // out = (Epert, Etot, divL2, u_top, u_bot, wall_shear_top, wall_shear_bot, mean_shear)
-__global__ void diag_finish_kernel(Dims d, const double* __restrict__ partial, int nblocks,
+__global__ void __launch_bounds__(kDiagFinish) diag_finish_kernel(Dims d, const double* __restrict__ partial, int nblocks,
                                    const double* __restrict__ meanterms, double ly, double lz,
                                    double x_lo, double x_hi, double* __restrict__ out,
                                    int* status) {
   const double lx = x_hi - x_lo;
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double eu = 0.0, ed = 0.0, base = 0.0;
-  for (int b = 0; b < nblocks; ++b) {
-    eu += partial[2 * b];
-    ed += partial[2 * b + 1];
+  double sum[3] = {0.0, 0.0, 0.0};  // |u|^2, |div u|^2, base-flow terms
+  for (int b = threadIdx.x; b < nblocks; b += kDiagFinish) {
+    sum[0] += partial[2 * b];
+    sum[1] += partial[2 * b + 1];
   }
-  for (int j = 0; j < d.Nx; ++j) base += meanterms[8 + j];
+  for (int j = threadIdx.x; j < d.Nx; j += kDiagFinish) sum[2] += meanterms[8 + j];
+  block_sum<3>(sum);
+  if (threadIdx.x != 0) return;
+  const double eu = sum[0], ed = sum[1], base = sum[2];
   const double area = ly * lz;
   out[0] = area * eu;
   out[1] = area * (eu + base);
