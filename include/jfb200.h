@@ -48,6 +48,20 @@ int jfb_dia_matvec(const double* data, const int64_t* offsets, int64_t n_diags,
                    int64_t outer, int64_t inner, int is_complex, int transpose,
                    void* stream);
 
+/* TPMatrices @ x (src/jaxfun/la/tpmatrix.py:153-157, 300-428) of a Fourier x
+ * polynomial operator as one launch: y = sum_k coefs[k] (w_k1 (x) w_k2 (x)
+ * data_k) x, x and y (outer, n_P, inner) with the polynomial axis in the
+ * middle and the flattened Fourier index f = o * inner + t over
+ * fourier_sizes (one or two axes).  data[k]: DIA storage (n_diags[k], n_P)
+ * with its offsets consecutively in `offsets` (host); weights[k * n_fourier +
+ * j]: the diagonal of Fourier axis j (device, NULL for ones).  At most eight
+ * terms and 512 diagonals, n_P within a CTA's shared memory (JFB_ERR_ARG
+ * else: apply the factors with jfb_dia_matvec).  x and y must not alias. */
+int jfb_tp_matvec(int64_t n_terms, const double* const* data, const int64_t* n_diags,
+                  const int64_t* offsets, const double* const* weights, int64_t n_fourier,
+                  const int64_t* fourier_sizes, const double* coefs, int64_t n_P, int64_t outer,
+                  int64_t inner, const double* x, double* y, int is_complex, void* stream);
+
 /* Batched banded LU without pivoting (src/jaxfun/la/diamatrix.py:394-504,
  * kernel 1936-1973; batched use in tpmatrix.py:1105-1149).
  * band has shape (n_batch, p + q + 1, n) with band[b, p + off, j] =

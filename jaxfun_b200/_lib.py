@@ -151,6 +151,12 @@ SIGNATURES = {
         [c_void_p, POINTER(c_int64), c_int64, c_int64, c_int64, c_void_p, c_void_p,
          c_int64, c_int64, c_int, c_int, c_void_p],
     ),
+    "jfb_tp_matvec": (
+        c_int,
+        [c_int64, POINTER(c_void_p), POINTER(c_int64), POINTER(c_int64), POINTER(c_void_p),
+         c_int64, POINTER(c_int64), POINTER(c_double), c_int64, c_int64, c_int64, c_void_p,
+         c_void_p, c_int, c_void_p],
+    ),
     "jfb_banded_lu_factor": (
         c_int, [c_void_p, c_int64, c_int64, c_int64, c_int64, c_void_p]
     ),

@@ -5,7 +5,9 @@
 //   DiaMatrix storage / matvec / rmatvec   src/jaxfun/la/diamatrix.py:100-348
 //   no-pivot banded LU kernel              src/jaxfun/la/diamatrix.py:1936-1973
 //   batched wavenumber solve               src/jaxfun/la/tpmatrix.py:686-799
+#include <algorithm>
 #include <climits>
+#include <cstdlib>
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -281,6 +283,444 @@ __global__ void wavenumber_solve_warp_kernel(const double* __restrict__ L, Offse
   }
 }
 
+// The same solve with the factors staged in shared memory.  A block owns M
+// consecutive modes (neighbours along `inner`, so that neighbouring vectors
+// share their memory sectors) and RB right-hand sides of each, and loads only
+// the entries a factor has (column c of diagonal s >= 0 from c = s on: half
+// the bytes of a full triangle), once for all right-hand sides.  When every
+// offset is even the two parity classes are independent systems.
+//   wide factors    (wavenumber_solve_tri_kernel) a warp per mode with the
+//                   unknowns in registers, lane = row of a class; U (and L,
+//                   when it has more than kTriFewL diagonals) as packed dense
+//                   triangles, so a column update is one shared-memory read
+//                   and one multiply-add per row.  y_c stays in place and is
+//                   scaled by 1 / U[c, c] on output.  Up to four right-hand
+//                   sides share a warp and its factor reads.  Bound by issue.
+//   narrow factors  (wavenumber_solve_narrow_kernel) a thread per vector and
+//                   class, rows in order, vectors in shared memory.
+// n_P = 63, 4096 modes, three complex right-hand sides (one class of 32 and
+// one of 31 rows): 76 us.  A warp per system reading strided vectors and the
+// factors once per right-hand side took 201 us; with the vectors in shared
+// memory instead of registers 279 us (two read-modify-writes of 16 bytes per
+// lane and column); one right-hand side per warp 84 us.
+struct StagedTable {
+  int n;
+  int off[kMaxOffsets];
+  int start[kMaxOffsets];  // first staged entry of the diagonal within the mode's record
+};
+struct StagedSolve {
+  StagedTable L, U;
+  int main, n, rec, ldx, M, RB, even, denseL, zero;
+  int oL, oD, m0;  // tri form: L part and reciprocal diagonal within the record, class 0 rows
+  unsigned outer, inner;
+  int64_t n_F, n_rhs;
+};
+constexpr int kStagedNarrow = 8;  // diagonals a single thread walks
+constexpr int kTriFewL = 4;       // diagonals of L kept as diagonals in the tri form
+
+// Element i of right-hand side r of mode f = o inner + t.
+__device__ __forceinline__ size_t staged_addr(const StagedSolve& q, unsigned f, int64_t r, int i) {
+  const unsigned o = f / q.inner, t = f - o * q.inner;
+  return ((size_t)(r * q.outer + o) * q.n + i) * q.inner + t;
+}
+
+template <typename V>
+__global__ void wavenumber_solve_narrow_kernel(const __grid_constant__ StagedSolve q,
+                                               const double* __restrict__ L,
+                                               const double* __restrict__ U, const V* rhs,
+                                               V* out) {
+  constexpr bool kCplx = sizeof(V) != sizeof(double);
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int n = q.n, nv = q.M * q.RB, tid = threadIdx.x, nt = blockDim.x;
+  V* xs = reinterpret_cast<V*>(smem_raw);                       // [nv][ldx]
+  double* fac = reinterpret_cast<double*>(xs + (size_t)nv * q.ldx);  // [M][rec]
+  const int64_t f0 = (int64_t)blockIdx.x * q.M, r0 = (int64_t)blockIdx.y * q.RB;
+  const int mv = (int)min((int64_t)q.M, q.n_F - f0), rv = (int)min((int64_t)q.RB, q.n_rhs - r0);
+  const int warp = tid >> 5, lane = tid & 31, nw = nt >> 5;
+  // factors: one warp per (mode, diagonal), lanes over its columns
+  for (int u = warp; u < mv * (q.L.n + q.U.n); u += nw) {
+    const int m = u / (q.L.n + q.U.n), dd = u - m * (q.L.n + q.U.n);
+    const bool up = dd >= q.L.n;
+    const int d = up ? dd - q.L.n : dd;
+    const int s = up ? q.U.off[d] : -q.L.off[d];
+    const double* src = up ? U + ((f0 + m) * q.U.n + d) * n + s : L + ((f0 + m) * q.L.n + d) * n;
+    double* dst = fac + (size_t)m * q.rec + (up ? q.U.start[d] : q.L.start[d]);
+    for (int c = lane; c < n - s; c += 32) dst[c] = src[c];
+  }
+  auto each = [&](auto&& fn) {  // all elements, the contiguous index fastest
+    for (int e = tid; e < nv * n; e += nt) {
+      int m, r, i;
+      if (q.inner == 1) {
+        i = e % n;
+        m = (e / n) % q.M;
+        r = e / (n * q.M);
+      } else {
+        m = e % q.M;
+        i = (e / q.M) % n;
+        r = e / (n * q.M);
+      }
+      if (m < mv && r < rv) fn(staged_addr(q, (unsigned)f0 + m, r0 + r, i), (r * q.M + m) * q.ldx + i);
+    }
+  };
+  each([&](size_t g, int k) { xs[k] = rhs[g]; });
+  __syncthreads();
+  const int step = q.even ? 2 : 1;
+  const int v = tid / step, cls = tid - v * step;
+  const int m = v % q.M, r = v / q.M;
+  if (v < nv && m < mv && r < rv) {
+    V* x = xs + (size_t)v * q.ldx;
+    const double* fm = fac + (size_t)m * q.rec;
+    for (int i = cls; i < n; i += step) {
+      V y = x[i], acc = V();
+      for (int d = 0; d < q.L.n; ++d) {
+        const int j = i + q.L.off[d];
+        if (j >= 0) acc = acc + fm[q.L.start[d] + j] * x[j];
+      }
+      x[i] = y - acc;
+    }
+    for (int i = n - 1 - ((n - 1 - cls) % step); i >= 0; i -= step) {
+      V y = x[i], acc = V();
+      for (int d = 0; d < q.U.n; ++d) {
+        const int sft = q.U.off[d], j = i + sft;
+        if (sft != 0 && j < n) acc = acc + fm[q.U.start[d] + i] * x[j];
+      }
+      const double dg = fm[q.U.start[q.main] + i];
+      y = y - acc;
+      if constexpr (kCplx) x[i] = cmk(y.re / dg, y.im / dg);
+      else x[i] = y / dg;
+    }
+  }
+  __syncthreads();
+  each([&](size_t g, int k) { out[g] = xs[k]; });
+}
+
+// S: rows per lane and class; R: right-hand sides per warp (they share every
+// factor read and keep R independent chains in flight).
+template <typename V, int S, int R>
+__global__ void wavenumber_solve_tri_kernel(const __grid_constant__ StagedSolve q,
+                                            const double* __restrict__ L,
+                                            const double* __restrict__ U, const V* rhs, V* out) {
+  constexpr bool kCplx = sizeof(V) != sizeof(double);
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double* fac = reinterpret_cast<double*>(smem_raw);  // [M][rec]
+  const int n = q.n, tid = threadIdx.x, nt = blockDim.x;
+  const int64_t f0 = (int64_t)blockIdx.x * q.M, r0 = (int64_t)blockIdx.y * q.RB;
+  const int mv = (int)min((int64_t)q.M, q.n_F - f0);
+  const int warp = tid >> 5, lane = tid & 31, nw = nt >> 5;
+  const int ncls = q.even ? 2 : 1, sh = q.even ? 1 : 0;
+  const int tri1 = q.m0 * (q.m0 + 1) / 2;  // first entry of class 1's triangle
+  // this warp's mode and right-hand sides, loaded first (lane + 32 s = row of
+  // the class)
+  const int m = warp % q.M;
+  const int64_t rw = r0 + (int64_t)(warp / q.M) * R;
+  const int rv = (int)min((int64_t)R, min(q.n_rhs, r0 + q.RB) - rw);
+  const bool live = m < mv && rv > 0;
+  V y[R][2][S];
+#pragma unroll
+  for (int k = 0; k < R; ++k)
+#pragma unroll
+    for (int cl = 0; cl < 2; ++cl)
+#pragma unroll
+      for (int s = 0; s < S; ++s) {
+        const int i = ((lane + 32 * s) << sh) + cl;
+        y[k][cl][s] = live && k < rv && cl < ncls && i < n
+                          ? rhs[staged_addr(q, (unsigned)f0 + m, rw + k, i)]
+                          : V();
+      }
+  // absent diagonals read as zero
+  if (q.zero)
+    for (int e = tid; e < q.M * q.rec; e += nt) fac[e] = 0.0;
+  __syncthreads();
+  // factors: one warp per (mode, diagonal), lanes over its columns, all
+  // copies in flight together
+  auto copy8 = [](double* dst, const double* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                     (unsigned)__cvta_generic_to_shared(dst)),
+                 "l"(src)
+                 : "memory");
+  };
+  for (int u = warp; u < mv * (q.L.n + q.U.n); u += nw) {
+    const int mm = u / (q.L.n + q.U.n), dd = u - mm * (q.L.n + q.U.n);
+    const bool up = dd >= q.L.n;
+    const int d = up ? dd - q.L.n : dd;
+    const int s = up ? q.U.off[d] : -q.L.off[d];
+    const double* src = up ? U + ((f0 + mm) * q.U.n + d) * n : L + ((f0 + mm) * q.L.n + d) * n;
+    double* F = fac + (size_t)mm * q.rec;
+    if (up && d == q.main) {
+      for (int c = lane; c < n; c += 32) copy8(F + q.oD + c, src + c);
+    } else if (up) {
+      for (int c = s + lane; c < n; c += 32) {  // entry (c - s, c)
+        const int cc = c >> sh, rr = (c - s) >> sh;
+        copy8(F + (sh && (c & 1) ? tri1 : 0) + cc * (cc + 1) / 2 + rr, src + c);
+      }
+    } else {
+      for (int c = lane; c < n - s; c += 32) {  // entry (c + s, c)
+        const int cc = c >> sh, rr = (c + s) >> sh;
+        copy8(F + q.oL + (q.denseL ? (sh && (c & 1) ? tri1 : 0) + rr * (rr + 1) / 2 + cc : d * n + c),
+              src + c);
+      }
+    }
+  }
+  asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  for (int e = tid; e < mv * n; e += nt) {
+    double* dg = fac + (size_t)(e / n) * q.rec + q.oD + e % n;
+    *dg = 1.0 / *dg;
+  }
+  __syncthreads();
+  if (!live) return;  // no barrier below
+  const double* F = fac + (size_t)m * q.rec;
+  const int mc[2] = {q.even ? q.m0 : n, q.even ? n / 2 : 0};
+  auto bcast = [&](const V (&v)[S], int c) {
+    V a = v[0];
+#pragma unroll
+    for (int s = 1; s < S; ++s)
+      if (c >= 32 * s) a = v[s];
+    if constexpr (kCplx)
+      return cmk(__shfl_sync(0xffffffffu, a.re, c & 31), __shfl_sync(0xffffffffu, a.im, c & 31));
+    else
+      return __shfl_sync(0xffffffffu, a, c & 31);
+  };
+  // forward, unit lower: column c of both classes per step
+  const int steps = mc[0];
+  if (q.L.n) {
+    const int s1 = q.denseL || q.L.n != 1 ? 0 : (-q.L.off[0]) >> sh;  // the only diagonal's row shift
+#pragma unroll 1
+    for (int c = 0; c < steps - 1; ++c) {
+#pragma unroll
+      for (int cl = 0; cl < 2; ++cl) {
+        if (c >= mc[cl]) continue;  // whole warp
+        double l[S];                // this lane's entries of column c
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+          const int rr = lane + 32 * s;
+          l[s] = 0.0;
+          if (q.denseL) {
+            if (rr > c && rr < mc[cl]) l[s] = F[q.oL + (cl ? tri1 : 0) + rr * (rr + 1) / 2 + c];
+          } else if (s1) {
+            if (rr == c + s1 && rr < mc[cl]) l[s] = F[q.oL + (c << sh) + cl];
+          } else {
+            for (int d = 0; d < q.L.n; ++d)
+              if (rr == c + ((-q.L.off[d]) >> sh) && rr < mc[cl])
+                l[s] = F[q.oL + d * n + (c << sh) + cl];
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < R; ++k) {
+          const V yc = bcast(y[k][cl], c);
+#pragma unroll
+          for (int s = 0; s < S; ++s)
+            if (l[s] != 0.0) y[k][cl][s] = y[k][cl][s] - l[s] * yc;
+        }
+      }
+    }
+  }
+  // backward with the upper factor
+#pragma unroll 2
+  for (int c = steps - 1; c > 0; --c) {
+#pragma unroll
+    for (int cl = 0; cl < 2; ++cl) {
+      if (c >= mc[cl]) continue;
+      const double* T = F + (cl ? tri1 : 0) + c * (c + 1) / 2;
+      const double rd = F[q.oD + (c << sh) + cl];
+      double u[S];
+#pragma unroll
+      for (int s = 0; s < S; ++s) u[s] = lane + 32 * s < c ? T[lane + 32 * s] : 0.0;
+#pragma unroll
+      for (int k = 0; k < R; ++k) {
+        const V xc = rd * bcast(y[k][cl], c);
+#pragma unroll
+        for (int s = 0; s < S; ++s)
+          if (lane + 32 * s < c) y[k][cl][s] = y[k][cl][s] - u[s] * xc;
+      }
+    }
+  }
+#pragma unroll
+  for (int cl = 0; cl < 2; ++cl)
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+      const int i = ((lane + 32 * s) << sh) + cl;
+      if (cl >= ncls || i >= n) continue;
+      const double rd = F[q.oD + i];
+#pragma unroll
+      for (int k = 0; k < R; ++k)
+        if (k < rv) out[staged_addr(q, (unsigned)f0 + m, rw + k, i)] = rd * y[k][cl][s];
+    }
+}
+
+// Launch of the staged solve, or false when one mode's factors and vector do
+// not fit a CTA's shared memory (or, wide, more than four rows per lane): the
+// unstaged kernels take those.
+template <typename V>
+static bool staged_solve(const double* L, const OffsetTable& lt, const double* U,
+                         const OffsetTable& ut, int main_idx, int n, int64_t outer, int64_t inner,
+                         int64_t n_rhs, const V* rhs, V* out, cudaStream_t s, cudaError_t* err) {
+  *err = cudaSuccess;
+  StagedSolve q;
+  std::memset(&q, 0, sizeof(q));
+  q.main = main_idx;
+  q.n = n;
+  q.n_F = outer * inner;
+  if (q.n_F > INT_MAX) return false;
+  q.outer = (unsigned)outer;
+  q.inner = (unsigned)inner;
+  q.n_rhs = n_rhs;
+  const bool narrow = lt.n + ut.n <= kStagedNarrow;
+  q.even = 1;
+  int64_t rec = 0;
+  auto fill = [&](StagedTable& t, const OffsetTable& o) {
+    t.n = o.n;
+    for (int d = 0; d < o.n; ++d) {
+      t.off[d] = o.off[d];
+      t.start[d] = (int)rec;
+      rec += std::max(0, n - std::abs(o.off[d]));
+      if (o.off[d] & 1) q.even = 0;
+    }
+  };
+  fill(q.L, lt);
+  fill(q.U, ut);
+  q.m0 = q.even ? (n + 1) / 2 : n;
+  int S = 0;
+  if (!narrow) {
+    const int64_t m1 = q.even ? n / 2 : 0, tri = (int64_t)q.m0 * (q.m0 + 1) / 2 + m1 * (m1 + 1) / 2;
+    if (q.m0 > 128) return false;
+    S = q.m0 <= 32 ? 1 : q.m0 <= 64 ? 2 : 4;
+    q.denseL = lt.n > kTriFewL;
+    q.oL = (int)tri;
+    q.oD = (int)(tri + (q.denseL ? tri : (int64_t)lt.n * n));
+    rec = q.oD + n;
+    int in_range = 0;
+    for (int d = 0; d < ut.n; ++d) in_range += ut.off[d] < n;
+    q.zero = in_range < q.m0 || q.denseL;
+  }
+  rec |= 1;  // consecutive modes' records in different banks
+  q.ldx = narrow ? (n | 1) : 0;
+  constexpr size_t kMost = 200 * 1024, kGood = 64 * 1024;
+  auto bytes = [&](int M, int RB) {
+    return (size_t)M * rec * sizeof(double) + (size_t)M * RB * q.ldx * sizeof(V);
+  };
+  if (bytes(1, 1) > kMost) return false;
+  q.rec = (int)rec;
+  // up to 16 vectors per block (a warp each; narrow: 128, one or two threads
+  // each): right-hand sides first, then modes, as long as the records leave
+  // about three blocks per SM
+  const int most = narrow ? 128 : 16, mmax = narrow ? 16 : 4;
+  q.M = 1;
+  q.RB = (int)std::min<int64_t>(n_rhs, 8);
+  const int R = narrow ? 1 : (int)std::min<int64_t>(S == 4 ? 2 : 4, n_rhs);
+  while (q.RB > 1 && bytes(1, q.RB) > kMost) q.RB = (q.RB + 1) / 2;
+  while (q.M * 2 <= mmax && q.M * 2 * q.RB <= most && q.M < q.n_F && bytes(q.M * 2, q.RB) <= kGood)
+    q.M *= 2;
+  const int vecs = q.M * ((q.RB + R - 1) / R);  // warps (narrow: vectors)
+  const int threads = narrow ? std::max(64, (vecs * (q.even ? 2 : 1) + 31) / 32 * 32)
+                             : std::max(2, vecs) * 32;
+  const int64_t gx = (q.n_F + q.M - 1) / q.M, gy = (n_rhs + q.RB - 1) / q.RB;
+  if (gy > 65535) return false;
+  auto* k = wavenumber_solve_narrow_kernel<V>;
+  switch (10 * S + R) {
+#define JFB_TRI(SS, RR) \
+  case 10 * SS + RR: k = wavenumber_solve_tri_kernel<V, SS, RR>; break;
+    JFB_TRI(1, 1) JFB_TRI(1, 2) JFB_TRI(1, 3) JFB_TRI(1, 4)
+    JFB_TRI(2, 1) JFB_TRI(2, 2) JFB_TRI(2, 3) JFB_TRI(2, 4)
+    JFB_TRI(4, 1) JFB_TRI(4, 2)
+#undef JFB_TRI
+    default: break;  // narrow (S = 0)
+  }
+  *err = cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)(kMost + 1024));
+  if (*err != cudaSuccess) return true;
+  k<<<dim3((unsigned)gx, (unsigned)gy), threads, bytes(q.M, q.RB), s>>>(q, L, U, rhs, out);
+  *err = cudaGetLastError();
+  return true;
+}
+
+// ---------------------------------------------------------------------------
+// Sum of Kronecker terms with one polynomial axis (TPMatrices @ x,
+// tpmatrix.py:300-428, for Fourier x polynomial operators):
+//   y[o, i, t] = sum_k c_k w_k(f) sum_d data_k[d, i + off] x[o, i + off, t],
+// f = o inner + t the flattened Fourier index, w_k the product of the term's
+// diagonal matrices.  A block stages kTpCols columns of x in shared memory
+// and forms all their rows: x is read and y written once, where one launch
+// per factor of each term moved the field nine times for three terms (48 us
+// of device time at 63 x 4096 complex in nine launches, plus the sums'; now
+// 20 us in one).  Bound by the latency of its operator reads.
+// ---------------------------------------------------------------------------
+constexpr int kTpTerms = 8, kTpCols = 16, kTpThreads = 256, kTpRows = 4;
+struct TpTerm {
+  const double* data;   // (n_diags, n) DIA
+  const double* w[2];   // Fourier diagonals (null: absent)
+  double coef;
+  int first, nd;        // its offsets in TpArgs::off
+};
+struct TpArgs {
+  TpTerm t[kTpTerms];
+  int off[kMaxOffsets];
+  int nt, n;
+  unsigned n_F, inner, size2;  // size2: length of the last Fourier axis
+};
+
+template <typename V>
+__global__ void __launch_bounds__(kTpThreads)
+    tp_matvec_kernel(const __grid_constant__ TpArgs a, const V* __restrict__ x, V* __restrict__ y) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ double ws[kTpTerms * kTpCols];  // weights of the block's columns per term
+  V* xs = reinterpret_cast<V*>(smem_raw);    // [n][kTpCols + 1]
+  constexpr int LD = kTpCols + 1;
+  const int n = a.n, tid = threadIdx.x;
+  const unsigned f0 = blockIdx.x * kTpCols;
+  const int nc = (int)min((unsigned)kTpCols, a.n_F - f0);
+  auto addr = [&](int c, int i) {
+    const unsigned f = f0 + c, o = f / a.inner, t = f - o * a.inner;
+    return ((size_t)o * n + i) * a.inner + t;
+  };
+  for (int e = tid; e < n * kTpCols; e += kTpThreads) {
+    const int c = a.inner == 1 ? e / n : e % kTpCols, i = a.inner == 1 ? e % n : e / kTpCols;
+    if (c < nc) xs[i * LD + c] = x[addr(c, i)];
+  }
+  if (tid < kTpTerms * kTpCols && tid / kTpCols < a.nt) {
+    const TpTerm& t = a.t[tid / kTpCols];
+    const unsigned f = f0 + min(tid % kTpCols, nc - 1), i1 = f / a.size2, i2 = f - i1 * a.size2;
+    double w = t.coef;
+    if (t.w[0]) w *= __ldg(t.w[0] + i1);
+    if (t.w[1]) w *= __ldg(t.w[1] + i2);
+    ws[tid] = w;
+  }
+  __syncthreads();
+  const int c = tid % kTpCols;
+  // kTpRows rows per thread: independent chains over the diagonals
+  constexpr int RG = kTpThreads / kTpCols;
+  for (int i0 = tid / kTpCols; i0 < n; i0 += RG * kTpRows) {
+    V sum[kTpRows];
+#pragma unroll
+    for (int r = 0; r < kTpRows; ++r) sum[r] = V();
+#pragma unroll 1
+    for (int k = 0; k < a.nt; ++k) {
+      const TpTerm& t = a.t[k];
+      V acc[kTpRows];
+#pragma unroll
+      for (int r = 0; r < kTpRows; ++r) acc[r] = V();
+#pragma unroll 2
+      for (int d = 0; d < t.nd; ++d) {
+        const int off = a.off[t.first + d];
+        const double* row = t.data + (size_t)d * n;
+#pragma unroll
+        for (int r = 0; r < kTpRows; ++r) {
+          const int i = i0 + RG * r, col = i + off;
+          if (i < n && col >= 0 && col < n) acc[r] = acc[r] + __ldg(row + col) * xs[col * LD + c];
+        }
+      }
+      const double wk = ws[k * kTpCols + c];
+#pragma unroll
+      for (int r = 0; r < kTpRows; ++r) sum[r] = sum[r] + wk * acc[r];
+    }
+#pragma unroll
+    for (int r = 0; r < kTpRows; ++r) {
+      const int i = i0 + RG * r;
+      if (c < nc && i < n) y[addr(c, i)] = sum[r];
+    }
+  }
+}
+
 static int fill_offsets(OffsetTable& t, const int64_t* offs, int64_t n) {
   if (n < 0 || n > kMaxOffsets) {
     set_error("too many DIA offsets (max 512)");
@@ -320,6 +760,57 @@ extern "C" int jfb_dia_matvec(const double* data, const int64_t* offsets,
     dia_matvec_kernel<double><<<blocks, threads, 0, s>>>(
         data, t, n_rows, n_cols, x, y, outer, inner, transpose);
   }
+  JFB_CHECK_LAUNCH();
+  return JFB_OK;
+}
+
+extern "C" int jfb_tp_matvec(int64_t n_terms, const double* const* data, const int64_t* n_diags,
+                             const int64_t* offsets, const double* const* weights,
+                             int64_t n_fourier, const int64_t* fourier_sizes, const double* coefs,
+                             int64_t n_P, int64_t outer, int64_t inner, const double* x,
+                             double* y, int is_complex, void* stream) {
+  JFB_REQUIRE(data && n_diags && offsets && weights && fourier_sizes && coefs && x && y,
+              "null pointer");
+  JFB_REQUIRE(n_terms >= 1 && n_terms <= kTpTerms, "between 1 and 8 terms");
+  JFB_REQUIRE(n_fourier >= 1 && n_fourier <= 2, "one or two Fourier axes");
+  JFB_REQUIRE(n_P > 0 && n_P <= 4096 && outer > 0 && inner > 0, "bad shape");
+  JFB_REQUIRE(outer <= INT_MAX / inner, "bad shape");
+  int64_t nf = 1;
+  for (int64_t k = 0; k < n_fourier; ++k) {
+    JFB_REQUIRE(fourier_sizes[k] > 0 && fourier_sizes[k] <= INT_MAX, "bad shape");
+    nf *= fourier_sizes[k];
+  }
+  JFB_REQUIRE(nf == outer * inner, "Fourier sizes do not match the field");
+  TpArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.nt = (int)n_terms;
+  a.n = (int)n_P;
+  a.n_F = (unsigned)nf;
+  a.inner = (unsigned)inner;
+  a.size2 = n_fourier == 2 ? (unsigned)fourier_sizes[1] : 1u;
+  int64_t at = 0;
+  for (int k = 0; k < a.nt; ++k) {
+    JFB_REQUIRE(data[k] && n_diags[k] >= 0 && at + n_diags[k] <= kMaxOffsets, "too many DIA offsets");
+    TpTerm& t = a.t[k];
+    t.data = data[k];
+    t.coef = coefs[k];
+    t.first = (int)at;
+    t.nd = (int)n_diags[k];
+    for (int64_t j = 0; j < n_fourier; ++j) t.w[j] = weights[k * n_fourier + j];
+    for (int d = 0; d < t.nd; ++d) a.off[at + d] = (int)offsets[at + d];
+    at += t.nd;
+  }
+  const size_t sm = (size_t)n_P * (kTpCols + 1) * (is_complex ? 16 : 8);
+  JFB_REQUIRE(sm <= 200 * 1024, "polynomial axis too long for the fused product");
+  const void* fn = is_complex ? (const void*)tp_matvec_kernel<c64>
+                              : (const void*)tp_matvec_kernel<double>;
+  JFB_CHECK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+  const unsigned blocks = (a.n_F + kTpCols - 1) / kTpCols;
+  cudaStream_t s = (cudaStream_t)stream;
+  if (is_complex)
+    tp_matvec_kernel<c64><<<blocks, kTpThreads, sm, s>>>(a, (const c64*)x, (c64*)y);
+  else
+    tp_matvec_kernel<double><<<blocks, kTpThreads, sm, s>>>(a, x, y);
   JFB_CHECK_LAUNCH();
   return JFB_OK;
 }
@@ -374,15 +865,30 @@ extern "C" int jfb_wavenumber_solve(const double* L, const int64_t* L_offsets, i
   cudaStream_t s = (cudaStream_t)stream;
   const int64_t total = n_rhs * outer * inner;
   const int threads = 128;
-  if (lt.n + ut.n > 8) {  // wide factors: a warp per system, rhs read in place
+  if (lt.n + ut.n > 8) {  // wide factors: a warp per system
     // the column updates of one step write one row per diagonal
     for (int a = 0; a < ut.n; ++a)
       for (int b = a + 1; b < ut.n; ++b) JFB_REQUIRE(ut.off[a] != ut.off[b], "repeated U offset");
     for (int a = 0; a < lt.n; ++a)
       for (int b = a + 1; b < lt.n; ++b) JFB_REQUIRE(lt.off[a] != lt.off[b], "repeated L offset");
-    const int64_t wblocks = (total * 32 + threads - 1) / threads;
     const size_t sm = (size_t)(threads / 32) * 2 * n_P * sizeof(double);
     JFB_REQUIRE(sm <= 48 * 1024, "n_P too large for the warp solve (max 768)");
+  }
+  {
+    cudaError_t e;
+    const bool done =
+        is_complex ? staged_solve<c64>(L, lt, U, ut, main_idx, (int)n_P, outer, inner, n_rhs,
+                                       (const c64*)rhs, (c64*)out, s, &e)
+                   : staged_solve<double>(L, lt, U, ut, main_idx, (int)n_P, outer, inner, n_rhs,
+                                          rhs, out, s, &e);
+    if (done) {
+      JFB_CHECK_CUDA(e);
+      return JFB_OK;
+    }
+  }
+  if (lt.n + ut.n > 8) {
+    const int64_t wblocks = (total * 32 + threads - 1) / threads;
+    const size_t sm = (size_t)(threads / 32) * 2 * n_P * sizeof(double);
     if (is_complex)
       wavenumber_solve_warp_kernel<c64><<<(unsigned)wblocks, threads, sm, s>>>(
           L, lt, U, ut, main_idx, (int)n_P, outer, inner, n_rhs, (const c64*)rhs, (c64*)out);

@@ -20,6 +20,7 @@ every product, factorisation and solve runs in ``libjfb200.so``.
 from __future__ import annotations
 
 import ctypes
+import math
 from collections.abc import Sequence
 
 import torch
@@ -194,6 +195,52 @@ class LUFactors:
         return torch.movedim(out.reshape(*rest, n), -1, axis)
 
 
+def _fused_sum(tpmats: Sequence[TPMatrix], u: torch.Tensor) -> torch.Tensor | None:
+    """``sum_t tpmats[t] @ u`` as one launch (``jfb_tp_matvec``) when every
+    term is square diagonal matrices on the same one or two axes and a
+    polynomial matrix on the remaining one, all on the field's device; None
+    otherwise (the general form applies the factors one by one)."""
+    nd = u.dim()
+    if nd not in (2, 3) or len(tpmats) > 8 or u.numel() == 0:
+        return None
+    poly = -1
+    for tp in tpmats:
+        if tp.dims != nd:
+            return None
+        for a, m in enumerate(tp.mats):
+            if (m.shape != (u.shape[a], u.shape[a]) or m.data.device != u.device
+                    or m.data.dtype != torch.float64):
+                return None
+            if m.offsets != (0,):
+                if poly not in (-1, a):
+                    return None
+                poly = a
+    if poly < 0:
+        return None
+    n = u.shape[poly]
+    cplx = u.is_complex()
+    diags_total = sum(len(tp.mats[poly].offsets) for tp in tpmats)
+    if diags_total > 512 or n > 4096 or n * 17 * (16 if cplx else 8) > 200 * 1024:
+        return None
+    fourier = [a for a in range(nd) if a != poly]
+    x = u.to(torch.complex128 if cplx else torch.float64).contiguous()
+    y = torch.empty_like(x)
+    outer = math.prod(u.shape[:poly])
+    inner = math.prod(u.shape[poly + 1:])
+    nt = len(tpmats)
+    data = [tp.mats[poly].data.contiguous() for tp in tpmats]
+    diags = [tp.mats[a].data.contiguous() for tp in tpmats for a in fourier]
+    _lib.call(
+        "jfb_tp_matvec", nt, (ctypes.c_void_p * nt)(*(d.data_ptr() for d in data)),
+        _lib.int64_array([len(tp.mats[poly].offsets) for tp in tpmats]),
+        _lib.int64_array([o for tp in tpmats for o in tp.mats[poly].offsets]),
+        (ctypes.c_void_p * len(diags))(*(d.data_ptr() for d in diags)), len(fourier),
+        _lib.int64_array([u.shape[a] for a in fourier]),
+        (ctypes.c_double * nt)(*(tp.coefficient for tp in tpmats)), n, outer, inner,
+        x.data_ptr(), y.data_ptr(), int(cplx), _stream(x))
+    return y
+
+
 class TPMatrix:
     """``coefficient * mats[0] (x) mats[1] (x) ...`` (tpmatrix.py:40-200)."""
 
@@ -219,6 +266,10 @@ class TPMatrices:
         self.tpmats = list(tpmats)
 
     def __matmul__(self, u: torch.Tensor) -> torch.Tensor:
+        if u.is_cuda:
+            out = _fused_sum(self.tpmats, u)
+            if out is not None:
+                return out
         out = None
         for tp in self.tpmats:
             r = tp @ u
