@@ -18,12 +18,14 @@
 #include "jfb_kmm_kernels.cuh"
 #include "jfb_kmm_warpk.cuh"
 #include "jfb_kmm_gemm.cuh"
+#include "jfb_kmm_split.cuh"
 #include "jfb_kmm_mhd.cuh"
 #include "jfb_kmm_adjoint.cuh"
 #include "jfb_kmm_ens.cuh"
 
 #ifdef JFB_PHASE_STAMPS
-// Copies the phase stamps (kernel 0: pencil_gemm_kernel, 1: plane_cross_kernel;
+// Copies the phase stamps (kernel 0: pencil_gemm_kernel, 1: plane_cross_kernel,
+// 2: pencil_rhs_kernel, 3: pencil_velocity_kernel;
 // [kernel][cta][phase] global-timer nanoseconds) to host memory.
 extern "C" int jfb_debug_read_stamps(unsigned long long* host, int64_t count) {
   JFB_REQUIRE(host && count > 0 && count <= 4 * jfb::kStampCTAs * jfb::kStampPhases,
@@ -73,53 +75,18 @@ __global__ void assemble_band_kernel(const double* __restrict__ X0,
   }
 }
 
-// Factored band -> packed parity record (see packed_rec_size).
-__global__ void pack_factor_kernel(const double* __restrict__ band, int n_modes, int n,
-                                   int p, int q, double* __restrict__ out) {
-  const int m = blockIdx.x;
-  if (m >= n_modes) return;
-  const int bw = p + q + 1;
-  const double* B = band + (size_t)m * bw * n;
-  double* R = out + (size_t)m * packed_rec_size(n);
-  auto at = [&](int off, int col) { return B[(size_t)(p + off) * n + col]; };
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    R[2 * i] = (i >= 2 && p >= 2) ? at(-2, i - 2) : 0.0;      // L[i, i-2]
-    R[2 * i + 1] = (i >= 4 && p >= 4) ? at(-4, i - 4) : 0.0;  // L[i, i-4]
-  }
-  const int m0 = (n + 1) / 2, m1 = n / 2;
-  double* U0 = R + 2 * n;
-  double* U1 = U0 + m0 * (m0 + 1) / 2;
-  for (int par = 0; par < 2; ++par) {
-    const int mp = par ? m1 : m0;
-    double* Up = par ? U1 : U0;
-    const int tot = mp * (mp + 1) / 2;
-    for (int e = threadIdx.x; e < tot; e += blockDim.x) {
-      // invert e -> (r, c) with e = c(c+1)/2 + r, r <= c
-      int c = (int)floor((sqrt(8.0 * e + 1.0) - 1.0) * 0.5);
-      while (c * (c + 1) / 2 > e) --c;
-      while ((c + 1) * (c + 2) / 2 <= e) ++c;
-      const int r = e - c * (c + 1) / 2;
-      const int row = 2 * r + par, col = 2 * c + par;
-      const int off = col - row;
-      double v = (off <= q) ? at(off, col) : 0.0;
-      if (r == c) v = 1.0 / v;
-      Up[e] = v;
-    }
-  }
-}
-
-// Factored band -> record of the tensor-core pencil stage: the L pairs as in
-// pack_factor_kernel, then per parity class the INVERSE of the upper factor,
-// packed column-major (entry (r, c), r <= c, at c (c + 1) / 2 + r).  Column c
-// is U^-1 e_c by back substitution (diamatrix.py:1936-1973 gives U).
+// Factored band -> factor record (packed_rec_size): the L pairs, then per
+// parity class the INVERSE of the upper factor.  Column c is U^-1 e_c
+// by back substitution (diamatrix.py:1936-1973 gives U); the records are
+// zeroed when they are allocated.
 constexpr int kMaxHalfInv = 64;
 __global__ void pack_factor_inv_kernel(const double* __restrict__ band, int n_modes, int n,
-                                       int p, int q, double* __restrict__ out) {
+                                       int p, int q, bool blocks, double* __restrict__ out) {
   const int mode = blockIdx.x;
   if (mode >= n_modes) return;
   const int bw = p + q + 1;
   const double* B = band + (size_t)mode * bw * n;
-  double* R = out + (size_t)mode * packed_rec_size(n);
+  double* R = out + (size_t)mode * packed_rec_size(n, blocks);
   auto at = [&](int off, int col) { return B[(size_t)(p + off) * n + col]; };
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     R[2 * i] = (i >= 2 && p >= 2) ? at(-2, i - 2) : 0.0;
@@ -128,7 +95,7 @@ __global__ void pack_factor_inv_kernel(const double* __restrict__ band, int n_mo
   const int m0 = (n + 1) / 2, m1 = n / 2;
   for (int par = 0; par < 2; ++par) {
     const int mp = par ? m1 : m0;
-    double* X = R + 2 * n + (par ? m0 * (m0 + 1) / 2 : 0);
+    double* X = R + 2 * n + (par ? inv_class_size(m0, blocks) : 0);
     auto U = [&](int r, int k) { return at(2 * (k - r), 2 * k + par); };
     for (int c = threadIdx.x; c < mp; c += blockDim.x) {
       double x[kMaxHalfInv];
@@ -138,7 +105,7 @@ __global__ void pack_factor_inv_kernel(const double* __restrict__ band, int n_mo
         for (int k = r + 1; k <= c && 2 * (k - r) <= q; ++k) s += U(r, k) * x[k];
         x[r] = -s / U(r, r);
       }
-      for (int r = 0; r <= c; ++r) X[c * (c + 1) / 2 + r] = x[r];
+      for (int r = 0; r <= c; ++r) X[inv_entry(r, c, blocks)] = x[r];
     }
   }
 }
@@ -295,7 +262,9 @@ struct jfb_kmm_plan {
   cudaGraphExec_t graph[3] = {nullptr, nullptr, nullptr};
   cudaStream_t cap = nullptr;  // private stream used only to capture the graphs
   cudaEvent_t* timing_events = nullptr;  // set by jfb_kmm_timed_steps
-  bool gemm = false;       // tensor-core pencil stage (pencil_gemm_kernel)
+  bool gemm = false;       // tensor-core pencil stage (pencil_gemm_kernel, or, split, its
+                           // two-kernel form for grids the one-kernel tile does not fit)
+  bool split = false;
   bool gemm_ok = false, plane_ok = false, tc_ok = false;  // variants this plan can run
   bool pdl = false;        // programmatic dependent launch of the step kernels
   bool plane = false;      // fused periodic-axis transforms (plane_cross_kernel)
@@ -511,14 +480,10 @@ static int build_factor_set(jfb_kmm_plan* pl, double gamma, FactorSet& fs, doubl
       if (st) return cleanup(), st;
     }
     double** dst = (sys == 0) ? &fs.su : (sys == 1) ? &fs.sg : &fs.s00;
-    st = dalloc(pl, (void**)dst, (size_t)modes * packed_rec_size(n) * sizeof(double));
+    st = dalloc(pl, (void**)dst, (size_t)modes * packed_rec_size(n, pl->split) * sizeof(double));
     if (st) return cleanup(), st;
-    if (inv) {
-      JFB_REQUIRE(n <= 2 * kMaxHalfInv, "system too large for the inverse-factor records");
-      pack_factor_inv_kernel<<<modes, 64>>>(dband, modes, n, p, q, *dst);
-    } else {
-      pack_factor_kernel<<<modes, 128>>>(dband, modes, n, p, q, *dst);
-    }
+    JFB_REQUIRE(n <= 2 * kMaxHalfInv, "system too large for the inverse-factor records");
+    pack_factor_inv_kernel<<<modes, 64>>>(dband, modes, n, p, q, pl->split, *dst);
     JFB_CHECK_LAUNCH();
     JFB_CHECK_CUDA(cudaDeviceSynchronize());
     // the temporaries were registered as plan allocations by upload(): release them
@@ -585,9 +550,10 @@ static int launch_pencil(jfb_kmm_plan* pl, const StageArgs& a0, cudaStream_t s) 
   const int blocks = pl->d.Ny * pl->d.nKb;
   StageArgs a = a0;
   a.status = pl->status;
-  // one instantiation per register-row count and nonlinear form
-  auto* k = pl->d.nD <= 64 ? (pl->d.grad ? pencil_stage_kernel<1, 1> : pencil_stage_kernel<1, 0>)
-                           : (pl->d.grad ? pencil_stage_kernel<2, 1> : pencil_stage_kernel<2, 0>);
+  // one instantiation per register-row count, nonlinear form and record layout
+  auto* k = pl->split ? (pl->d.grad ? pencil_stage_kernel<2, 1, true> : pencil_stage_kernel<2, 0, true>)
+            : pl->d.nD <= 64 ? (pl->d.grad ? pencil_stage_kernel<1, 1> : pencil_stage_kernel<1, 0>)
+                             : (pl->d.grad ? pencil_stage_kernel<2, 1> : pencil_stage_kernel<2, 0>);
   k<<<blocks, kNW * 32, pl->smem_pencil, s>>>(pl->ops, pl->d, a);
   JFB_CHECK_LAUNCH();
   return JFB_OK;
@@ -648,6 +614,16 @@ static int launch_implicit(jfb_kmm_plan* pl, const StageArgs& a, cudaStream_t s)
   }
   const GemmStageArgs g = gemm_args(pl, a);
   const int blocks = (pl->d.Ny / 2) * ceil_div(pl->d.Kz, 8);
+  if (pl->split) {
+    const Dims& d = pl->d;
+    const size_t sr = split_rhs_smem(d.Nx, d.nB, d.nD, g.slin != 0.0);
+    JFB_CHECK_CUDA(launch_ex(pl->pdl, d.grad ? pencil_rhs_kernel<1> : pencil_rhs_kernel<0>,
+                             dim3(blocks), dim3(kSThreads), sr, s, d, pl->ops, pl->gops, g));
+    JFB_CHECK_CUDA(launch_ex(pl->pdl, d.grad ? pencil_velocity_kernel<1> : pencil_velocity_kernel<0>,
+                             dim3(blocks), dim3(kSThreads), split_vel_smem(d.nB, d.nD), s, d,
+                             pl->gops, g));
+    return JFB_OK;
+  }
   // the tcgen05 variant exists for the rotational form only
   auto* k = pl->gops.tc ? pencil_gemm_kernel<true, 0>
             : pl->d.grad ? pencil_gemm_kernel<false, 1>
@@ -1380,6 +1356,8 @@ static int create_plan(const jfb_kmm_config* cfg, const jfb_mhd_params* mhd,
     set_error("grid too large for the shared-memory tiling");
     return fail(JFB_ERR_ARG);
   }
+  allow_smem((const void*)pencil_stage_kernel<2, 0, true>);
+  allow_smem((const void*)pencil_stage_kernel<2, 1, true>);
   allow_smem((const void*)pencil_stage_kernel<1, 0>);
   allow_smem((const void*)pencil_stage_kernel<2, 0>);
   allow_smem((const void*)pencil_stage_kernel<1, 1>);
@@ -1511,12 +1489,17 @@ static int create_plan(const jfb_kmm_config* cfg, const jfb_mhd_params* mhd,
     const bool want = !(env && std::string(env) == "warp");
     pl->gemm = smem <= 227 * 1024 && (d.nD + 1) / 2 <= kMaxM && Jl <= kMaxM;
     GemmHost gh;
-    if (pl->gemm) {
+    // the two-kernel form takes what the one-kernel tile does not fit (FP64)
+    const bool two_kernels = !pl->mixed && !pl->mhd && want;
+    if (pl->gemm || two_kernels) {
       std::string err;
-      if (!build_gemm_operators(pl->hop, gh, err, d.grad)) {
+      // (the tcgen05 image of the mixed form needs the dense operators)
+      if (!build_gemm_operators(pl->hop, gh, err, d.grad, pl->mixed)) {
         set_error(err);
         return fail(JFB_ERR_ARG);
       }
+    }
+    if (pl->gemm) {
       // unrolled k ranges and the staged velocity operators must fit
       bool fits = (size_t)G.oVel * kGLd + (gh.frag.size() - gh.off[gA0Ee]) <=
                   (size_t)G.oRU * kGLd;
@@ -1525,7 +1508,14 @@ static int create_plan(const jfb_kmm_config* cfg, const jfb_mhd_params* mhd,
           const int span = gh.krange[gh.kr[k] + 2 * mt + 1] - gh.krange[gh.kr[k] + 2 * mt];
           if ((k <= gNgO && span > kKtN) || (k >= gMuE && k <= gMgO && span > kKtM)) fits = false;
         }
-      pl->gemm = fits;  // otherwise the warp-per-pencil kernel handles this size
+      pl->gemm = fits;
+    }
+    if (!pl->gemm && two_kernels) {
+      bool fits = N <= kSMaxN && split_rhs_smem(N, d.nB, d.nD, true) <= 227 * 1024 &&
+                  split_vel_smem(d.nB, d.nD) <= 113 * 1024;
+      for (int k = 0; k < gNumSub && fits; ++k)  // row tiles of a product over eight warps
+        if (k <= gMgO && gh.mt[k] > kSWarps) fits = false;
+      pl->gemm = pl->split = fits;
     }
     pl->gemm_ok = pl->gemm;
     if (pl->gemm) {
@@ -1533,12 +1523,13 @@ static int create_plan(const jfb_kmm_config* cfg, const jfb_mhd_params* mhd,
       // the CTAs that all read every operator line do not queue on the same
       // L2 slices
       constexpr int kReplicas = 16;
-      std::vector<double> rep((size_t)kReplicas * gh.frag.size());
-      for (int r = 0; r < kReplicas; ++r)
-        std::copy(gh.frag.begin(), gh.frag.end(), rep.begin() + (size_t)r * gh.frag.size());
+      const size_t fb = gh.frag.size() * sizeof(double);
       double *fr, *r3, *x2, *md;
       int* kr;
-      if ((st = upload(pl, &fr, rep))) return fail(st);
+      if ((st = dalloc(pl, (void**)&fr, kReplicas * fb))) return fail(st);
+      JFB_CHECK_CUDA(cudaMemcpy(fr, gh.frag.data(), fb, cudaMemcpyHostToDevice));
+      for (int r = 1; r < kReplicas; ++r)
+        JFB_CHECK_CUDA(cudaMemcpyAsync(fr + r * gh.frag.size(), fr, fb, cudaMemcpyDeviceToDevice));
       if ((st = upload(pl, &kr, gh.krange))) return fail(st);
       if ((st = upload(pl, &r3, gh.R3))) return fail(st);
       if ((st = upload(pl, &x2, gh.X2D))) return fail(st);
@@ -1564,6 +1555,10 @@ static int create_plan(const jfb_kmm_config* cfg, const jfb_mhd_params* mhd,
       G.kt_mg_lin[0] = ceil_div(nDe, 4);
       G.kt_mg_lin[1] = ceil_div(nDo, 4);
       pl->smem_gemm = smem;
+      for (const void* fn : {(const void*)pencil_rhs_kernel<0>, (const void*)pencil_rhs_kernel<1>,
+                             (const void*)pencil_velocity_kernel<0>,
+                             (const void*)pencil_velocity_kernel<1>})
+        JFB_CHECK_CUDA(allow_smem(fn));
       JFB_CHECK_CUDA(allow_smem((const void*)pencil_gemm_kernel<false, 0>));
       JFB_CHECK_CUDA(allow_smem((const void*)pencil_gemm_kernel<false, 1>));
       JFB_CHECK_CUDA(allow_smem((const void*)pencil_gemm_kernel<true, 0>));
@@ -1577,7 +1572,7 @@ static int create_plan(const jfb_kmm_config* cfg, const jfb_mhd_params* mhd,
       const char* tce = std::getenv("JFB200_TC");
       const size_t oTA = (size_t)G.oVel * kGLd * sizeof(double);
       const size_t oTB = (size_t)G.oRU * kGLd * sizeof(double);
-      const bool tc_fit = Jl <= 32 && nBe <= 32 && nBo <= 32 && nDe <= 32 && nDo <= 32 &&
+      const bool tc_fit = !pl->split && Jl <= 32 && nBe <= 32 && nBo <= 32 && nDe <= 32 && nDo <= 32 &&
                           oTA + kTcImgA <= oTB &&
                           oTB + kTcImgB <= (size_t)G.rows * kGLd * sizeof(double) &&
                           (size_t)10 * 32 * kTcStagePitch * sizeof(float) <= (size_t)kTcImgA;
@@ -1683,8 +1678,8 @@ static int create_plan(const jfb_kmm_config* cfg, const jfb_mhd_params* mhd,
 
   // factors: steady SBDF3 and the three IMEXRK3 startup stages
   pl->n_modes = (d.Ny / 2) * d.Kz;
-  pl->su_rec = packed_rec_size(d.nB);
-  pl->sg_rec = packed_rec_size(d.nD);
+  pl->su_rec = packed_rec_size(d.nB, pl->split);
+  pl->sg_rec = packed_rec_size(d.nD, pl->split);
   // records with the explicit inverses of the upper factors (both pencil kernels)
   st = build_factor_set(pl, kSBDF3Implicit * cfg->dt, pl->steady, cfg->nu, 0, 2, true);
   if (st) return fail(st);
@@ -1794,7 +1789,7 @@ extern "C" int jfb_kmm_get_info(const jfb_kmm_plan* pl, jfb_kmm_info* info) {
   const Dims& d = pl->d;
   info->n_pencils = d.P;
   info->device_bytes = pl->device_bytes;
-  info->launches_per_step = pl->mhd ? 5 : pl->plane ? 2 : 4;
+  info->launches_per_step = (pl->mhd ? 5 : pl->plane ? 2 : 4) + (pl->gemm && pl->split ? 1 : 0);
   // stage model: 43 E_s + 18 E_m complex values, E_s = Nx Ny (Nz/2+1), E_m = Nx My (Nz/2+1)
   const int64_t H = d.Nz / 2 + 1;
   const int64_t Es = (int64_t)d.Nx * d.Ny * H, Em = (int64_t)d.Nx * d.My * H;
@@ -3089,7 +3084,7 @@ static bool ensemble_batchable(const jfb_ensemble* e) {
   if (env && std::string(env) == "streams") return false;
   if (e->m.size() > (size_t)kEnsMax) return false;
   for (const jfb_kmm_plan* pl : e->m)
-    if (!pl->mhd || !pl->gemm || pl->py == 0 || pl->py != e->m[0]->py ||
+    if (!pl->mhd || !pl->gemm || pl->split || pl->py == 0 || pl->py != e->m[0]->py ||
         pl->mixed != e->m[0]->mixed)
       return false;
   return true;
@@ -3304,7 +3299,8 @@ extern "C" int jfb_ensemble_info(const jfb_ensemble* e, int32_t* batched,
   if (batched) *batched = e->batched ? 1 : 0;
   if (launches_per_step) {
     int64_t n = 0;
-    for (const jfb_kmm_plan* pl : e->m) n += pl->mhd ? 5 : pl->plane ? 2 : 4;
+    for (const jfb_kmm_plan* pl : e->m)
+      n += (pl->mhd ? 5 : pl->plane ? 2 : 4) + (pl->gemm && pl->split ? 1 : 0);
     *launches_per_step = e->batched ? 5 * (int64_t)e->groups.size() : n;
   }
   return JFB_OK;

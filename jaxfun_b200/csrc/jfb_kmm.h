@@ -114,9 +114,10 @@ std::vector<double> x_map_matrix(const XBasis& xb, int map, int k, int* rows, in
 
 Stencil make_stencil(int N, bool biharmonic, int family = 0);
 // Builds GemmHost from the 1-D operators; returns false (with a message) if a
-// parity property the split relies on does not hold.
+// parity property the split relies on does not hold.  extras: also the dense
+// operators of the MHD stage and of the adjoint (B1 ... GD).
 bool build_gemm_operators(const HostOperators& op, GemmHost& gh, std::string& err,
-                          bool gradient = false);
+                          bool gradient = false, bool extras = true);
 void build_host_operators(const jfb_kmm_config& cfg, HostOperators& op);
 void mode_coefficients(const HostOperators& op, const jfb_kmm_config& cfg, int ky,
                        int kz, double gamma, bool biharmonic, double out[3]);

@@ -100,9 +100,27 @@ struct StageArgs {
   double emf_b0z, emf_b0x;
 };
 
-__host__ __device__ inline int packed_rec_size(int n) {
-  const int m0 = (n + 1) / 2, m1 = n / 2;
-  return 2 * n + m0 * (m0 + 1) / 2 + m1 * (m1 + 1) / 2;
+// Factor record of one wavenumber's system of n unknowns: the unit-lower
+// multipliers L[i, i-2], L[i, i-4] (2 n doubles), then per parity class of m
+// rows the inverse of the upper factor, either by columns (entry (r, c),
+// r <= c, at c (c + 1) / 2 + r; lanes over the rows of a column read
+// consecutively) or, for plans on the two-kernel stage, in blocks: the 8x8
+// blocks on and above the diagonal, block column by block column, each
+// holding per lane the A fragments of its two 8x4 tiles, so that one
+// coalesced 512-byte load per warp feeds two mma.m8n8k4 (zeros below the
+// diagonal and in the padding).
+__host__ __device__ inline int inv_class_size(int m, bool blocks) {
+  const int MT = (m + 7) / 8;
+  return blocks ? MT * (MT + 1) / 2 * 64 : m * (m + 1) / 2;
+}
+// Offset of entry (r, c), r <= c, of a class's inverse.
+__host__ __device__ inline int inv_entry(int r, int c, bool blocks) {
+  if (!blocks) return c * (c + 1) / 2 + r;
+  const int mt = r >> 3, j = c >> 3;
+  return (j * (j + 1) / 2 + mt) * 64 + ((r & 7) * 4 + (c & 3)) * 2 + ((c >> 2) & 1);
+}
+__host__ __device__ inline int packed_rec_size(int n, bool blocks) {
+  return 2 * n + inv_class_size((n + 1) / 2, blocks) + inv_class_size(n / 2, blocks);
 }
 
 // ---------------------------------------------------------------------------
@@ -251,17 +269,16 @@ __device__ __forceinline__ void bmass_solve_lane(const DevOps& o, const Dims& d,
 // row 2r + par (and 2(r+32) + par when m > 32).  Forward elimination with
 // the unit-lower factor (L[i, i-2], L[i, i-4]) passes the solved rows down
 // the lanes with shuffles; then x = U^-1 y with the record's explicit inverse
-// of the parity's upper factor (column-major packed, entry (r, c), r <= c, at
-// c (c + 1) / 2 + r): y_c is broadcast and every lane r <= c accumulates
+// of the parity's upper factor: y_c is broadcast and every lane r <= c accumulates
 // U^-1[r, c] y_c, kSolveChunk columns of the inverse loaded at a time.  Not
 // inlined: the call sites (Su, Sg, S00, two parities each) share one copy in
 // the instruction cache.
-template <int NR>
+template <int NR, bool blocks>
 __device__ __noinline__ void parity_solve_regs(const double* __restrict__ rec, int n, c64* y,
                                                int par, int lane) {
   const int m0 = (n + 1) / 2;
   const int m = par ? n / 2 : m0;
-  const double* __restrict__ Ui = rec + 2 * n + (par ? m0 * (m0 + 1) / 2 : 0);
+  const double* __restrict__ Ui = rec + 2 * n + (par ? inv_class_size(m0, blocks) : 0);
   c64 yr[NR];
   double l1[NR], l2[NR];
 #pragma unroll
@@ -300,7 +317,7 @@ __device__ __noinline__ void parity_solve_regs(const double* __restrict__ rec, i
       for (int cc = 0; cc < kSolveChunk; ++cc) {
         const int c = cc + kSolveChunk * ch;
         const int r = lane + 32 * s;
-        u[s][cc] = (c < m && r <= c) ? __ldg(Ui + c * (c + 1) / 2 + r) : 0.0;
+        u[s][cc] = (c < m && r <= c) ? __ldg(Ui + inv_entry(r, c, blocks)) : 0.0;
       }
 #pragma unroll
     for (int cc = 0; cc < kSolveChunk; ++cc) {
@@ -327,11 +344,11 @@ __device__ __noinline__ void parity_solve_regs(const double* __restrict__ rec, i
 }
 
 // Solve a packed system of size n <= 64 * NR in place on y (both parities).
-template <int NR>
+template <int NR, bool blocks>
 __device__ __forceinline__ void packed_solve_warp(const double* __restrict__ rec, int n,
                                                   c64* y, int lane) {
-  parity_solve_regs<NR>(rec, n, y, 0, lane);
-  parity_solve_regs<NR>(rec, n, y, 1, lane);
+  parity_solve_regs<NR, blocks>(rec, n, y, 0, lane);
+  parity_solve_regs<NR, blocks>(rec, n, y, 1, lane);
 }
 
 // Rows i = lane + 32 t of one pencil (n <= 128: the host limits Nx to 129),
@@ -725,8 +742,9 @@ __device__ JFB_CTA_DMMA_INLINE void cta_forward_dmma(const double* __restrict__ 
 // ---------------------------------------------------------------------------
 // pencil_stage: see file header.  Block = kNW warps, one pencil per warp.
 // ---------------------------------------------------------------------------
-// kForm: 0 rotational, 1 gradient (each compiled without the other's code).
-template <int NR, int kForm>
+// kForm: 0 rotational, 1 gradient (each compiled without the other's code);
+// kBlocks: the layout of the factor records (inv_entry; a runtime flag cost 10 %).
+template <int NR, int kForm, bool kBlocks = false>
 __global__ void __launch_bounds__(256, 1) pencil_stage_kernel(DevOps o, Dims d, StageArgs a) {
   const bool grad = kForm == 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1091,10 +1109,10 @@ __global__ void __launch_bounds__(256, 1) pencil_stage_kernel(DevOps o, Dims d, 
       // ---- solves ----
       const double* rec_u = a.fac.su + (size_t)mode_idx * a.fac.su_rec;
       const double* rec_g = a.fac.sg + (size_t)mode_idx * a.fac.sg_rec;
-      packed_solve_warp<NR>(rec_u, d.nB, A3, lane);
-      packed_solve_warp<NR>(rec_g, d.nD, A4, lane);
+      packed_solve_warp<NR, kBlocks>(rec_u, d.nB, A3, lane);
+      packed_solve_warp<NR, kBlocks>(rec_g, d.nD, A4, lane);
       if (mean_pencil) {
-        packed_solve_warp<NR>(a.fac.s00, d.nD, sVW, lane);
+        packed_solve_warp<NR, kBlocks>(a.fac.s00, d.nD, sVW, lane);
         for (int i = lane; i < d.nD; i += 32) a.vw_out[i] = sVW[i];
         __syncwarp();
       }

@@ -322,11 +322,21 @@ struct LMat {
 };
 LMat mul(const LMat& A, const LMat& B) {
   LMat C(A.r, B.c);
+  // the nonzero columns of each row of B (stencils, weights and derivative
+  // matrices are mostly zeros)
+  std::vector<std::vector<int>> nz(B.r);
+  for (int k = 0; k < B.r; ++k)
+    for (int j = 0; j < B.c; ++j)
+      if (B(k, j) != 0.0L) nz[k].push_back(j);
   for (int i = 0; i < A.r; ++i)
     for (int k = 0; k < A.c; ++k) {
       const LD a = A(i, k);
       if (a == 0.0L) continue;
-      for (int j = 0; j < B.c; ++j) C(i, j) += a * B(k, j);
+      if ((int)nz[k].size() == B.c) {
+        for (int j = 0; j < B.c; ++j) C(i, j) += a * B(k, j);
+      } else {
+        for (int j : nz[k]) C(i, j) += a * B(k, j);
+      }
     }
   return C;
 }
@@ -399,7 +409,7 @@ bool cols_mirror(const LMat& M, int sign_even_col) {
 }  // namespace
 
 bool build_gemm_operators(const HostOperators& op, GemmHost& gh, std::string& err,
-                          bool gradient) {
+                          bool gradient, bool extras) {
   const int N = op.N, nB = op.nB, nD = op.nD;
   const LD pi = std::acos(-1.0L);
   const LD dfx = op.dfx;
@@ -448,7 +458,8 @@ bool build_gemm_operators(const HostOperators& op, GemmHost& gh, std::string& er
   const LMat B2 = mul(mul(V, D), SDt);
   const LMat P1 = mul(B1, F);
   const LMat P2 = mul(B2, F);
-  const LMat A1 = mul(mul(V, D), SBt);  // d/dx of a TB field at the nodes (gradient form)
+  // d/dx of a TB field at the nodes (gradient form)
+  const LMat A1 = gradient ? mul(mul(V, D), SBt) : LMat(N, nB);
   const LMat K0 = from_dense(op.XB0, nB, nB), K2 = from_dense(op.XB2, nB, nB),
              K4 = from_dense(op.XB4, nB, nB);
   const LMat X0D = from_dense(op.XD0, nD, nD), X2D = from_dense(op.XD2, nD, nD);
@@ -562,7 +573,7 @@ bool build_gemm_operators(const HostOperators& op, GemmHost& gh, std::string& er
       for (int k = 0; k < nBo; ++k) gh.mid[5 * gh.mid_stride + k] = (double)A1(j, 2 * k + 1);
   }
 
-  {
+  if (extras) {  // dense operators of the MHD stage and of the adjoint
     const LMat WD2 = mul(WD, D);
     const LMat C1 = mul(mul(mul(mul(V, SDt), MDi), mul(SD, WD)), SDt);
     const LMat C2 = mul(mul(mul(mul(V, SDt), MDi), mul(SD, WD2)), SDt);
