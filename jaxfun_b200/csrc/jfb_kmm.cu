@@ -210,16 +210,40 @@ struct FactorSet {
   double* sg = nullptr;
   double* s00 = nullptr;
   double* s00inv = nullptr;  // explicit inverse of the mean-flow system (tensor-core stage)
-  // factored bands kept for the transposed solves of the adjoint (Su, Sg, S00)
-  double* band[3] = {nullptr, nullptr, nullptr};
-  int bp[3] = {0, 0, 0}, bq[3] = {0, 0, 0};
 };
 
-// Real x-matrices of the adjoint (row-major, forward orientation).
+// x-operators of the adjoint: the reverse stage's half matrices in fragment
+// order, and the real matrices (row-major) of the energy gradient.
 struct AdjOps {
-  double *A0 = nullptr, *F = nullptr, *R0 = nullptr, *R1 = nullptr, *R2 = nullptr,
-         *R3 = nullptr, *B1 = nullptr, *B2 = nullptr, *GB = nullptr, *GD = nullptr,
-         *XB0 = nullptr, *XB2 = nullptr, *XB4 = nullptr, *XD0 = nullptr, *XD2 = nullptr;
+  AdjStageOps st;
+  double *F = nullptr, *GB = nullptr, *GD = nullptr;
+};
+
+// Device buffers of a gain-gradient run (kept by the plan while they are at
+// most kAdjKeep bytes, so that an ascent's repeated calls do not allocate).
+constexpr size_t kAdjKeep = (size_t)4 << 30;
+struct AdjRun {
+  struct Mu {
+    c64 *u, *g, *vw;
+  };
+  std::vector<void*> mem;
+  size_t bytes = 0;
+  int64_t K = 0, nck = 0;
+  c64 *YF, *AH, *AW, *HZ6, *AX, *EU[3];
+  Mu M[4], Q[2][3], S;      // steady ring, the startup stages' solutions, an adjoint state
+  c64* TX = nullptr;        // x-physical fields of the segment's states, K slots
+  c64* recX[2][2];          // and of the two inner stages of the two startup steps
+  c64* X0;                  // and of the explicit initial velocity
+  c64 *IU0, *IU1, *IU2;     // explicit initial leaves
+  std::vector<c64*> ck;     // checkpoints: rings + HX
+  double* dev8 = nullptr;
+  void release() {
+    for (void* p : mem) cudaFree(p);
+    mem.clear();
+    bytes = 0;
+    K = nck = 0;
+  }
+  ~AdjRun() { release(); }
 };
 
 }  // namespace jfb
@@ -284,7 +308,7 @@ struct jfb_kmm_plan {
   // adjoint: operators and kept factor bands, built on first use
   bool adj_ready = false;
   jfb::AdjOps aops;
-  jfb::FactorSet adj_steady, adj_startup[3];
+  jfb::AdjRun adj;
   size_t smem_za = 0;
 };
 
@@ -358,10 +382,9 @@ static std::vector<c64> twiddles(int n) {
 // gamma (tpmatrix.py:1900-2029 assembly, 1105-1149 batched LU).
 // Systems sys_first..sys_last (0: Su, 1: Sg, 2: S00) with diffusivity nu;
 // inv selects the explicit inverse-factor records (always used by the
-// tensor-core pencil stage and the A solves); keep_band keeps the factored
-// band instead of packing it (the adjoint's transposed solves).
+// tensor-core pencil stage and the A solves).
 static int build_factor_set(jfb_kmm_plan* pl, double gamma, FactorSet& fs, double nu,
-                            int sys_first, int sys_last, bool inv, bool keep_band = false) {
+                            int sys_first, int sys_last, bool inv) {
   const HostOperators& op = pl->hop;
   jfb_kmm_config cfg = pl->cfg;
   cfg.nu = nu;
@@ -423,29 +446,6 @@ static int build_factor_set(jfb_kmm_plan* pl, double gamma, FactorSet& fs, doubl
     JFB_CHECK_LAUNCH();
     st = jfb_banded_lu_factor(dband, modes, p, q, n, nullptr);
     if (st) return cleanup(), st;
-    if (keep_band) {
-      fs.band[sys] = dband;
-      fs.bp[sys] = p;
-      fs.bq[sys] = q;
-      pl->allocs.push_back(dband);
-      pl->device_bytes += (int64_t)(band_elems * sizeof(double));
-      dband = nullptr;
-      JFB_CHECK_CUDA(cudaDeviceSynchronize());
-      for (void* ptr : {(void*)dX0, (void*)dX2, (void*)dX4, (void*)dcoef}) {
-        if (!ptr) continue;
-        for (size_t k = 0; k < pl->allocs.size(); ++k)
-          if (pl->allocs[k] == ptr) {
-            pl->allocs.erase(pl->allocs.begin() + k);
-            break;
-          }
-      }
-      pl->device_bytes -= (int64_t)(X0.size() + X2.size() + (bih ? op.XB4.size() : 0) +
-                                    coef.size()) *
-                          sizeof(double);
-      cleanup();
-      dX0 = dX2 = dX4 = dcoef = nullptr;
-      continue;
-    }
     if (sys == 2 && inv) {
       // dense S00 = X0 - gamma nu X2 inverted in long double (Gauss-Jordan,
       // partial pivoting); rows of one parity stay within that parity
@@ -1025,8 +1025,8 @@ static int steady_step_timed(jfb_kmm_plan* pl, int64_t m, cudaStream_t s, cudaEv
 }
 
 // One IMEXRK3 startup step (_step_sbdf3 startup branch).
-// rec (optional): receives the stage states after stages 0 and 1 as
-// (u0, g, vw) of stage 1 then of stage 2 (the adjoint's linearisation points).
+// rec (optional): receives the x-physical fields after stages 0 and 1 (the
+// adjoint's linearisation points).
 static int startup_step(jfb_kmm_plan* pl, cudaStream_t s, c64* const* rec = nullptr) {
   const int64_t m = pl->n;
   const int c = slot(m), nw = slot(m + 1);
@@ -1086,15 +1086,9 @@ static int startup_step(jfb_kmm_plan* pl, cudaStream_t s, c64* const* rec = null
       m.XB = x_field(pl, 6);
       if ((st = launch_mhd(pl, m, s))) return st;
     }
-    if (rec && rk < 2) {
-      const size_t P = pl->d.P;
-      JFB_CHECK_CUDA(cudaMemcpyAsync(rec[3 * rk], pl->U0[nw], (size_t)pl->d.nB * P * sizeof(c64),
+    if (rec && rk < 2)
+      JFB_CHECK_CUDA(cudaMemcpyAsync(rec[rk], pl->X, (size_t)6 * pl->d.Nx * pl->d.P * sizeof(c64),
                                      cudaMemcpyDeviceToDevice, s));
-      JFB_CHECK_CUDA(cudaMemcpyAsync(rec[3 * rk + 1], pl->G[nw], (size_t)pl->d.nD * P * sizeof(c64),
-                                     cudaMemcpyDeviceToDevice, s));
-      JFB_CHECK_CUDA(cudaMemcpyAsync(rec[3 * rk + 2], pl->VW[nw], (size_t)pl->d.nD * sizeof(c64),
-                                     cudaMemcpyDeviceToDevice, s));
-    }
     st = launch_transforms(pl, s);
     if (st) return st;
   }
@@ -2260,30 +2254,12 @@ extern "C" int jfb_mhd_diagnostics(jfb_kmm_plan* pl, double* out, void* stream) 
 
 namespace jfb {
 
-struct AState {
-  c64 *u = nullptr, *g = nullptr, *v = nullptr, *w = nullptr;  // v, w: mean column only
-};
-
-struct AdjRun {
-  std::vector<void*> mem;
-  c64 *XF, *YF, *AH, *AW, *HZ6, *AX, *U1w, *U2w, *EU[3];
-  AState S[4], Nn[4], MU, Z, NZ[3];
-  int K = 0;
-  c64 *TU0, *TG, *TVW;          // states of the segment being reversed, K + 1 slots
-  c64* rec[2][6];               // stage states of the two startup steps
-  c64 *IU0, *IU1, *IU2, *IG;    // explicit initial leaves
-  std::vector<c64*> ck;         // checkpoints: rings + HX
-  size_t ck_elems = 0;
-  ~AdjRun() {
-    for (void* p : mem) cudaFree(p);
-  }
-  int alloc(c64** p, size_t elems) {
-    JFB_CHECK_CUDA(cudaMalloc((void**)p, std::max<size_t>(1, elems) * sizeof(c64)));
-    JFB_CHECK_CUDA(cudaMemset(*p, 0, std::max<size_t>(1, elems) * sizeof(c64)));
-    mem.push_back(*p);
-    return JFB_OK;
-  }
-};
+static size_t checkpoint_elems(const jfb_kmm_plan* pl) {
+  const Dims& d = pl->d;
+  const size_t P = d.P;
+  return 3 * (2 * (size_t)d.nB * P + 2 * (size_t)d.nD * P + 2 * (size_t)d.nD) +
+         (size_t)3 * d.Nx * P;
+}
 
 static int adj_prepare(jfb_kmm_plan* pl) {
   if (pl->adj_ready) return JFB_OK;
@@ -2294,41 +2270,159 @@ static int adj_prepare(jfb_kmm_plan* pl) {
     set_error(err);
     return JFB_ERR_ARG;
   }
-  AdjOps& A = pl->aops;
   const HostOperators& op = pl->hop;
+  AdjOps& A = pl->aops;
+  AdjStageOps& G = A.st;
+  const int N = d.Nx, nB = d.nB, nD = d.nD;
+  G.Jh = (N + 1) / 2;
+  G.Jl = N / 2;
+  G.nBe = (nB + 1) / 2;
+  G.nBo = nB / 2;
+  G.nDe = (nD + 1) / 2;
+  G.nDo = nD / 2;
+  std::vector<double> frag;
+  std::vector<int> krange;
+  auto add = [&](int id, int R, int K, auto val) {
+    const int MT = (R + 7) / 8, KT = (K + 3) / 4;
+    G.sub[id] = SubDesc{(int)frag.size(), MT, KT, (int)krange.size()};
+    for (int mt = 0; mt < MT; ++mt) {
+      int kb = KT, ke = 0;
+      for (int kt = 0; kt < KT; ++kt)
+        for (int lane = 0; lane < 32; ++lane) {
+          const int r = mt * 8 + lane / 4, k = kt * 4 + lane % 4;
+          const double v = (r < R && k < K) ? val(r, k) : 0.0;
+          frag.push_back(v);
+          if (v != 0.0) {
+            kb = std::min(kb, kt);
+            ke = std::max(ke, kt + 1);
+          }
+        }
+      if (ke == 0) kb = 0;
+      krange.push_back(kb);
+      krange.push_back(ke);
+    }
+  };
+  auto at = [](const std::vector<double>& M, int cols, int i, int j) { return M[(size_t)i * cols + j]; };
+  const int Jh = G.Jh, Jl = G.Jl;
+  // inputs of the transposed velocity operators: mirror sums in rows j <= Jl
+  // (the middle node last), differences in row N-1-j, i.e. Jl-1-k of base Jh
+  add(qA0E, G.nBe, Jh, [&](int r, int k) { return at(gh.A0, nB, k, 2 * r); });
+  add(qA0O, G.nBo, Jl, [&](int r, int k) { return at(gh.A0, nB, Jl - 1 - k, 2 * r + 1); });
+  add(qB1E, G.nDe, Jh, [&](int r, int k) { return at(gh.B1, nD, k, 2 * r); });
+  add(qB1O, G.nDo, Jl, [&](int r, int k) { return at(gh.B1, nD, Jl - 1 - k, 2 * r + 1); });
+  add(qB2E, G.nDe, Jl, [&](int r, int k) { return at(gh.B2, nD, Jl - 1 - k, 2 * r); });
+  add(qB2O, G.nDo, Jh, [&](int r, int k) { return at(gh.B2, nD, k, 2 * r + 1); });
+  add(qFE, G.nBe, G.nDo, [&](int r, int k) { return at(gh.F, nB, 2 * k + 1, 2 * r); });
+  add(qFO, G.nBo, G.nDe, [&](int r, int k) { return at(gh.F, nB, 2 * k, 2 * r + 1); });
+  auto half = [&](const std::vector<double>& M, int n, int par) {
+    return [&M, n, par](int r, int k) { return M[(size_t)(2 * k + par) * n + 2 * r + par]; };
+  };
+  add(qK0E, G.nBe, G.nBe, half(op.XB0, nB, 0));
+  add(qK0O, G.nBo, G.nBo, half(op.XB0, nB, 1));
+  add(qK2E, G.nBe, G.nBe, half(op.XB2, nB, 0));
+  add(qK2O, G.nBo, G.nBo, half(op.XB2, nB, 1));
+  add(qK4E, G.nBe, G.nBe, half(op.XB4, nB, 0));
+  add(qK4O, G.nBo, G.nBo, half(op.XB4, nB, 1));
+  add(qD0E, G.nDe, G.nDe, half(op.XD0, nD, 0));
+  add(qD0O, G.nDo, G.nDo, half(op.XD0, nD, 1));
+  add(qD2E, G.nDe, G.nDe, half(op.XD2, nD, 0));
+  add(qD2O, G.nDo, G.nDo, half(op.XD2, nD, 1));
+  auto rows = [&](const std::vector<double>& M, int par) {
+    return [&M, N, par](int j, int k) { return M[(size_t)(2 * k + par) * N + j]; };
+  };
+  add(qR0E, Jh, G.nBe, rows(gh.R0, 0));
+  add(qR0O, Jh, G.nBo, rows(gh.R0, 1));
+  add(qR1E, Jh, G.nBe, rows(gh.R1, 0));
+  add(qR1O, Jh, G.nBo, rows(gh.R1, 1));
+  add(qR2E, Jh, G.nDe, rows(gh.R2, 0));
+  add(qR2O, Jh, G.nDo, rows(gh.R2, 1));
   int st;
-#define UPA(field, vec) \
-  if ((st = upload(pl, &A.field, vec))) return st;
-  UPA(A0, gh.A0);
-  UPA(F, gh.F);
-  UPA(R0, gh.R0);
-  UPA(R1, gh.R1);
-  UPA(R2, gh.R2);
-  UPA(R3, gh.R3);
-  UPA(B1, gh.B1);
-  UPA(B2, gh.B2);
-  UPA(GB, gh.GB);
-  UPA(GD, gh.GD);
-  UPA(XB0, op.XB0);
-  UPA(XB2, op.XB2);
-  UPA(XB4, op.XB4);
-  UPA(XD0, op.XD0);
-  UPA(XD2, op.XD2);
-#undef UPA
-  const double nu = pl->cfg.nu, dt = pl->cfg.dt;
-  if ((st = build_factor_set(pl, kSBDF3Implicit * dt, pl->adj_steady, nu, 0, 2, false, true)))
-    return st;
-  for (int rk = 0; rk < 3; ++rk)
-    if ((st = build_factor_set(pl, (kRK3A[rk] + kRK3B[rk]) * dt / 2.0, pl->adj_startup[rk], nu,
-                               0, 2, false, true)))
-      return st;
+  double *fr, *r3, *x0, *x2;
+  int* kr;
+  if ((st = upload(pl, &fr, frag))) return st;
+  if ((st = upload(pl, &kr, krange))) return st;
+  if ((st = upload(pl, &r3, gh.R3))) return st;
+  if ((st = upload(pl, &x0, op.XD0))) return st;
+  if ((st = upload(pl, &x2, op.XD2))) return st;
+  G.frag = fr;
+  G.krange = kr;
+  G.R3 = r3;
+  G.XD0 = x0;
+  G.XD2 = x2;
+  if ((st = upload(pl, &A.F, gh.F))) return st;
+  if ((st = upload(pl, &A.GB, gh.GB))) return st;
+  if ((st = upload(pl, &A.GD, gh.GD))) return st;
   pl->smem_za = (size_t)2 * d.Mz * kZRows * 5 * sizeof(c64);
   if (pl->smem_za > 227 * 1024) {
     set_error("grid too large for the adjoint z stage");
     return JFB_ERR_ARG;
   }
   JFB_CHECK_CUDA(allow_smem((const void*)z_adjoint_kernel));
+  JFB_CHECK_CUDA(allow_smem((const void*)adj_stage_kernel));
   pl->adj_ready = true;
+  return JFB_OK;
+}
+
+// The run's buffers for T steps in segments of K (zeroed once: the Nyquist
+// rows of the spectra are never written).
+static int adj_buffers(jfb_kmm_plan* pl, int64_t K, int64_t nck) {
+  AdjRun& R = pl->adj;
+  if (R.K == K && R.nck == nck) return JFB_OK;
+  R.release();
+  const Dims& d = pl->d;
+  const size_t P = d.P, nBP = (size_t)d.nB * P, nDP = (size_t)d.nD * P;
+  const size_t f = (size_t)d.Nx * P, fm = (size_t)d.Nx * d.My * d.Kz;
+  auto al = [&](c64** p, size_t n) -> int {
+    const size_t bytes = std::max<size_t>(1, n) * sizeof(c64);
+    JFB_CHECK_CUDA(cudaMalloc((void**)p, bytes));
+    R.mem.push_back(*p);
+    R.bytes += bytes;
+    JFB_CHECK_CUDA(cudaMemset(*p, 0, bytes));
+    return JFB_OK;
+  };
+  auto all = [&]() -> int {
+    int st;
+#define AL(p, n) \
+  if ((st = al(&(p), (n)))) return st;
+    AL(R.YF, 6 * fm);
+    AL(R.AH, 3 * f);
+    AL(R.AW, 3 * fm);
+    AL(R.HZ6, 6 * fm);
+    AL(R.AX, 6 * f);
+    AL(R.EU[0], nBP);
+    AL(R.EU[1], nDP);
+    AL(R.EU[2], nDP);
+    std::vector<AdjRun::Mu*> mus = {&R.S};
+    for (auto& m : R.M) mus.push_back(&m);
+    for (auto& q : R.Q)
+      for (auto& m : q) mus.push_back(&m);
+    for (AdjRun::Mu* m : mus) {
+      AL(m->u, nBP);
+      AL(m->g, nDP);
+      AL(m->vw, d.nD);
+    }
+    AL(R.TX, (size_t)K * 6 * f);
+    for (auto& r : R.recX)
+      for (auto& x : r) AL(x, 6 * f);
+    AL(R.X0, 6 * f);
+    AL(R.IU0, nBP);
+    AL(R.IU1, nDP);
+    AL(R.IU2, nDP);
+    R.ck.assign(nck, nullptr);
+    for (auto& c : R.ck) AL(c, checkpoint_elems(pl));
+    c64* dv;
+    AL(dv, 5);
+    R.dev8 = (double*)dv;
+#undef AL
+    return JFB_OK;
+  };
+  const int st = all();
+  if (st) {
+    R.release();
+    return st;
+  }
+  R.K = K;
+  R.nck = nck;
   return JFB_OK;
 }
 
@@ -2371,186 +2465,109 @@ static int run(jfb_kmm_plan* pl, const PTermList& L, cudaStream_t s) {
 #define JFB_RUN(L) \
   if ((st = run(pl, L, s))) return st;
 
-// explicit adjoint (a_u0, a_u1, a_u2) = pro^H (adjoint of the six x-physical
-// fields u, omega of the prologue map)
-static int adj_pro(jfb_kmm_plan* pl, AdjRun& R, cudaStream_t s) {
-  const Dims& d = pl->d;
-  const AdjOps& A = pl->aops;
-  const size_t f = (size_t)d.Nx * d.P;
-  const c64* X = R.AX;
-  const int N = d.Nx;
-  int st;
-  PTermList L = tlist(R.EU[0], d.nB, false);
-  term(L, X + 0 * f, A.A0, N, 1, 1, 0);
-  term(L, X + 4 * f, A.A0, N, 1, 0, -1, 0, 1);  // -i kz
-  term(L, X + 5 * f, A.A0, N, 1, 0, 1, 1, 0);   // +i ky
-  JFB_RUN(L);
-  L = tlist(R.EU[1], d.nD, false);
-  term(L, X + 1 * f, A.B1, N, 1, 1, 0);
-  term(L, X + 3 * f, A.B1, N, 1, 0, 1, 0, 1);  // +i kz
-  term(L, X + 5 * f, A.B2, N, 1, 1, 0);
-  JFB_RUN(L);
-  L = tlist(R.EU[2], d.nD, false);
-  term(L, X + 2 * f, A.B1, N, 1, 1, 0);
-  term(L, X + 3 * f, A.B1, N, 1, 0, -1, 1, 0);  // -i ky
-  term(L, X + 4 * f, A.B2, N, 1, -1, 0);
-  JFB_RUN(L);
-  return JFB_OK;
-}
-
-// dst (+)= recon^H (EU): reconstruct_velocity (channelflow_kmm.py:855-870)
-static int adj_recon(jfb_kmm_plan* pl, AdjRun& R, const AState& dst, bool acc, cudaStream_t s) {
+// dst = recon^H EU: reconstruct_velocity (channelflow_kmm.py:855-870); the
+// mean flow's part is the real (0, 0) column of EU1, EU2.
+static int adj_recon(jfb_kmm_plan* pl, AdjRun& R, const AdjRun::Mu& dst, cudaStream_t s) {
   const Dims& d = pl->d;
   const AdjOps& A = pl->aops;
   int st;
-  PTermList L = tlist(dst.u, d.nB, acc);
+  PTermList L = tlist(dst.u, d.nB, false);
   term(L, R.EU[0], nullptr, d.nB, 0, 1, 0);
   term(L, R.EU[1], A.F, d.nD, 1, 0, -1, 1, 0, -1);  // -i ky / k^2
   term(L, R.EU[2], A.F, d.nD, 1, 0, -1, 0, 1, -1);  // -i kz / k^2
   JFB_RUN(L);
-  L = tlist(dst.g, d.nD, acc);
+  L = tlist(dst.g, d.nD, false);
   term(L, R.EU[1], nullptr, d.nD, 0, 0, -1, 0, 1, -1);  // -i kz / k^2
   term(L, R.EU[2], nullptr, d.nD, 0, 0, 1, 1, 0, -1);   // +i ky / k^2
   JFB_RUN(L);
-  L = tlist(dst.v, d.nD, acc);
-  term(L, R.EU[1], nullptr, d.nD, 0, 1, 0, 0, 0, 0, 2, 1);
-  JFB_RUN(L);
-  L = tlist(dst.w, d.nD, acc);
-  term(L, R.EU[2], nullptr, d.nD, 0, 1, 0, 0, 0, 0, 2, 1);
-  JFB_RUN(L);
-  return JFB_OK;
+  LayoutJobs J = layout_jobs(d);
+  add_pair(J, R.EU[1], R.EU[2], (int64_t)2 * d.P, dst.vw);
+  return run_layout(J, true, s);
 }
 
-// AH = R_n^H mu: adjoint of the nonlinear rows (channelflow_kmm.py:810-829)
-static int adj_rows(jfb_kmm_plan* pl, AdjRun& R, const AState& mu, cudaStream_t s) {
+// y transforms of the reverse sweep (nf fields, FP64).
+static int adj_y(jfb_kmm_plan* pl, bool backward, int nf, const c64* in, c64* out,
+                 cudaStream_t s) {
   const Dims& d = pl->d;
-  const AdjOps& A = pl->aops;
-  const size_t f = (size_t)d.Nx * d.P;
-  const double myz = d.Myz;
-  int st;
-  PTermList L = tlist(R.AH, d.Nx, false);
-  term(L, mu.u, A.R0, d.nB, 1, myz, 0, 0, 0, 1);  // Myz k^2
-  JFB_RUN(L);
-  L = tlist(R.AH + f, d.Nx, false);
-  term(L, mu.u, A.R1, d.nB, 1, 0, -myz, 1, 0);  // -i ky Myz
-  term(L, mu.g, A.R2, d.nD, 1, 0, -myz, 0, 1);  // -i kz Myz
-  term(L, mu.v, A.R3, d.nD, 1, -1, 0, 0, 0, 0, 2, 1);
-  JFB_RUN(L);
-  L = tlist(R.AH + 2 * f, d.Nx, false);
-  term(L, mu.u, A.R1, d.nB, 1, 0, -myz, 0, 1);  // -i kz Myz
-  term(L, mu.g, A.R2, d.nD, 1, 0, myz, 1, 0);   // +i ky Myz
-  term(L, mu.w, A.R3, d.nD, 1, -1, 0, 0, 0, 0, 2, 1);
-  JFB_RUN(L);
-  return JFB_OK;
-}
-
-// dst += cm (M + gamma L)^T mu, gl = gamma nu (mass rows channelflow_kmm.py:261-409)
-static int adj_mass(jfb_kmm_plan* pl, const AState& mu, double cm, double gl, const AState& dst,
-                    cudaStream_t s) {
-  const Dims& d = pl->d;
-  const AdjOps& A = pl->aops;
-  const double m = cm * d.Myz;
-  int st;
-  PTermList L = tlist(dst.u, d.nB, true);
-  term(L, mu.u, A.XB0, d.nB, 1, -m, 0, 0, 0, 1);
-  term(L, mu.u, A.XB0, d.nB, 1, m * gl, 0, 0, 0, 2);
-  term(L, mu.u, A.XB2, d.nB, 1, m, 0);
-  term(L, mu.u, A.XB2, d.nB, 1, -2.0 * m * gl, 0, 0, 0, 1);
-  term(L, mu.u, A.XB4, d.nB, 1, m * gl, 0);
-  JFB_RUN(L);
-  L = tlist(dst.g, d.nD, true);
-  term(L, mu.g, A.XD0, d.nD, 1, m, 0);
-  term(L, mu.g, A.XD0, d.nD, 1, -m * gl, 0, 0, 0, 1);
-  term(L, mu.g, A.XD2, d.nD, 1, m * gl, 0);
-  JFB_RUN(L);
-  for (int k = 0; k < 2; ++k) {
-    c64* out = k ? dst.w : dst.v;
-    const c64* in = k ? mu.w : mu.v;
-    L = tlist(out, d.nD, true);
-    term(L, in, A.XD0, d.nD, 1, cm, 0, 0, 0, 0, 2);
-    term(L, in, A.XD2, d.nD, 1, cm * gl, 0, 0, 0, 0, 2);
-    JFB_RUN(L);
+  if (pl->py) {
+    const dim3 g(d.Nx, nf, ceil_div(d.Kz, pl->KCw));
+    const size_t sm = backward ? pl->smem_yw_b : pl->smem_yw_f;
+    switch (pl->py) {
+#define JFB_AY(P)                                                                           \
+  case P:                                                                                   \
+    if (backward) y_backward_warp_kernel<P, double><<<g, 256, sm, s>>>(d, pl->KCw, pl->twy, in, out); \
+    else y_forward_warp_kernel<P, double><<<g, 256, sm, s>>>(d, pl->KCw, pl->twy, in, out, nullptr);  \
+    break;
+      JFB_AY(2) JFB_AY(3) JFB_AY(4) JFB_AY(6)
+#undef JFB_AY
+    }
+  } else {
+    const dim3 g(d.Nx, nf, d.Kz / pl->KC);
+    if (backward)
+      y_backward_kernel<double><<<g, 256, pl->smem_y, s>>>(d, pl->fy, pl->KC, pl->twy, in, out);
+    else
+      y_forward_kernel<double><<<g, 256, pl->smem_y, s>>>(d, pl->fy, pl->KC, pl->twy, in, out, nullptr);
   }
-  return JFB_OK;
-}
-
-// dst = S^-T src with the kept factor bands
-static int adj_solve(jfb_kmm_plan* pl, const FactorSet& fs, const AState& src, const AState& dst,
-                     cudaStream_t s) {
-  const Dims& d = pl->d;
-  // a warp per pencil (kBandWarps pencils per block), the vector in shared memory
-  const int blocks = ceil_div(d.P, kBandWarps);
-  const size_t smB = (size_t)kBandWarps * d.nB * sizeof(c64), smD = (size_t)kBandWarps * d.nD * sizeof(c64);
-  band_solve_t_warp_kernel<<<blocks, 32 * kBandWarps, smB, s>>>(d, fs.band[0], fs.bp[0], fs.bq[0],
-                                                                d.nB, 0, src.u, dst.u);
-  band_solve_t_warp_kernel<<<blocks, 32 * kBandWarps, smD, s>>>(d, fs.band[1], fs.bp[1], fs.bq[1],
-                                                                d.nD, 0, src.g, dst.g);
-  band_solve_t_warp_kernel<<<1, 32 * kBandWarps, smD, s>>>(d, fs.band[2], fs.bp[2], fs.bq[2], d.nD,
-                                                           1, src.v, dst.v);
-  band_solve_t_warp_kernel<<<1, 32 * kBandWarps, smD, s>>>(d, fs.band[2], fs.bp[2], fs.bq[2], d.nD,
-                                                           1, src.w, dst.w);
   JFB_CHECK_LAUNCH();
   return JFB_OK;
 }
 
-static void astate_axpy(const jfb_kmm_plan* pl, const AState& y, const AState& x, double a,
-                        cudaStream_t s) {
-  const Dims& d = pl->d;
-  const size_t P = d.P;
-  axpy_kernel<<<256, 256, 0, s>>>(y.u, x.u, a, (size_t)d.nB * P);
-  axpy_kernel<<<256, 256, 0, s>>>(y.g, x.g, a, (size_t)d.nD * P);
-  axpy_kernel<<<64, 256, 0, s>>>(y.v, x.v, a, (size_t)d.nD * P);
-  axpy_kernel<<<64, 256, 0, s>>>(y.w, x.w, a, (size_t)d.nD * P);
-}
-
-static int astate_zero(const jfb_kmm_plan* pl, const AState& y, cudaStream_t s) {
-  const Dims& d = pl->d;
-  const size_t P = d.P;
-  JFB_CHECK_CUDA(cudaMemsetAsync(y.u, 0, (size_t)d.nB * P * sizeof(c64), s));
-  JFB_CHECK_CUDA(cudaMemsetAsync(y.g, 0, (size_t)d.nD * P * sizeof(c64), s));
-  JFB_CHECK_CUDA(cudaMemsetAsync(y.v, 0, (size_t)d.nD * P * sizeof(c64), s));
-  JFB_CHECK_CUDA(cudaMemsetAsync(y.w, 0, (size_t)d.nD * P * sizeof(c64), s));
-  return JFB_OK;
-}
-
-// EU = J^H mu at a linearisation point: the state (u0, g, vw) or, with u1
-// and u2 given, the explicit velocity (u0, u1, u2).
-static int adj_nonlinear(jfb_kmm_plan* pl, AdjRun& R, const c64* u0, const c64* g, const c64* vw,
-                         const c64* u1, const c64* u2, const AState& mu, cudaStream_t s) {
+// AX = adjoint of the x-physical fields at the linearisation point X for the
+// nonlinear rows' adjoint AH.
+static int adj_linearise(jfb_kmm_plan* pl, AdjRun& R, const c64* X, cudaStream_t s) {
   const Dims& d = pl->d;
   int st;
-  if (!u1) {
-    StageArgs a = blank_args();
-    a.mode = kReconstruct;
-    a.u0a = u0;
-    a.ga = g;
-    a.vwa = vw;
-    a.X = R.U1w;
-    a.Hd_out = R.U2w;
-    if ((st = launch_pencil(pl, a, s))) return st;
-    u1 = R.U1w;
-    u2 = R.U2w;
+  if ((st = adj_y(pl, true, 6, X, R.YF, s))) return st;
+  if ((st = adj_y(pl, true, 3, R.AH, R.AW, s))) return st;
+  const int wb = ceil_div((int64_t)d.Nx * d.My, 8);
+  switch (pl->pz * 10 + pl->qk) {
+#define JFB_ZA(P, Q)                                                                             \
+  case P * 10 + Q:                                                                               \
+    z_adjoint_warp_kernel<P, Q><<<wb, 256, 0, s>>>(pl->ops, d, pl->twz, R.YF, R.AW, R.HZ6); \
+    break;
+    JFB_ZA(2, 1) JFB_ZA(2, 2) JFB_ZA(3, 1) JFB_ZA(3, 2) JFB_ZA(4, 1) JFB_ZA(4, 2)
+#undef JFB_ZA
+    default:  // other lengths (and six points per lane: too many registers)
+      z_adjoint_kernel<<<ceil_div((int64_t)d.Nx * d.My, kZRows), 256, pl->smem_za, s>>>(
+          pl->ops, d, pl->fz, pl->twz, R.YF, R.AW, R.HZ6);
   }
-  StageArgs a = blank_args();
-  a.mode = kPrologue;
-  a.pu0 = u0;
-  a.pu1 = u1;
-  a.pu2 = u2;
-  a.X = R.XF;
-  if ((st = launch_pencil(pl, a, s))) return st;
-  dim3 gy6(d.Nx, 6, d.Kz / pl->KC), gy3(d.Nx, 3, d.Kz / pl->KC);
-  y_backward_kernel<double><<<gy6, 256, pl->smem_y, s>>>(d, pl->fy, pl->KC, pl->twy, R.XF, R.YF);
   JFB_CHECK_LAUNCH();
-  if ((st = adj_rows(pl, R, mu, s))) return st;
-  y_backward_kernel<double><<<gy3, 256, pl->smem_y, s>>>(d, pl->fy, pl->KC, pl->twy, R.AH, R.AW);
+  return adj_y(pl, false, 6, R.HZ6, R.AX, s);
+}
+
+static AdjStageArgs adj_args(const AdjRun& R, bool ax) {
+  AdjStageArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.AX = ax ? R.AX : nullptr;
+  return a;
+}
+static void adj_mu(AdjStageArgs& a, const AdjRun::Mu& m, double cm, double gl, double cn) {
+  a.mu[a.nmu++] = AdjMu{m.u, m.g, m.vw, cm, gl, cn};
+}
+// Runs a stage; with factors, solves into `out` and forms AH with cn_new.
+static int adj_stage(jfb_kmm_plan* pl, AdjRun& R, AdjStageArgs& a, const FactorSet* fs,
+                     double cn_new, const AdjRun::Mu* out, cudaStream_t s) {
+  const Dims& d = pl->d;
+  if (out) {
+    a.out_u = out->u;
+    a.out_g = out->g;
+    a.out_vw = out->vw;
+  }
+  if (fs) {
+    a.solve = 1;
+    a.su = fs->su;
+    a.sg = fs->sg;
+    a.s00inv = fs->s00inv;
+    a.su_rec = pl->su_rec;
+    a.sg_rec = pl->sg_rec;
+    a.blocks = pl->split;
+    a.cn_new = cn_new;
+    a.AH = R.AH;
+  }
+  adj_stage_kernel<<<(d.Ny / 2) * ceil_div(d.Kz, 8), kSThreads, adj_smem(d.Nx, d.nB, d.nD), s>>>(
+      d, pl->aops.st, a);
   JFB_CHECK_LAUNCH();
-  const int zb = ceil_div((int64_t)d.Nx * d.My, kZRows);
-  z_adjoint_kernel<<<zb, 256, pl->smem_za, s>>>(pl->ops, d, pl->fz, pl->twz, R.YF, R.AW, R.HZ6);
-  JFB_CHECK_LAUNCH();
-  y_forward_kernel<double><<<gy6, 256, pl->smem_y, s>>>(d, pl->fy, pl->KC, pl->twy, R.HZ6, R.AX,
-                                                        nullptr);
-  JFB_CHECK_LAUNCH();
-  return adj_pro(pl, R, s);
+  return JFB_OK;
 }
 
 // EU (+)= scale G u (gradient of the perturbation energy, 2 Ly Lz G u)
@@ -2604,34 +2621,14 @@ static int checkpoint_io(jfb_kmm_plan* pl, c64* buf, bool save, cudaStream_t s) 
   return io(pl->HX, (size_t)3 * d.Nx * P);
 }
 
-static size_t checkpoint_elems(const jfb_kmm_plan* pl) {
-  const Dims& d = pl->d;
-  const size_t P = d.P;
-  return 3 * (2 * (size_t)d.nB * P + 2 * (size_t)d.nD * P + 2 * (size_t)d.nD) +
-         (size_t)3 * d.Nx * P;
-}
-
 // One forward step from ring position pl->n (startup while hist < 2),
-// recording the startup stage states when rec is given.
+// recording the startup stages' fields when rec is given.
 static int forward_step(jfb_kmm_plan* pl, cudaStream_t s, c64* const* rec) {
   int st = (pl->hist < 2) ? startup_step(pl, s, rec) : steady_step(pl, pl->n, s);
   if (st) return st;
   pl->n += 1;
   if (pl->hist < 2) pl->hist += 1;
   pl->explicit_u12 = false;
-  return JFB_OK;
-}
-
-static int record_state(jfb_kmm_plan* pl, AdjRun& R, int slot_idx, cudaStream_t s) {
-  const Dims& d = pl->d;
-  const size_t P = d.P;
-  const int c = slot(pl->n);
-  JFB_CHECK_CUDA(cudaMemcpyAsync(R.TU0 + (size_t)slot_idx * d.nB * P, pl->U0[c],
-                                 (size_t)d.nB * P * sizeof(c64), cudaMemcpyDeviceToDevice, s));
-  JFB_CHECK_CUDA(cudaMemcpyAsync(R.TG + (size_t)slot_idx * d.nD * P, pl->G[c],
-                                 (size_t)d.nD * P * sizeof(c64), cudaMemcpyDeviceToDevice, s));
-  JFB_CHECK_CUDA(cudaMemcpyAsync(R.TVW + (size_t)slot_idx * d.nD, pl->VW[c], (size_t)d.nD * sizeof(c64),
-                                 cudaMemcpyDeviceToDevice, s));
   return JFB_OK;
 }
 
@@ -2652,7 +2649,13 @@ extern "C" int jfb_kmm_gain_gradient(jfb_kmm_plan* pl, const jfb_kmm_state* init
   const Dims& d = pl->d;
   const size_t P = d.P, nBP = (size_t)d.nB * P, nDP = (size_t)d.nD * P;
   const int64_t T = steps;
-  const int K = (int)std::max<int64_t>(1, std::min<int64_t>(checkpoint > 0 ? checkpoint : T, T));
+  // a segment keeps the x-physical fields of its states (at most kAdjSegment
+  // bytes: longer segments are cut, the result does not depend on it)
+  constexpr size_t kAdjSegment = (size_t)8 << 30;
+  const size_t f = (size_t)d.Nx * P;
+  int64_t K = std::max<int64_t>(1, std::min<int64_t>(checkpoint > 0 ? checkpoint : T, T));
+  K = std::min<int64_t>(K, std::max<int64_t>(1, (int64_t)(kAdjSegment / (6 * f * sizeof(c64)))));
+  const int64_t nck = (T + K - 1) / K;
   int st = adj_prepare(pl);
   if (st) return st;
   // the initial state with a zero history
@@ -2660,76 +2663,43 @@ extern "C" int jfb_kmm_gain_gradient(jfb_kmm_plan* pl, const jfb_kmm_state* init
   for (int k = 0; k < 4; ++k)
     z.nonlinear_old[k] = z.nonlinear_older[k] = z.solution_old[k] = z.solution_older[k] = nullptr;
   if ((st = jfb_kmm_set_state(pl, &z, stream))) return st;
-
-  AdjRun R;
-  const size_t f = (size_t)d.Nx * P, fm = (size_t)d.Nx * d.My * d.Kz;
-#define AL(p, n) \
-  if ((st = R.alloc(&(p), (n)))) return st;
-  AL(R.XF, 6 * f);
-  AL(R.YF, 6 * fm);
-  AL(R.AH, 3 * f);
-  AL(R.AW, 3 * fm);
-  AL(R.HZ6, 6 * fm);
-  AL(R.AX, 6 * f);
-  AL(R.U1w, nDP);
-  AL(R.U2w, nDP);
-  AL(R.EU[0], nBP);
-  AL(R.EU[1], nDP);
-  AL(R.EU[2], nDP);
-  auto alloc_state = [&](AState& a) -> int {
-    int e;
-    if ((e = R.alloc(&a.u, nBP))) return e;
-    if ((e = R.alloc(&a.g, nDP))) return e;
-    if ((e = R.alloc(&a.v, nDP))) return e;
-    return R.alloc(&a.w, nDP);
-  };
-  for (int k = 0; k < 4; ++k) {
-    if ((st = alloc_state(R.S[k]))) return st;
-    if ((st = alloc_state(R.Nn[k]))) return st;
-  }
-  if ((st = alloc_state(R.MU))) return st;
-  if ((st = alloc_state(R.Z))) return st;
-  for (int k = 0; k < 3; ++k)
-    if ((st = alloc_state(R.NZ[k]))) return st;
-  AL(R.TU0, (size_t)(K + 1) * nBP);
-  AL(R.TG, (size_t)(K + 1) * nDP);
-  AL(R.TVW, (size_t)(K + 1) * d.nD);
-  for (int n = 0; n < 2; ++n)
-    for (int z1 = 0; z1 < 2; ++z1) {
-      AL(R.rec[n][3 * z1], nBP);
-      AL(R.rec[n][3 * z1 + 1], nDP);
-      AL(R.rec[n][3 * z1 + 2], (size_t)d.nD);
+  if ((st = adj_buffers(pl, K, nck))) return st;
+  AdjRun& R = pl->adj;
+  struct Keep {  // large buffers are given back at the end of the call
+    AdjRun& R;
+    ~Keep() {
+      if (R.bytes > kAdjKeep) R.release();
     }
-  AL(R.IU0, nBP);
-  AL(R.IU1, nDP);
-  AL(R.IU2, nDP);
-  AL(R.IG, nDP);
-  const int nck = (int)((T + K - 1) / K);
-  R.ck_elems = checkpoint_elems(pl);
-  R.ck.resize(nck);
-  for (int k = 0; k < nck; ++k) AL(R.ck[k], R.ck_elems);
-  double* dev8 = nullptr;
-  JFB_CHECK_CUDA(cudaMalloc((void**)&dev8, 10 * sizeof(double)));
-  R.mem.push_back(dev8);
-#undef AL
+  } keep{R};
+  double* dev8 = R.dev8;
 
   // explicit initial leaves and E(0)
-  const int c0 = slot(0);
-  JFB_CHECK_CUDA(cudaMemcpyAsync(R.IU0, pl->U0[c0], nBP * sizeof(c64), cudaMemcpyDeviceToDevice, s));
-  JFB_CHECK_CUDA(cudaMemcpyAsync(R.IG, pl->G[c0], nDP * sizeof(c64), cudaMemcpyDeviceToDevice, s));
+  JFB_CHECK_CUDA(cudaMemcpyAsync(R.IU0, pl->U0[slot(0)], nBP * sizeof(c64), cudaMemcpyDeviceToDevice, s));
   JFB_CHECK_CUDA(cudaMemcpyAsync(R.IU1, pl->U1S, nDP * sizeof(c64), cudaMemcpyDeviceToDevice, s));
   JFB_CHECK_CUDA(cudaMemcpyAsync(R.IU2, pl->U2S, nDP * sizeof(c64), cudaMemcpyDeviceToDevice, s));
   double E0 = 0.0, ET = 0.0;
   if ((st = perturbation_energy(pl, dev8, s, &E0))) return st;
   JFB_REQUIRE(std::isfinite(E0) && E0 > 0.0, "initial energy must be positive");
   if ((st = ensure_H(pl, s))) return st;
+  JFB_CHECK_CUDA(cudaMemcpyAsync(R.X0, pl->X, 6 * f * sizeof(c64), cudaMemcpyDeviceToDevice, s));
 
-  // forward sweep with checkpoints
+  // forward sweep with checkpoints; the last segment's fields are recorded on
+  // the way, so that it is not recomputed
+  auto step_recorded = [&](int64_t m, int64_t a) -> int {
+    c64* const* rec = (m < 2) ? R.recX[m] : nullptr;
+    int e = forward_step(pl, s, rec);
+    if (e) return e;
+    JFB_CHECK_CUDA(cudaMemcpyAsync(R.TX + (size_t)(m - a) * 6 * f, pl->X, 6 * f * sizeof(c64),
+                                   cudaMemcpyDeviceToDevice, s));
+    return JFB_OK;
+  };
+  const int64_t a_last = (nck - 1) * K;
   for (int64_t m = 0; m < T; ++m) {
-    if (m % K == 0) {
+    if (grad && m % K == 0 && m < a_last) {
       if ((st = checkpoint_io(pl, R.ck[m / K], true, s))) return st;
     }
-    if ((st = forward_step(pl, s, nullptr))) return st;
+    if ((st = grad && m >= a_last ? step_recorded(m, a_last) : forward_step(pl, s, nullptr)))
+      return st;
   }
   if ((st = perturbation_energy(pl, dev8, s, &ET))) return st;
   const double gain = ET / E0;
@@ -2738,101 +2708,81 @@ extern "C" int jfb_kmm_gain_gradient(jfb_kmm_plan* pl, const jfb_kmm_state* init
 
   // terminal adjoint: grad of E(T) / E(0) through the reconstruction of u(T)
   const double area = pl->cfg.ly * pl->cfg.lz;
-  for (int k = 0; k < 4; ++k) {
-    if ((st = astate_zero(pl, R.S[k], s))) return st;
-    if ((st = astate_zero(pl, R.Nn[k], s))) return st;
-  }
-  {
-    const int cT = slot(pl->n);
-    if ((st = adj_energy(pl, R, pl->U0[cT], pl->U1S, pl->U2S, 2.0 * area / E0, false, s)))
-      return st;
-    if ((st = adj_recon(pl, R, R.S[T % 4], false, s))) return st;
-  }
-  const double dt = pl->cfg.dt;
+  if ((st = adj_energy(pl, R, pl->U0[slot(pl->n)], pl->U1S, pl->U2S, 2.0 * area / E0, false, s)))
+    return st;
+  if ((st = adj_recon(pl, R, R.S, s))) return st;
+  const double dt = pl->cfg.dt, nu = pl->cfg.nu;
   const double cS[3] = {18.0 / 11.0, -9.0 / 11.0, 2.0 / 11.0};
   const double dS[3] = {18.0 / 11.0, -18.0 / 11.0, 6.0 / 11.0};
-  auto ring = [](int64_t i) { return (int)(((i % 4) + 4) % 4); };
-  for (int seg = nck - 1; seg >= 0; --seg) {
-    const int64_t a = (int64_t)seg * K, b = std::min<int64_t>(T, a + K);
-    // recompute s_a .. s_b
-    if ((st = checkpoint_io(pl, R.ck[seg], false, s))) return st;
-    pl->n = a;
-    pl->hist = (int)std::min<int64_t>(2, a);
-    pl->have_H = true;
-    pl->explicit_u12 = false;
-    if ((st = record_state(pl, R, 0, s))) return st;
-    for (int64_t m = a; m < b; ++m) {
-      c64* const* rec = (m < 2) ? R.rec[m] : nullptr;
-      if ((st = forward_step(pl, s, rec))) return st;
-      if ((st = record_state(pl, R, (int)(m + 1 - a), s))) return st;
+  double gl[3];  // linear coefficients of the startup stages
+  for (int rk = 0; rk < 3; ++rk) gl[rk] = (kRK3A[rk] + kRK3B[rk]) * dt / 2.0 * nu;
+  auto mu = [&](int64_t n) -> const AdjRun::Mu& { return R.M[n % 4]; };  // step n >= 2
+  for (int64_t seg = nck - 1; seg >= 0; --seg) {
+    const int64_t a = seg * K, b = std::min<int64_t>(T, a + K);
+    if (seg < nck - 1) {  // recompute s_a .. s_b
+      if ((st = checkpoint_io(pl, R.ck[seg], false, s))) return st;
+      pl->n = a;
+      pl->hist = (int)std::min<int64_t>(2, a);
+      pl->have_H = true;
+      pl->explicit_u12 = false;
+      for (int64_t m = a; m < b; ++m)
+        if ((st = step_recorded(m, a))) return st;
     }
-    auto su0 = [&](int64_t m) { return R.TU0 + (size_t)(m - a) * nBP; };
-    auto sg = [&](int64_t m) { return R.TG + (size_t)(m - a) * nDP; };
-    auto svw = [&](int64_t m) { return R.TVW + (size_t)(m - a) * d.nD; };
     for (int64_t n = b - 1; n >= a; --n) {
-      // the nonlinear term of s_{n+1} is complete: fold it into its state adjoint
-      if (n + 1 <= T - 1) {
-        if ((st = adj_nonlinear(pl, R, su0(n + 1), sg(n + 1), svw(n + 1), nullptr, nullptr,
-                                R.Nn[ring(n + 1)], s)))
-          return st;
-        if ((st = adj_recon(pl, R, R.S[ring(n + 1)], true, s))) return st;
+      // step n: s_{n+1} from its readers (the steps n+1 .. n+3, its own
+      // nonlinear term), solved back through the step
+      const bool inner = n + 1 <= T - 1;
+      if (inner && (st = adj_linearise(pl, R, R.TX + (size_t)(n - a) * 6 * f, s))) return st;
+      AdjStageArgs A = adj_args(R, inner);
+      if (!inner) {
+        A.add_u = R.S.u;
+        A.add_g = R.S.g;
+        A.add_vw = R.S.vw;
+      }
+      const AdjRun::Mu* Q = n < 2 ? R.Q[n] : nullptr;
+      if (n == 0 && T > 1) adj_mu(A, R.Q[1][0], 1.0, gl[0], 0.0);
+      for (int l = 0; l < 3; ++l) {  // step n + 1 + l reads s_{n+1} as its level l
+        const int64_t k = n + 1 + l;
+        if (k >= 2 && k <= T - 1)  // and s_n as its level l + 1
+          adj_mu(A, mu(k), cS[l], 0.0, n >= 2 && l < 2 ? dt * dS[l + 1] : 0.0);
       }
       if (n >= 2) {
-        if ((st = adj_solve(pl, pl->adj_steady, R.S[ring(n + 1)], R.MU, s))) return st;
-        for (int l = 0; l < 3; ++l) {
-          if ((st = adj_mass(pl, R.MU, cS[l], 0.0, R.S[ring(n - l)], s))) return st;
-          astate_axpy(pl, R.Nn[ring(n - l)], R.MU, dt * dS[l], s);
-        }
-      } else {
-        // IMEXRK3 startup step from s_n: stage states z0 = s_n, z1, z2 (rec)
-        JFB_CHECK_CUDA(cudaMemcpyAsync(R.Z.u, R.S[ring(n + 1)].u, nBP * sizeof(c64),
-                                       cudaMemcpyDeviceToDevice, s));
-        JFB_CHECK_CUDA(cudaMemcpyAsync(R.Z.g, R.S[ring(n + 1)].g, nDP * sizeof(c64),
-                                       cudaMemcpyDeviceToDevice, s));
-        JFB_CHECK_CUDA(cudaMemcpyAsync(R.Z.v, R.S[ring(n + 1)].v, nDP * sizeof(c64),
-                                       cudaMemcpyDeviceToDevice, s));
-        JFB_CHECK_CUDA(cudaMemcpyAsync(R.Z.w, R.S[ring(n + 1)].w, nDP * sizeof(c64),
-                                       cudaMemcpyDeviceToDevice, s));
-        for (int k = 0; k < 3; ++k)
-          if ((st = astate_zero(pl, R.NZ[k], s))) return st;
-        for (int rk = 2; rk >= 0; --rk) {
-          const double gl = (kRK3A[rk] + kRK3B[rk]) * dt / 2.0 * pl->cfg.nu;
-          if ((st = adj_solve(pl, pl->adj_startup[rk], R.Z, R.MU, s))) return st;
-          if ((st = astate_zero(pl, R.Z, s))) return st;
-          if ((st = adj_mass(pl, R.MU, 1.0, gl, R.Z, s))) return st;
-          astate_axpy(pl, R.NZ[rk], R.MU, dt * kRK3A[rk], s);
-          if (rk > 0) astate_axpy(pl, R.NZ[rk - 1], R.MU, dt * kRK3B[rk], s);
-          if (rk > 0) {
-            // the stage state's own nonlinear term is complete
-            c64* const* z = R.rec[n] + 3 * (rk - 1);
-            if ((st = adj_nonlinear(pl, R, z[0], z[1], z[2], nullptr, nullptr, R.NZ[rk], s)))
-              return st;
-            if ((st = adj_recon(pl, R, R.Z, true, s))) return st;
-          }
-        }
-        astate_axpy(pl, R.S[ring(n)], R.Z, 1.0, s);
-        astate_axpy(pl, R.Nn[ring(n)], R.NZ[0], 1.0, s);
+        if ((st = adj_stage(pl, R, A, &pl->steady, dt * dS[0], &mu(n), s))) return st;
+        continue;
       }
-      // index n + 1 is finished; its ring slot serves index n - 3 next
-      if ((st = astate_zero(pl, R.S[ring(n + 1)], s))) return st;
-      if ((st = astate_zero(pl, R.Nn[ring(n + 1)], s))) return st;
+      // IMEXRK3 startup step: its stages from the last
+      if ((st = adj_stage(pl, R, A, &pl->startup[2], dt * kRK3A[2], &Q[2], s))) return st;
+      for (int rk = 1; rk >= 0; --rk) {
+        if ((st = adj_linearise(pl, R, R.recX[n][rk], s))) return st;
+        A = adj_args(R, true);
+        adj_mu(A, Q[rk + 1], 1.0, gl[rk + 1], dt * kRK3B[rk + 1]);
+        if (rk == 0)  // the next point is s_n itself, which later steps read too
+          for (int64_t k = 2; k <= std::min<int64_t>(n + 2, T - 1); ++k)
+            adj_mu(A, mu(k), 0.0, 0.0, dt * dS[k - n]);
+        if ((st = adj_stage(pl, R, A, &pl->startup[rk], dt * kRK3A[rk], &Q[rk], s))) return st;
+      }
     }
   }
+  // the primary state's adjoint S_0
+  {
+    AdjStageArgs A = adj_args(R, false);
+    adj_mu(A, R.Q[0][0], 1.0, gl[0], 0.0);
+    if (T > 2) adj_mu(A, mu(2), cS[2], 0.0, 0.0);
+    if ((st = adj_stage(pl, R, A, nullptr, 0.0, &R.S, s))) return st;
+  }
   // explicit leaves: the first nonlinear term (explicit velocity) ...
-  if ((st = adj_nonlinear(pl, R, R.IU0, R.IG, nullptr, R.IU1, R.IU2, R.Nn[ring(0)], s))) return st;
+  if ((st = adj_linearise(pl, R, R.X0, s))) return st;
+  {
+    AdjStageArgs A = adj_args(R, true);
+    for (int k = 0; k < 3; ++k) A.EU[k] = R.EU[k];
+    if ((st = adj_stage(pl, R, A, nullptr, 0.0, nullptr, s))) return st;
+  }
   // ... minus gain * grad E(0) / E(0) ...
   if ((st = adj_energy(pl, R, R.IU0, R.IU1, R.IU2, -2.0 * area * gain / E0, true, s))) return st;
   // ... plus the primary-state adjoint: u0, g, and the means of u1, u2
-  const AState& S0 = R.S[ring(0)];
+  const AdjRun::Mu& S0 = R.S;
   axpy_kernel<<<256, 256, 0, s>>>(R.EU[0], S0.u, 1.0, nBP);
-  {
-    PTermList L = tlist(R.EU[1], d.nD, true);
-    term(L, S0.v, nullptr, d.nD, 0, 1, 0, 0, 0, 0, 2, 1);
-    if ((st = run(pl, L, s))) return st;
-    L = tlist(R.EU[2], d.nD, true);
-    term(L, S0.w, nullptr, d.nD, 0, 1, 0, 0, 0, 0, 2, 1);
-    if ((st = run(pl, L, s))) return st;
-  }
+  add_mean_kernel<<<1, 128, 0, s>>>(S0.vw, d.nD, P, R.EU[1], R.EU[2]);
   JFB_CHECK_LAUNCH();
   // jax.grad convention (directional derivative Re sum(g d)): conjugate
   const c64* outs_half[4] = {R.EU[0], R.EU[1], R.EU[2], S0.g};
@@ -2870,11 +2820,10 @@ extern "C" int jfb_kmm_energy_gradient(jfb_kmm_plan* pl, const jfb_kmm_state* st
   if ((st = jfb_kmm_set_state(pl, &z, stream))) return st;
   cudaStream_t s = (cudaStream_t)stream;
   const Dims& d = pl->d;
+  // the gradient's three arrays in the plan's HD buffer (3 x nD rows, unused here)
   AdjRun R;
   const size_t P = d.P;
-  if ((st = R.alloc(&R.EU[0], (size_t)d.nB * P))) return st;
-  if ((st = R.alloc(&R.EU[1], (size_t)d.nD * P))) return st;
-  if ((st = R.alloc(&R.EU[2], (size_t)d.nD * P))) return st;
+  for (int k = 0; k < 3; ++k) R.EU[k] = pl->HD + (size_t)k * d.nD * P;
   const double area = pl->cfg.ly * pl->cfg.lz;
   if ((st = adj_energy(pl, R, pl->U0[slot(0)], pl->U1S, pl->U2S, 2.0 * area, false, s))) return st;
   void* outs[3] = {grad->u0, grad->u1, grad->u2};
