@@ -787,8 +787,8 @@ def main(argv=None):
         out = {
             "workload": "-lap u + u = f, 64 Chebyshev-Dirichlet x 64 Fourier, seeded forcing",
             "us_per_solve": us,
-            "path": ("one launch (jfb_helmholtz2d_solve: 8-CTA cluster, problem in distributed "
-                     "shared memory)" if h.fused else "separate launches"),
+            "path": ("two launches (jfb_helmholtz2d_solve: a CTA per Fourier mode, y transform)"
+                     if h.fused else "separate launches"),
             "us_per_solve_graph_replay": us_graph,
             "us_per_solve_separate_launches": us_sep,
             "solves": K,

@@ -439,18 +439,19 @@ int jfb_tps_project_from_orthogonal(jfb_tps* tps, const void* orth, void* coeffs
 int jfb_tps_scalar_product_from_orthogonal(jfb_tps* tps, const void* orth, void* out,
                                            void* stream);
 
-/* The 2-D Helmholtz solve -lap u + alpha u = f of la/solvers.py:22-61 as one
- * launch: orthogonal-Chebyshev x Fourier coefficients f_hat (N, n1) ->
+/* The 2-D Helmholtz solve -lap u + alpha u = f of la/solvers.py:22-61 as two
+ * launches: orthogonal-Chebyshev x Fourier coefficients f_hat (N, n1) ->
  * backward of tc, scalar products of td divided by fourier_mass, the
  * per-wavenumber banded solve with the no-pivot LU factors (L, U) of
  * TPMatricesWavenumberSolver (tpmatrix.py:1550-1677; DIA data (n1, n_diag,
  * N - 2), L offsets < 0, U offsets >= 0 with 0), backward of td -> u (N, n1)
  * complex128.  tc: 2-D, JFB_BASIS_ORTHOGONAL; td: 2-D, JFB_BASIS_DIRICHLET,
- * same sizes.  One cluster of 8 CTAs holds the whole problem in distributed
- * shared memory (per CTA 16 (2 N c + N q + 2 n1 ceil(N/8)) + 8 N (N - 2)
- * bytes, c = ceil(n1/8), q = c rounded up to 1 mod 4): JFB_ERR_ARG when that
- * exceeds a CTA's shared memory (use the separate transforms and
- * jfb_wavenumber_solve then).  U_inv (optional, N - 2 <= 128): the inverse of
+ * same sizes.  A CTA per Fourier mode forms its right-hand side (backward and
+ * scalar products cancel up to the basis norms under Gauss quadrature), solves
+ * and evaluates; the y transform follows.  Sizes: JFB_ERR_ARG when
+ * 16 (2 N c + N q + 2 n1 ceil(N/8)) + 8 N (N - 2) bytes, c = ceil(n1/8), q = c
+ * rounded up to 1 mod 4, exceed a CTA's shared memory (use the separate
+ * transforms and jfb_wavenumber_solve then).  U_inv (optional, N - 2 <= 128): the inverse of
  * each mode's U, (n1, N - 2, N - 2) with entry (r, c) at c (N - 2) + r; with
  * it and L offsets among {-2, -4} the solve is two short recurrences and a
  * product (no dependent column chain); NULL: column-oriented substitution. */

@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(256) y_backward_warp_kernel(const __grid_const
 // y_forward: per (x-plane, field, kz chunk): forward FFT My along y, keep the
 // Ny retained modes (Nyquist zeroed), scale 1/My.
 // ---------------------------------------------------------------------------
-template <int P, typename T>
+template <int P, typename T, bool kKeepNyq = false>
 __device__ __forceinline__ void y_forward_warp_body(const Dims& d, const int KC,
                                                     const cpx<T>* __restrict__ tw,
                                                     const cpx<T>* __restrict__ HZ,
@@ -107,7 +107,8 @@ __device__ __forceinline__ void y_forward_warp_body(const Dims& d, const int KC,
       const int k = 32 * k1 + lane;
       if (k < half) out[k * ld + c] = scale * v[k1];
       else if (k > d.My - half) out[(k - d.My + d.Ny) * ld + c] = scale * v[k1];
-      else if (k == d.My - half) out[half * ld + c] = cmk(T(0), T(0));  // Nyquist
+      else if (k == d.My - half)  // the -Ny/2 mode
+        out[half * ld + c] = kKeepNyq ? scale * v[k1] : cmk(T(0), T(0));
     }
   }
   __syncthreads();
@@ -123,13 +124,13 @@ __device__ __forceinline__ void y_forward_warp_body(const Dims& d, const int KC,
   }
 }
 
-template <int P, typename T>
+template <int P, typename T, bool kKeepNyq = false>
 __global__ void __launch_bounds__(256) y_forward_warp_kernel(const __grid_constant__ Dims d, int KC,
                                                              const cpx<T>* __restrict__ tw,
                                                              const cpx<T>* __restrict__ HZ,
                                                              cpx<T>* __restrict__ HX,
                                                              const double* __restrict__ xb) {
-  y_forward_warp_body<P, T>(d, KC, tw, HZ, HX, xb, blockIdx.x, blockIdx.y, blockIdx.z);
+  y_forward_warp_body<P, T, kKeepNyq>(d, KC, tw, HZ, HX, xb, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
 // Hermitian-extended packed spectrum Z = A + i B of two real fields whose

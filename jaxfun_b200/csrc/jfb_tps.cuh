@@ -6,34 +6,18 @@
 // unnormalised inverse, forward scaled 1/M and truncated to the modes
 // wavenumbers() keeps, Nyquist included).
 //
-//   x axis:       dense real operator per axis-0 line (x_apply_kernel)
-//   middle axis:  y_backward_kernel / y_forward_kernel (shared with the step)
-//   last axis:    fft_rows_kernel (contiguous lines, shared-memory Stockham)
+//   x axis:       dense real operator per axis-0 line (x_apply_kernel, FP64
+//                 tensor cores)
+//   middle axis:  the step's y kernels (warp-shuffle FFT, or Stockham)
+//   last axis:    fft_rows_warp_kernel / fft_rows_kernel (contiguous lines)
 //
 // Included at the end of jfb_kmm.cu (one translation unit with the step).
 #pragma once
 
-#include "jfb_kmm_kernels.cuh"
+#include "jfb_kmm_split.cuh"
+#include "jfb_kmm_warpk.cuh"
 
 namespace jfb {
-
-// out[i][m] = sum_k A[i][k] in[k][m], A real (rows x cols), m < M contiguous.
-__global__ void __launch_bounds__(256) x_apply_kernel(const double* __restrict__ A, int rows,
-                                                      int cols, const c64* __restrict__ in,
-                                                      c64* __restrict__ out, int64_t M) {
-  const int64_t m = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int i = blockIdx.y;
-  if (m >= M || i >= rows) return;
-  const double* a = A + (size_t)i * cols;
-  c64 s0 = cmk(0.0, 0.0), s1 = s0;
-  int k = 0;
-  for (; k + 1 < cols; k += 2) {
-    s0 = s0 + __ldg(a + k) * in[(size_t)k * M + m];
-    s1 = s1 + __ldg(a + k + 1) * in[(size_t)(k + 1) * M + m];
-  }
-  if (k < cols) s0 = s0 + __ldg(a + k) * in[(size_t)k * M + m];
-  out[(size_t)i * M + m] = s0 + s1;
-}
 
 // Per-mode Fourier weight of the separable maps: scale * prod over the
 // periodic axes of (i m df)^k, m the FFT-ordered wavenumber, with the Nyquist
@@ -54,46 +38,83 @@ __device__ __forceinline__ c64 ipow_times(c64 w, int idx, int n, int k, double d
   return w;
 }
 
-// out[i][m] = w(m) sum_k A[i][k] in[k][m]: an x-axis matrix with per-mode
-// Fourier weights (m = i1 n2 + i2 over the periodic axes).
-__global__ void __launch_bounds__(256) x_apply_w_kernel(const double* __restrict__ A, int rows,
-                                                        int cols, const c64* __restrict__ in,
-                                                        c64* __restrict__ out, FourierWeight fw) {
-  const int64_t M = (int64_t)fw.n1 * fw.n2;
-  const int64_t m = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int i = blockIdx.y;
-  if (m >= M || i >= rows) return;
-  const double* a = A + (size_t)i * cols;
-  c64 s0 = cmk(0.0, 0.0), s1 = s0;
-  int k = 0;
-  for (; k + 1 < cols; k += 2) {
-    s0 = s0 + __ldg(a + k) * in[(size_t)k * M + m];
-    s1 = s1 + __ldg(a + k + 1) * in[(size_t)(k + 1) * M + m];
+// out[i][m] = w(m) sum_k A[i][k] in[k][m], A real (rows x cols) in 8x4 mma
+// fragment tiles, w a per-mode Fourier weight (m = i1 n2 + i2 over the
+// periodic axes).  A block stages 16 columns of the field as B-operand rows
+// (swizzled as in gemm_sw) and its warps take the row tiles of A: the field is
+// read once, where one thread per output read every column once per row from
+// L2 (23 -> 7 us for 65 x 63 on 4096 columns).  Bound by memory.
+constexpr int kXThreads = 256;
+__global__ void __launch_bounds__(kXThreads)
+    x_apply_kernel(const double* __restrict__ frag, int rows, int cols, const c64* __restrict__ in,
+                   c64* __restrict__ out, const __grid_constant__ FourierWeight fw) {
+  extern __shared__ __align__(128) double sm[];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int64_t M = (int64_t)fw.n1 * fw.n2, m0 = (int64_t)blockIdx.x * kGW;
+  const int c = tid & 15, nc = (int)min((int64_t)kGW, M - m0);
+  const int KT = (cols + 3) / 4;
+  if (c < nc)
+    for (int k = tid >> 4; k < cols; k += kXThreads / 16)
+      cp_async16(sat(sm, k, c), in + (size_t)k * M + m0 + c);
+  else
+    for (int k = tid >> 4; k < cols; k += kXThreads / 16) *sat(sm, k, c) = cmk(0.0, 0.0);
+  for (int e = tid; e < (4 * KT - cols) * kSLd; e += kXThreads) sm[(size_t)cols * kSLd + e] = 0.0;
+  cp_async_commit();
+  cp_async_wait_all();
+  __syncthreads();
+  const int g = lane >> 2, t4 = lane & 3;
+  c64 w[4];
+#pragma unroll
+  for (int nt = 0; nt < 4; ++nt) {
+    const int64_t m = m0 + nt * 4 + t4;
+    w[nt] = cmk(fw.scale, 0.0);
+    if (m < M) {
+      w[nt] = ipow_times(w[nt], (int)(m / fw.n2), fw.n1, fw.k1, fw.df1);
+      w[nt] = ipow_times(w[nt], (int)(m % fw.n2), fw.n2, fw.k2, fw.df2);
+    }
   }
-  if (k < cols) s0 = s0 + __ldg(a + k) * in[(size_t)k * M + m];
-  c64 w = cmk(fw.scale, 0.0);
-  w = ipow_times(w, (int)(m / fw.n2), fw.n1, fw.k1, fw.df1);
-  w = ipow_times(w, (int)(m % fw.n2), fw.n2, fw.k2, fw.df2);
-  out[(size_t)i * M + m] = w * (s0 + s1);
+  for (int mt = warp + blockIdx.y * (kXThreads / 32); mt * 8 < rows;
+       mt += gridDim.y * (kXThreads / 32)) {
+    double acc[4][2];
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) acc[nt][0] = acc[nt][1] = 0.0;
+    gemm_sw<4, 8>(frag + (size_t)mt * KT * 32, 0, KT, sm, 0, 0, lane, acc);
+    const int i = mt * 8 + g;
+    if (i >= rows) continue;
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) {
+      const int64_t m = m0 + nt * 4 + t4;
+      if (m < M) out[(size_t)i * M + m] = w[nt] * cmk(acc[nt][0], acc[nt][1]);
+    }
+  }
+}
+
+// A real (rows x cols) matrix as 8x4 mma fragment tiles (zero padded).
+static std::vector<double> fragment_tiles(const std::vector<double>& A, int rows, int cols) {
+  const int MT = (rows + 7) / 8, KT = (cols + 3) / 4;
+  std::vector<double> f((size_t)MT * KT * 32, 0.0);
+  for (int i = 0; i < rows; ++i)
+    for (int k = 0; k < cols; ++k)
+      f[((size_t)(i >> 3) * KT + (k >> 2)) * 32 + (i & 7) * 4 + (k & 3)] = A[(size_t)i * cols + k];
+  return f;
 }
 
 // Complex FFT along contiguous lines: `lines` rows of length nin -> nout.
 // Inverse (sign +1, transform length nout): pad nin -> nout in the middle,
 // unnormalised.  Forward (sign -1, transform length nin): scaled 1/nin,
 // truncated to nout modes in FFT order (k < nout/2 and the last nout/2 of
-// the spectrum, the -nout/2 mode included).  kTpsRows lines per block.
-constexpr int kTpsRows = 8;
+// the spectrum, the -nout/2 mode included).  2^lr lines per block.
+constexpr int kTpsLogRows = 3;
 __global__ void __launch_bounds__(256) fft_rows_kernel(FFTPlan plan, const c64* __restrict__ tw,
-                                                       int sign, const c64* __restrict__ in,
-                                                       c64* __restrict__ out, int64_t lines,
-                                                       int nin, int nout) {
+                                                       int sign, const c64* in, c64* out,
+                                                       int64_t lines, int nin, int nout, int lr) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int n = plan.n;
+  const int n = plan.n, R = 1 << lr;
   c64* A = reinterpret_cast<c64*>(smem_raw);
-  c64* B = A + (size_t)n * kTpsRows;
-  const int64_t l0 = blockIdx.x * (int64_t)kTpsRows;
-  for (int idx = threadIdx.x; idx < n * kTpsRows; idx += blockDim.x) {
-    const int c = idx % kTpsRows, k = idx / kTpsRows;
+  c64* B = A + (size_t)n * R;
+  const int64_t l0 = blockIdx.x * (int64_t)R;
+  for (int idx = threadIdx.x; idx < n * R; idx += blockDim.x) {
+    const int c = idx & (R - 1), k = idx >> lr;
     const int64_t line = l0 + c;
     c64 v = cmk(0.0, 0.0);
     if (line < lines) {
@@ -105,304 +126,214 @@ __global__ void __launch_bounds__(256) fft_rows_kernel(FFTPlan plan, const c64* 
         v = in[line * nin + k];
       }
     }
-    A[k * kTpsRows + c] = v;
+    A[k * R + c] = v;
   }
   __syncthreads();
-  c64* res = fft_columns<double>(A, B, plan, kTpsRows, kTpsRows, tw, sign);
+  c64* res = fft_columns<double>(A, B, plan, R, R, tw, sign);
   const double scale = sign > 0 ? 1.0 : 1.0 / n;
   const int h = nout / 2;
-  for (int idx = threadIdx.x; idx < nout * kTpsRows; idx += blockDim.x) {
-    const int c = idx % kTpsRows, k = idx / kTpsRows;
+  for (int idx = threadIdx.x; idx < nout * R; idx += blockDim.x) {
+    const int c = idx & (R - 1), k = idx >> lr;
     const int64_t line = l0 + c;
     if (line >= lines) continue;
     int src = k;
     if (sign < 0 && k >= h) src = k - nout + n;
-    out[line * nout + k] = scale * res[src * kTpsRows + c];
+    out[line * nout + k] = scale * res[src * R + c];
   }
 }
 
-__global__ void tps_scale_kernel(c64* __restrict__ y, double a, size_t n) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x)
-    y[i] = a * y[i];
+// The same with warp-shuffle transforms for lengths 32 P: a warp per line,
+// natural order on the global side (coalesced), the transform's scrambled
+// order through the warp's shared-memory row.  In place allowed when
+// nin == nout (a warp reads its whole line first).  16 -> 8 us for 6240 lines
+// of 64 -> 96 points against the shared-memory form, whose radix passes wait
+// on block barriers.
+template <int P>
+__global__ void __launch_bounds__(256) fft_rows_warp_kernel(const c64* __restrict__ tw, int sign,
+                                                            const c64* in, c64* out, int64_t lines,
+                                                            int nin, int nout) {
+  constexpr int n = 32 * P;
+  __shared__ c64 rowbuf[8][n];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t line = blockIdx.x * (int64_t)8 + warp;
+  if (line >= lines) return;
+  c64* row = rowbuf[warp];
+  const int br = bitrev5(lane);
+  WarpTw<P, double> w;
+  load_warp_tw<P, double>(w, tw, lane);
+  c64 v[P];
+  if (sign > 0) {
+    const int h = nin / 2;
+#pragma unroll
+    for (int r = 0; r < P; ++r) {
+      const int k = 32 * r + lane;
+      v[r] = k < h ? in[line * nin + k]
+                   : k >= n - (nin - h) ? in[line * nin + (k - n + nin)] : cmk(0.0, 0.0);
+    }
+    warp_fft_inverse<P, double>(v, w, lane);
+#pragma unroll
+    for (int r = 0; r < P; ++r) row[r + P * br] = v[r];
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < P; ++r) out[line * n + 32 * r + lane] = row[32 * r + lane];
+  } else {
+#pragma unroll
+    for (int r = 0; r < P; ++r) row[32 * r + lane] = in[line * n + 32 * r + lane];
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < P; ++r) v[r] = row[r + P * br];
+    warp_fft_forward<P, double>(v, w, lane);
+    const int h = nout / 2;
+    const double scale = 1.0 / n;
+#pragma unroll
+    for (int r = 0; r < P; ++r) {
+      const int k = 32 * r + lane;
+      if (k < h) out[line * nout + k] = scale * v[r];
+      else if (k >= n - (nout - h)) out[line * nout + (k - n + nout)] = scale * v[r];
+    }
+  }
 }
 
-
 // ---------------------------------------------------------------------------
-// 2-D Helmholtz solve in one launch (la/solvers.py:22-61 with the per-
-// wavenumber solve of tpmatrix.py:1550-1677) on one cluster of kHelmCTAs
-// CTAs that keeps the whole (N x n1) problem in distributed shared memory:
-// CTA c owns the Fourier columns [c KC, (c+1) KC) for the x-direction work
-// (products against the x operators, the per-mode solves) and the x rows
-// [c JR, (c+1) JR) for the y transforms; the stages exchange their slices
-// through DSMEM reads between cluster barriers, instead of about ten
-// launches through global memory.
+// 2-D Helmholtz solve (la/solvers.py:22-61 with the per-wavenumber solve of
+// tpmatrix.py:1550-1677), one CTA per Fourier mode, then the y transform of
+// the rows.  The backward transform of f and its scalar products cancel up to
+// the norms: the y transforms are inverse to each other, and the Gauss
+// quadrature is exact for products of degree 2 N - 2, so
+//   rhs_r = scale sum_n S_D[r, n] (P_n, P_n) f_n
+// is two terms per row.  A CTA forms its mode's right-hand side, solves and
+// evaluates the solution at the nodes; the launch pair replaces one cluster of
+// eight CTAs that held the whole problem and worked through four transforms
+// between cluster barriers (64 x 64: 38 us, now 5.4 + 2.1).  Bound by latency:
+// the column of f, the recurrence, two products of which a thread takes a
+// quarter of a row (9.4 us with a thread per row and no loads ahead).
 // ---------------------------------------------------------------------------
 constexpr int kHelmMaxDiag = 256;
-constexpr int kHelmCTAs = 8;
-constexpr int kHelmThreads = 256;
-constexpr int kHelmChunk = 8;  // solve columns whose factor entries are loaded together
+constexpr int kHelmCTAs = 8;  // of the size range (jfb_helmholtz2d_solve)
+constexpr int kHelmRows = 128, kHelmSplit = 4;  // thread = (row, every 4th column)
+constexpr int kHelmThreads = kHelmRows * kHelmSplit;
+constexpr int kHelmCols = 16;  // matrix entries a thread loads ahead
 struct Helm2DArgs {
-  const double* BC;  // orthogonal backward, N x N (row j: T_n(x_j))
-  const double* SD;  // Dirichlet scalar products, nb x N
-  const double* BD;  // Dirichlet backward, N x nb
-  const c64* tw;     // n1-point twiddles
-  FFTPlan plan;
+  const double* ns;    // (P_n, P_n) / df
+  const double* BDT;   // Dirichlet backward, transposed (nb x N)
   const double *L, *U;  // (n1, nL, nb), (n1, nU, nb)
   const double* Uinv;   // optional (n1, nb, nb): U^-1 per mode, entry (r, c) at c nb + r
   int nL, nU, umain;
   int l2, l4;  // indices of the L offsets -2 / -4 (-1: absent) when those are all of L
   int loff[kHelmMaxDiag], uoff[kHelmMaxDiag];
-  int N, nb, M, KC, JR, QS;
-  double scale;  // Fourier scalar-product weight / fourier_mass / n1
+  int N, nb, M;
+  double scale;  // Fourier scalar-product weight / fourier_mass
   const c64* f;
   c64* u;
 };
 
-__global__ void __cluster_dims__(kHelmCTAs, 1, 1) __launch_bounds__(kHelmThreads, 1)
+__global__ void __launch_bounds__(kHelmThreads)
     helmholtz2d_kernel(const __grid_constant__ Helm2DArgs h) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  namespace cg = cooperative_groups;
-  cg::cluster_group cluster = cg::this_cluster();
-  const int rank = (int)cluster.block_rank();
-  const int N = h.N, M = h.M, nb = h.nb, KC = h.KC, JR = h.JR, QS = h.QS;
-  const int k0 = rank * KC, kn = min(KC, M - k0);  // owned Fourier columns
-  const int j0 = rank * JR, jn = min(JR, N - j0);  // owned x rows
-  c64* A = reinterpret_cast<c64*>(smem_raw);  // [n][kk]: f slice, then gathered columns
-  c64* B = A + (size_t)N * KC;                // [j][kk]: x-backward slices
-  c64* Q = B + (size_t)N * KC;                // [r][kk] (row stride QS): scalar products -> solutions
-  c64* F0 = Q + (size_t)N * h.QS;             // [k][jj]: y-transform lines
-  c64* F1 = F0 + (size_t)M * JR;
-  double* SdT = reinterpret_cast<double*>(F1 + (size_t)M * JR);  // [j][r]
-  const int tid = threadIdx.x, nt = blockDim.x;
-  for (int i = tid; i < N * KC; i += nt) {
-    const int kk = i % KC, n = i / KC;
-    A[i] = (kk < kn) ? h.f[(size_t)n * M + k0 + kk] : cmk(0.0, 0.0);
-  }
-  for (int i = tid; i < nb * N; i += nt) {
-    const int j = i % N, r = i / N;
-    SdT[j * nb + r] = h.SD[i];
-  }
-  __syncthreads();
-  // x backward (orthogonal) of the owned columns: B[j][kk] = sum_n BC[j][n] f[n][kk]
-  for (int i = tid; i < N * KC; i += nt) {
-    const int kk = i % KC, j = i / KC;
-    const double* a = h.BC + (size_t)j * N;
-    c64 s = cmk(0.0, 0.0);
-    for (int n = 0; n < N; ++n) s = s + __ldg(a + n) * A[n * KC + kk];
-    B[i] = s;
-  }
-  cluster.sync();
-  // y: gather the owned rows across all columns, inverse (unnormalised) then
-  // forward transform
-  for (int i = tid; i < M * JR; i += nt) {
-    const int jj = i % JR, k = i / JR;
-    c64 v = cmk(0.0, 0.0);
-    if (jj < jn) {
-      const c64* src = cluster.map_shared_rank(B, (unsigned)(k / KC));
-      v = src[(j0 + jj) * KC + k % KC];
+  const int N = h.N, M = h.M, nb = h.nb, k = blockIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31;
+  c64* F = reinterpret_cast<c64*>(smem_raw);  // N: the mode's column of f
+  c64* x = F + N;                             // nb: right-hand side, then y
+  c64* z = x + nb;                            // nb: solution
+  c64* part = z + nb;                         // kHelmThreads: partial sums
+  double* l2s = reinterpret_cast<double*>(part + kHelmThreads);  // nb: L[r, r-2], L[r, r-4]
+  double* l4s = l2s + nb;
+  const double* Lk = h.L + (size_t)k * h.nL * nb;
+  const double* Uk = h.U + (size_t)k * h.nU * nb;
+  const bool fast = h.Uinv && h.l2 + h.l4 > -2;
+  const int row = tid & (kHelmRows - 1), grp = tid / kHelmRows;
+  for (int n = tid; n < N; n += kHelmThreads) F[n] = h.f[(size_t)n * M + k];
+  if (fast)
+    for (int r = tid; r < nb; r += kHelmThreads) {
+      l2s[r] = (h.l2 >= 0 && r >= 2) ? __ldg(Lk + (size_t)h.l2 * nb + r - 2) : 0.0;
+      l4s[r] = (h.l4 >= 0 && r >= 4) ? __ldg(Lk + (size_t)h.l4 * nb + r - 4) : 0.0;
     }
-    F0[i] = v;
+  // the matrix entries of the two products do not depend on f: on their way
+  // while the right-hand side and the recurrence run
+  const double* Ui = h.Uinv + (size_t)k * nb * nb + row;
+  double u[kHelmCols], b[kHelmCols];
+#pragma unroll
+  for (int q = 0; q < kHelmCols; ++q) {
+    const int c = grp + kHelmSplit * q;
+    u[q] = fast && c < nb && row <= c ? __ldg(Ui + (size_t)c * nb) : 0.0;
+    b[q] = c < nb && row < N ? __ldg(h.BDT + (size_t)c * N + row) : 0.0;
   }
   __syncthreads();
-  c64* P = fft_columns<double>(F0, F1, h.plan, JR, JR, h.tw, +1);
-  P = fft_columns<double>(P, (P == F0) ? F1 : F0, h.plan, JR, JR, h.tw, -1);
-  cluster.sync();
-  // gather the owned columns across all rows (P sits at the same offset in
-  // every CTA), then the Dirichlet scalar products Q[r][kk]
-  for (int i = tid; i < N * KC; i += nt) {
-    const int kk = i % KC, j = i / KC;
-    c64 v = cmk(0.0, 0.0);
-    if (kk < kn) {
-      const c64* src = cluster.map_shared_rank(P, (unsigned)(j / JR));
-      v = src[(k0 + kk) * JR + j % JR];
+  for (int r = tid; r < nb; r += kHelmThreads)
+    x[r] = h.scale * (h.ns[r] * F[r] - h.ns[r + 2] * F[r + 2]);
+  __syncthreads();
+  // this thread's columns of row i of a matrix (entry (i, c) at m[c * ld]),
+  // c >= first, against v; the first kHelmCols of them are in registers
+  auto dot = [&](const double (&reg)[kHelmCols], const double* m, int ld, int first, const c64* v) {
+    c64 s0 = cmk(0.0, 0.0), s1 = s0;
+#pragma unroll
+    for (int q = 0; q < kHelmCols; q += 2) {
+      const int c = grp + kHelmSplit * q;
+      if (c < nb) s0 = s0 + reg[q] * v[c];
+      if (c + kHelmSplit < nb) s1 = s1 + reg[q + 1] * v[c + kHelmSplit];
     }
-    A[i] = v;
-  }
-  __syncthreads();
-  for (int i = tid; i < nb * KC; i += nt) {
-    const int r = i % nb, kk = i / nb;
-    c64 s = cmk(0.0, 0.0);
-    for (int j = 0; j < N; ++j) s = s + SdT[j * nb + r] * A[j * KC + kk];
-    Q[r * QS + kk] = h.scale * s;
-  }
-  __syncthreads();
-  // per-wavenumber solves, a warp per owned mode, column-oriented
-  // substitution: once x_c is final each lane applies its diagonals' entries
-  // of column c to their rows (distinct rows per diagonal); the entries of
-  // diagonals lane and lane + 32 are loaded one column ahead
-  if (h.Uinv && h.l2 + h.l4 > -2) {
-    // fast form: L with offsets -2 / -4 only is two independent recurrences
-    // (one per parity class, lanes 0 and 1, in registers); then x = U^-1 y
-    // as a product with the mode's explicit inverse (lanes = rows)
-    const int lane = tid & 31, warp = tid >> 5, nwarps = nt >> 5;
-    for (int kk = warp; kk < kn; kk += nwarps) {
-      const int k = k0 + kk;
-      const double* Lk = h.L + (size_t)k * h.nL * nb;
-      c64* x = Q + kk;  // element c at x[c * QS]
-      if (lane < 2) {
-        // the right-hand side and the multipliers of the next row are loaded
-        // before the current row's update (off the dependent chain)
-        auto l2v = [&](int r) { return (h.l2 >= 0 && r >= 2 && r < nb) ? __ldg(Lk + (size_t)h.l2 * nb + r - 2) : 0.0; };
-        auto l4v = [&](int r) { return (h.l4 >= 0 && r >= 4 && r < nb) ? __ldg(Lk + (size_t)h.l4 * nb + r - 4) : 0.0; };
-        c64 ym2 = cmk(0.0, 0.0), ym4 = cmk(0.0, 0.0);  // y_{r-2}, y_{r-4}
-        c64 vn = (lane < nb) ? x[lane * QS] : cmk(0.0, 0.0);
-        double an = l2v(lane), bn = l4v(lane);
-        for (int r = lane; r < nb; r += 2) {
-          const c64 v0 = vn;
-          const double a2 = an, a4 = bn;
-          if (r + 2 < nb) {
-            vn = x[(r + 2) * QS];
-            an = l2v(r + 2);
-            bn = l4v(r + 2);
-          }
-          const c64 v = v0 - a2 * ym2 - a4 * ym4;
-          x[r * QS] = v;
-          ym4 = ym2;
-          ym2 = v;
-        }
+#pragma unroll 8
+    for (int c = grp + kHelmSplit * kHelmCols; c < nb; c += kHelmSplit)
+      if (c >= first) s0 = s0 + __ldg(m + (size_t)c * ld) * v[c];
+    return s0 + s1;
+  };
+  auto total = [&](int i) {
+    return (part[i] + part[i + kHelmRows]) + (part[i + 2 * kHelmRows] + part[i + 3 * kHelmRows]);
+  };
+  if (fast) {
+    // two independent recurrences (one per parity class), then x = U^-1 y as a
+    // product with the mode's explicit inverse
+    if (tid < 2) {
+      c64 ym2 = cmk(0.0, 0.0), ym4 = cmk(0.0, 0.0);  // y_{r-2}, y_{r-4}
+#pragma unroll 4
+      for (int r = tid; r < nb; r += 2) {
+        const c64 v = x[r] - l4s[r] * ym4 - l2s[r] * ym2;
+        x[r] = v;
+        ym4 = ym2;
+        ym2 = v;
+      }
+    }
+    __syncthreads();
+    part[tid] = row < nb ? dot(u, Ui, nb, row, x) : cmk(0.0, 0.0);
+    __syncthreads();
+    if (tid < nb) z[tid] = total(tid);
+  } else if (tid < 32) {
+    // column-oriented substitution: once x_c is final each lane applies its
+    // diagonals' entries of column c to their rows (distinct per diagonal)
+    for (int c = 0; c < nb; ++c) {
+      const c64 y = x[c];
+      for (int d = lane; d < h.nL; d += 32) {
+        const int r = c - h.loff[d];
+        if (r < nb) x[r] = x[r] - __ldg(Lk + (size_t)d * nb + c) * y;
       }
       __syncwarp();
-      const double* Ui = h.Uinv + (size_t)k * nb * nb;
-      c64 acc0 = cmk(0.0, 0.0), acc1 = cmk(0.0, 0.0);  // rows lane, lane + 32, ...
-      c64 acc2 = cmk(0.0, 0.0), acc3 = cmk(0.0, 0.0);
-#pragma unroll 8
-      for (int c = 0; c < nb; ++c) {
-        const c64 y = x[c * QS];
-        const double* col = Ui + (size_t)c * nb;
-        if (lane <= c) acc0 = acc0 + __ldg(col + lane) * y;
-        if (lane + 32 <= c) acc1 = acc1 + __ldg(col + lane + 32) * y;
-        if (lane + 64 <= c) acc2 = acc2 + __ldg(col + lane + 64) * y;
-        if (lane + 96 <= c) acc3 = acc3 + __ldg(col + lane + 96) * y;
-      }
-      c64* O = A + kk;
-      if (lane < nb) O[lane * KC] = acc0;
-      if (lane + 32 < nb) O[(lane + 32) * KC] = acc1;
-      if (lane + 64 < nb) O[(lane + 64) * KC] = acc2;
-      if (lane + 96 < nb) O[(lane + 96) * KC] = acc3;
     }
-  } else {
-    const int lane = tid & 31, warp = tid >> 5, nwarps = nt >> 5;
-    for (int kk = warp; kk < kn; kk += nwarps) {
-      const int k = k0 + kk;
-      const double* Lk = h.L + (size_t)k * h.nL * nb;
-      const double* Uk = h.U + (size_t)k * h.nU * nb;
-      c64* x = Q + kk;  // element c at x[c * QS]
-      c64* O = A + kk;  // solution, element c at O[c * KC] (A is free after the scalar products)
-      auto lld = [&](int d, int c) {
-        return (d < h.nL && c < nb) ? __ldg(Lk + (size_t)d * nb + c) : 0.0;
-      };
-      auto uld = [&](int d, int c) {
-        return (d < h.nU && c >= 0) ? __ldg(Uk + (size_t)d * nb + c) : 0.0;
-      };
-      // row shifts of this lane's diagonals (lane, lane + 32), held in
-      // registers: s > 0 below / above the diagonal, 0 when the lane has none
-      const int ls0 = lane < h.nL ? -h.loff[lane] : 0;
-      const int ls1 = lane + 32 < h.nL ? -h.loff[lane + 32] : 0;
-      const int us0 = lane < h.nU ? h.uoff[lane] : 0;
-      const int us1 = lane + 32 < h.nU ? h.uoff[lane + 32] : 0;
-      // factor entries of diagonals lane and lane + 32, kHelmChunk columns at
-      // a time, loaded one chunk ahead (the chunk's work covers the latency)
-      double a0[kHelmChunk], a1[kHelmChunk], b0[kHelmChunk], b1[kHelmChunk];
-#pragma unroll
-      for (int q = 0; q < kHelmChunk; ++q) {
-        a0[q] = lld(lane, q);
-        a1[q] = lld(lane + 32, q);
+    for (int c = nb - 1; c >= 0; --c) {
+      const double dg = __ldg(Uk + (size_t)h.umain * nb + c);
+      const c64 v = x[c], xc = cmk(v.re / dg, v.im / dg);
+      if (lane == 0) z[c] = xc;
+      for (int d = lane; d < h.nU; d += 32) {
+        const int sft = h.uoff[d], r = c - sft;
+        if (sft > 0 && r >= 0) x[r] = x[r] - __ldg(Uk + (size_t)d * nb + c) * xc;
       }
-      for (int c0 = 0; c0 < nb; c0 += kHelmChunk) {  // unit lower: L[c - s][c] at Lk[d][c], s < 0
-#pragma unroll
-        for (int q = 0; q < kHelmChunk; ++q) {
-          b0[q] = lld(lane, c0 + kHelmChunk + q);
-          b1[q] = lld(lane + 32, c0 + kHelmChunk + q);
-        }
-#pragma unroll
-        for (int q = 0; q < kHelmChunk; ++q) {
-          const int c = c0 + q;
-          if (c >= nb) break;
-          const c64 y = x[c * QS];
-          if (ls0 > 0 && c + ls0 < nb) x[(c + ls0) * QS] = x[(c + ls0) * QS] - a0[q] * y;
-          if (ls1 > 0 && c + ls1 < nb) x[(c + ls1) * QS] = x[(c + ls1) * QS] - a1[q] * y;
-          for (int d = lane + 64; d < h.nL; d += 32) {
-            const int r = c - h.loff[d];
-            if (r < nb) x[r * QS] = x[r * QS] - __ldg(Lk + (size_t)d * nb + c) * y;
-          }
-          __syncwarp();
-        }
-#pragma unroll
-        for (int q = 0; q < kHelmChunk; ++q) {
-          a0[q] = b0[q];
-          a1[q] = b1[q];
-        }
-      }
-      // reciprocal main-diagonal entries of the current / next chunk (formed
-      // off the dependent chain)
-      double g0[kHelmChunk], g1[kHelmChunk];
-#pragma unroll
-      for (int q = 0; q < kHelmChunk; ++q) {
-        a0[q] = uld(lane, nb - 1 - q);
-        a1[q] = uld(lane + 32, nb - 1 - q);
-        g0[q] = 1.0 / uld(h.umain, nb - 1 - q);
-      }
-      for (int t0 = 0; t0 < nb; t0 += kHelmChunk) {  // upper: U[c - s][c] at Uk[d][c], s > 0
-#pragma unroll
-        for (int q = 0; q < kHelmChunk; ++q) {
-          const int c = nb - 1 - (t0 + kHelmChunk + q);
-          b0[q] = uld(lane, c);
-          b1[q] = uld(lane + 32, c);
-          g1[q] = (c >= 0) ? 1.0 / uld(h.umain, c) : 0.0;
-        }
-#pragma unroll
-        for (int q = 0; q < kHelmChunk; ++q) {
-          const int c = nb - 1 - (t0 + q);
-          if (c < 0) break;
-          const c64 v = x[c * QS];
-          const c64 xc = cmk(v.re * g0[q], v.im * g0[q]);
-          if (lane == 0) O[c * KC] = xc;  // the solution goes to O: x[c] is not written
-          if (us0 > 0 && c - us0 >= 0) x[(c - us0) * QS] = x[(c - us0) * QS] - a0[q] * xc;
-          if (us1 > 0 && c - us1 >= 0) x[(c - us1) * QS] = x[(c - us1) * QS] - a1[q] * xc;
-          for (int d = lane + 64; d < h.nU; d += 32) {
-            const int sft = h.uoff[d], r = c - sft;
-            if (sft > 0 && r >= 0) x[r * QS] = x[r * QS] - __ldg(Uk + (size_t)d * nb + c) * xc;
-          }
-          __syncwarp();
-        }
-#pragma unroll
-        for (int q = 0; q < kHelmChunk; ++q) {
-          a0[q] = b0[q];
-          a1[q] = b1[q];
-          g0[q] = g1[q];
-        }
-      }
+      __syncwarp();
     }
   }
   __syncthreads();
-  // x backward (Dirichlet) of the owned solutions (in A) into B (its earlier
-  // contents were read by the other CTAs before the last cluster barrier)
-  for (int i = tid; i < N * KC; i += nt) {
-    const int kk = i % KC, j = i / KC;
-    const double* a = h.BD + (size_t)j * nb;
-    c64 s = cmk(0.0, 0.0);
-    for (int r = 0; r < nb; ++r) s = s + __ldg(a + r) * A[r * KC + kk];
-    B[i] = s;
-  }
-  cluster.sync();
-  // y: gather the owned rows, inverse transform, store u[j][l]
-  for (int i = tid; i < M * JR; i += nt) {
-    const int jj = i % JR, k = i / JR;
-    c64 v = cmk(0.0, 0.0);
-    if (jj < jn) {
-      const c64* src = cluster.map_shared_rank(B, (unsigned)(k / KC));
-      v = src[(j0 + jj) * KC + k % KC];
+  for (int j0 = 0; j0 < N; j0 += kHelmRows) {
+    const int j = j0 + row;
+    if (j0 > 0) {
+      __syncthreads();
+#pragma unroll
+      for (int q = 0; q < kHelmCols; ++q) {
+        const int c = grp + kHelmSplit * q;
+        b[q] = c < nb && j < N ? __ldg(h.BDT + (size_t)c * N + j) : 0.0;
+      }
     }
-    F0[i] = v;
+    part[tid] = j < N ? dot(b, h.BDT + j, N, 0, z) : cmk(0.0, 0.0);
+    __syncthreads();
+    if (grp == 0 && j < N) h.u[(size_t)j * M + k] = total(row);
   }
-  __syncthreads();
-  const c64* R = fft_columns<double>(F0, F1, h.plan, JR, JR, h.tw, +1);
-  for (int i = tid; i < jn * M; i += nt) {
-    const int l = i % M, jj = i / M;
-    h.u[(size_t)(j0 + jj) * M + l] = R[l * JR + jj];
-  }
-  cluster.sync();  // no CTA leaves while another still reads its slices
 }
 
 }  // namespace jfb
@@ -413,7 +344,8 @@ struct jfb_tps {
   std::map<int64_t, std::pair<double*, std::pair<int, int>>> xmaps;  // (map, k) -> device matrix
   int nb = 0, N = 0;
   int n1 = 1, n2 = 1, m1 = 1, m2 = 1;  // Fourier modes and padded counts
-  double *B = nullptr, *F = nullptr, *Sq = nullptr;
+  double *B = nullptr, *F = nullptr, *Sq = nullptr;  // mma fragment tiles
+  double *BT = nullptr, *ns = nullptr;               // B transposed (nb x N), norms
   std::vector<double> G0, G2;
   c64 *tw1n = nullptr, *tw1m = nullptr, *tw2n = nullptr, *tw2m = nullptr;
   FFTPlan f1n, f1m, f2n, f2m;
@@ -501,7 +433,17 @@ extern "C" int jfb_tps_create(const jfb_tps_config* cfg, jfb_tps** out) {
     return JFB_OK;
   };
   int st;
-  if ((st = up(&t->B, x.B)) || (st = up(&t->F, x.F)) || (st = up(&t->Sq, x.Sq))) return fail(st);
+  if ((st = up(&t->B, fragment_tiles(x.B, t->N, t->nb))) ||
+      (st = up(&t->F, fragment_tiles(x.F, t->nb, t->N))) ||
+      (st = up(&t->Sq, fragment_tiles(x.Sq, t->nb, t->N))))
+    return fail(st);
+  {
+    std::vector<double> bt((size_t)t->nb * t->N), ns(t->N);
+    for (int j = 0; j < t->N; ++j)
+      for (int r = 0; r < t->nb; ++r) bt[(size_t)r * t->N + j] = x.B[(size_t)j * t->nb + r];
+    for (int n = 0; n < t->N; ++n) ns[n] = (double)t->xb.ns[n];
+    if ((st = up(&t->BT, bt)) || (st = up(&t->ns, ns))) return fail(st);
+  }
   if ((st = up(&t->tw1n, twiddles(t->n1))) || (st = up(&t->tw1m, twiddles(t->m1))))
     return fail(st);
   if (cfg->ndim == 3 &&
@@ -516,9 +458,19 @@ extern "C" int jfb_tps_create(const jfb_tps_config* cfg, jfb_tps** out) {
     }
     t->allocs.push_back(*w);
   }
+#define JFB_YW(P)                                                       \
+  for (const void* fn : {(const void*)y_backward_warp_kernel<P, double>, \
+                         (const void*)y_forward_warp_kernel<P, double, true>}) \
+    if (allow_smem(fn) != cudaSuccess) {                                \
+      set_error("cannot configure the transform kernels");              \
+      return fail(JFB_ERR_CUDA);                                        \
+    }
+  JFB_YW(2) JFB_YW(3) JFB_YW(4) JFB_YW(6)
+#undef JFB_YW
   if (allow_smem((const void*)y_backward_kernel<double>) != cudaSuccess ||
       allow_smem((const void*)y_forward_kernel<double>) != cudaSuccess ||
-      allow_smem((const void*)fft_rows_kernel) != cudaSuccess) {
+      allow_smem((const void*)fft_rows_kernel) != cudaSuccess ||
+      allow_smem((const void*)x_apply_kernel) != cudaSuccess) {
     set_error("cannot configure the transform kernels");
     return fail(JFB_ERR_CUDA);
   }
@@ -528,13 +480,15 @@ extern "C" int jfb_tps_create(const jfb_tps_config* cfg, jfb_tps** out) {
 
 namespace jfb {
 
-// Device copy of one separable x-axis map (built and uploaded on first use).
+// Device copy of one separable x-axis map in fragment tiles (built and
+// uploaded on first use).
 static int tps_xmap(jfb_tps* t, int map, int k, const double** A, int* rows, int* cols) {
   const int64_t key = (int64_t)map * 64 + k;
   auto it = t->xmaps.find(key);
   if (it == t->xmaps.end()) {
     int r = 0, c = 0;
-    const std::vector<double> h = x_map_matrix(t->xb, map, k, &r, &c);
+    const std::vector<double> A0 = x_map_matrix(t->xb, map, k, &r, &c);
+    const std::vector<double> h = fragment_tiles(A0, r, c);
     double* d = nullptr;
     JFB_CHECK_CUDA(cudaMalloc((void**)&d, h.size() * sizeof(double)));
     cudaError_t e = cudaMemcpy(d, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice);
@@ -555,6 +509,21 @@ static double fourier_df(const jfb_tps* t, int a) {
   return std::fabs(L - 2.0 * M_PI) < 1e-12 ? 1.0 : 2.0 * M_PI / L;
 }
 
+static int tps_x(const double* A, int rows, int cols, const c64* in, c64* out,
+                 const FourierWeight& fw, cudaStream_t s) {
+  const int64_t M = (int64_t)fw.n1 * fw.n2;
+  // few columns (2-D spaces): the row tiles over several blocks
+  const unsigned gx = (unsigned)((M + kGW - 1) / kGW);
+  const unsigned gy = gx >= 148 ? 1 : std::min<unsigned>(148 / gx + 1, (rows + 63) / 64);
+  x_apply_kernel<<<dim3(gx, gy), kXThreads, (size_t)(cols + 3) / 4 * 4 * kSLd * sizeof(double), s>>>(
+      A, rows, cols, in, out, fw);
+  JFB_CHECK_LAUNCH();
+  return JFB_OK;
+}
+static FourierWeight no_weight(const jfb_tps* t, double scale) {
+  return FourierWeight{t->n1, t->n2, 0, 0, 1.0, 1.0, scale};
+}
+
 // out = w * (map_k along x) in, w the Fourier weights of orders k1, k2.
 static int tps_xw(jfb_tps* t, int map, int kx, int k1, int k2, double scale, const c64* in,
                   c64* out, cudaStream_t s) {
@@ -570,11 +539,7 @@ static int tps_xw(jfb_tps* t, int map, int kx, int k1, int k2, double scale, con
   fw.df1 = fourier_df(t, 0);
   fw.df2 = t->cfg.ndim == 3 ? fourier_df(t, 1) : 1.0;
   fw.scale = scale;
-  const int64_t M = (int64_t)t->n1 * t->n2;
-  dim3 g((unsigned)((M + 255) / 256), rows);
-  x_apply_w_kernel<<<g, 256, 0, s>>>(A, rows, cols, in, out, fw);
-  JFB_CHECK_LAUNCH();
-  return JFB_OK;
+  return tps_x(A, rows, cols, in, out, fw, s);
 }
 
 static int check_orders(const jfb_tps* t, const int32_t* k) {
@@ -584,10 +549,27 @@ static int check_orders(const jfb_tps* t, const int32_t* k) {
   return JFB_OK;
 }
 
-static int tps_x(const double* A, int rows, int cols, const c64* in, c64* out, int64_t M,
-                 cudaStream_t s) {
-  dim3 g((unsigned)((M + 255) / 256), rows);
-  x_apply_kernel<<<g, 256, 0, s>>>(A, rows, cols, in, out, M);
+// contiguous lines: padded inverse (sign +1, n -> m) or truncated forward (m -> n)
+static int tps_lines(const FFTPlan& plan, const c64* tw, int sign, int64_t lines, int n, int m,
+                     const c64* in, c64* out, cudaStream_t s) {
+  const int nin = sign > 0 ? n : m, nout = sign > 0 ? m : n;
+  switch (warp_radix(m)) {
+#define JFB_FR(P) \
+  case P:                                                                                        \
+    fft_rows_warp_kernel<P><<<(unsigned)((lines + 7) / 8), 256, 0, s>>>(tw, sign, in, out, lines, nin, nout); \
+    break;
+    JFB_FR(2) JFB_FR(3) JFB_FR(4) JFB_FR(6)
+#undef JFB_FR
+    default: {
+      // 8 lines per block, fewer where that would leave SMs idle or not fit
+      int lr = kTpsLogRows;
+      while (lr > 0 && ((lines >> lr) < 148 || ((size_t)2 * m << lr) * sizeof(c64) > 200 * 1024)) --lr;
+      const size_t sm = ((size_t)2 * m << lr) * sizeof(c64);
+      JFB_REQUIRE(sm <= 200 * 1024, "Fourier axis too long");
+      const unsigned blocks = (unsigned)((lines + (1 << lr) - 1) >> lr);
+      fft_rows_kernel<<<blocks, 256, sm, s>>>(plan, tw, sign, in, out, lines, nin, nout, lr);
+    }
+  }
   JFB_CHECK_LAUNCH();
   return JFB_OK;
 }
@@ -595,15 +577,35 @@ static int tps_x(const double* A, int rows, int cols, const c64* in, c64* out, i
 // middle axis of an array (rows, len, inner): the y kernels with Kz = inner
 static int tps_y(jfb_tps* t, int sign, int rows, int inner, const c64* in, c64* out,
                  bool padded, cudaStream_t s) {
+  const FFTPlan& plan = padded ? t->f1m : t->f1n;
+  const c64* tw = padded ? t->tw1m : t->tw1n;
+  const int m = padded ? t->m1 : t->n1;
+  if (inner == 1) return tps_lines(plan, tw, sign, rows, t->n1, m, in, out, s);
   Dims d;
   std::memset(&d, 0, sizeof(d));
   d.Nx = rows;
   d.Ny = t->n1;
   d.Kz = inner;
   d.P = t->n1 * inner;
-  d.My = padded ? t->m1 : t->n1;
-  const FFTPlan& plan = padded ? t->f1m : t->f1n;
-  const c64* tw = padded ? t->tw1m : t->tw1n;
+  d.My = m;
+  if (warp_radix(m) && inner >= 8) {
+    const int kc = std::min(16, inner);
+    const dim3 g(rows, 1, ceil_div(inner, kc));
+    const size_t sm = (size_t)(d.Ny + d.My) * (kc + 1) * sizeof(c64);
+    if (sm <= 200 * 1024) {
+      switch (warp_radix(m)) {
+#define JFB_YW(P)                                                                            \
+  case P:                                                                                    \
+    if (sign > 0) y_backward_warp_kernel<P, double><<<g, 256, sm, s>>>(d, kc, tw, in, out);   \
+    else y_forward_warp_kernel<P, double, true><<<g, 256, sm, s>>>(d, kc, tw, in, out, nullptr); \
+    break;
+        JFB_YW(2) JFB_YW(3) JFB_YW(4) JFB_YW(6)
+#undef JFB_YW
+      }
+      JFB_CHECK_LAUNCH();
+      return JFB_OK;
+    }
+  }
   int KC = inner;
   while ((size_t)2 * d.My * KC * sizeof(c64) > 96 * 1024 && KC % 2 == 0) KC /= 2;
   JFB_REQUIRE((size_t)2 * d.My * KC * sizeof(c64) <= 200 * 1024, "Fourier axis too long");
@@ -617,16 +619,10 @@ static int tps_y(jfb_tps* t, int sign, int rows, int inner, const c64* in, c64* 
 
 static int tps_z(jfb_tps* t, int sign, int64_t lines, const c64* in, c64* out, bool padded,
                  cudaStream_t s) {
-  const int n = t->n2, m = padded ? t->m2 : t->n2;
-  const FFTPlan& plan = padded ? t->f2m : t->f2n;
-  const c64* tw = padded ? t->tw2m : t->tw2n;
-  const size_t sm = (size_t)2 * m * kTpsRows * sizeof(c64);
-  JFB_REQUIRE(sm <= 200 * 1024, "Fourier axis too long");
-  const int blocks = (int)((lines + kTpsRows - 1) / kTpsRows);
-  if (sign > 0) fft_rows_kernel<<<blocks, 256, sm, s>>>(plan, tw, +1, in, out, lines, n, m);
-  else fft_rows_kernel<<<blocks, 256, sm, s>>>(plan, tw, -1, in, out, lines, m, n);
-  JFB_CHECK_LAUNCH();
-  return JFB_OK;
+  JFB_REQUIRE(((size_t)2 * (padded ? t->m2 : t->n2) << kTpsLogRows) * sizeof(c64) <= 200 * 1024,
+              "Fourier axis too long");
+  return tps_lines(padded ? t->f2m : t->f2n, padded ? t->tw2m : t->tw2n, sign, lines, t->n2,
+                   padded ? t->m2 : t->n2, in, out, s);
 }
 
 }  // namespace jfb
@@ -640,11 +636,10 @@ extern "C" int jfb_tps_backward(jfb_tps* t, const void* coeffs, void* phys, int 
   int st;
   if (t->cfg.ndim == 2) {
     // x: (nb, n1) -> (N, n1); y: -> (N, m1)
-    if ((st = tps_x(t->B, t->N, t->nb, (const c64*)coeffs, t->w0, t->n1, s))) return st;
+    if ((st = tps_x(t->B, t->N, t->nb, (const c64*)coeffs, t->w0, no_weight(t, 1.0), s))) return st;
     return tps_y(t, +1, t->N, 1, t->w0, (c64*)phys, pad, s);
   }
-  if ((st = tps_x(t->B, t->N, t->nb, (const c64*)coeffs, t->w0, (int64_t)t->n1 * t->n2, s)))
-    return st;
+  if ((st = tps_x(t->B, t->N, t->nb, (const c64*)coeffs, t->w0, no_weight(t, 1.0), s))) return st;
   if ((st = tps_y(t, +1, t->N, t->n2, t->w0, t->w1, pad, s))) return st;
   return tps_z(t, +1, (int64_t)t->N * m1, t->w1, (c64*)phys, pad, s);
 }
@@ -657,29 +652,19 @@ extern "C" int jfb_tps_forward(jfb_tps* t, const void* phys, void* coeffs, int p
   const bool pad = padded != 0;
   const int m1 = pad ? t->m1 : t->n1;
   const double* X = kind ? t->Sq : t->F;
+  // scalar products carry the Fourier weight 2 pi / df per periodic axis
+  // (Fourier.py:152-167); the forward transform does not
+  double w = 1.0;
+  if (kind == 1)
+    for (int a = 0; a + 1 < t->cfg.ndim; ++a) w *= 2.0 * M_PI / fourier_df(t, a);
   int st;
   if (t->cfg.ndim == 2) {
     if ((st = tps_y(t, -1, t->N, 1, (const c64*)phys, t->w0, pad, s))) return st;
-    if ((st = tps_x(X, t->nb, t->N, t->w0, (c64*)coeffs, t->n1, s))) return st;
-  } else {
-    if ((st = tps_z(t, -1, (int64_t)t->N * m1, (const c64*)phys, t->w0, pad, s))) return st;
-    if ((st = tps_y(t, -1, t->N, t->n2, t->w0, t->w1, pad, s))) return st;
-    if ((st = tps_x(X, t->nb, t->N, t->w1, (c64*)coeffs, (int64_t)t->n1 * t->n2, s))) return st;
+    return tps_x(X, t->nb, t->N, t->w0, (c64*)coeffs, no_weight(t, w), s);
   }
-  if (kind == 1) {
-    // scalar products carry the Fourier weight 2 pi / df per periodic axis
-    // (Fourier.py:152-167); the forward transform does not
-    double w = 1.0;
-    for (int a = 0; a + 1 < t->cfg.ndim; ++a) {
-      const double L = t->cfg.l[a];
-      const double df = std::fabs(L - 2.0 * M_PI) < 1e-12 ? 1.0 : 2.0 * M_PI / L;
-      w *= 2.0 * M_PI / df;
-    }
-    const size_t n = (size_t)t->nb * t->n1 * t->n2;
-    tps_scale_kernel<<<256, 256, 0, s>>>((c64*)coeffs, w, n);
-    JFB_CHECK_LAUNCH();
-  }
-  return JFB_OK;
+  if ((st = tps_z(t, -1, (int64_t)t->N * m1, (const c64*)phys, t->w0, pad, s))) return st;
+  if ((st = tps_y(t, -1, t->N, t->n2, t->w0, t->w1, pad, s))) return st;
+  return tps_x(X, t->nb, t->N, t->w1, (c64*)coeffs, no_weight(t, w), s);
 }
 
 extern "C" int jfb_tps_backward_primitive(jfb_tps* t, const void* coeffs, void* phys,
@@ -761,8 +746,7 @@ extern "C" int jfb_helmholtz2d_solve(const jfb_tps* tc, const jfb_tps* td, const
               "too many diagonals");
   const int N = td->N, nb = td->nb, M = td->n1;
   const int KC = (M + kHelmCTAs - 1) / kHelmCTAs, JR = (N + kHelmCTAs - 1) / kHelmCTAs;
-  // solve vectors: row stride QS = 1 mod 4 complex values, so that the rows
-  // one column step updates (even offsets apart) spread over the banks
+  // the size range of this call: problems that fit one cluster's shared memory
   const int QS = KC + ((5 - KC % 4) % 4);
   const size_t smem = ((size_t)2 * N * KC + (size_t)N * QS + (size_t)2 * M * JR) * sizeof(c64) +
                       (size_t)nb * N * sizeof(double);
@@ -770,7 +754,7 @@ extern "C" int jfb_helmholtz2d_solve(const jfb_tps* tc, const jfb_tps* td, const
   JFB_CHECK_CUDA(cudaGetDevice(&dev));
   JFB_CHECK_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   if (smem > (size_t)optin) {
-    set_error("problem too large for the one-cluster Helmholtz solve");
+    set_error("problem too large for the fused Helmholtz solve");
     return JFB_ERR_ARG;
   }
   Helm2DArgs h;
@@ -803,33 +787,24 @@ extern "C" int jfb_helmholtz2d_solve(const jfb_tps* tc, const jfb_tps* td, const
     for (int b = a + 1; b < h.nU; ++b) JFB_REQUIRE(h.uoff[a] != h.uoff[b], "repeated U offset");
   for (int a = 0; a < h.nL; ++a)
     for (int b = a + 1; b < h.nL; ++b) JFB_REQUIRE(h.loff[a] != h.loff[b], "repeated L offset");
-  h.BC = tc->B;
-  h.SD = td->Sq;
-  h.BD = td->B;
-  h.tw = td->tw1n;
-  h.plan = td->f1n;
+  h.ns = td->ns;
+  h.BDT = td->BT;
   h.L = L;
   h.U = U;
   h.N = N;
   h.nb = nb;
   h.M = M;
-  h.KC = KC;
-  h.JR = JR;
-  h.QS = QS;
-  // Fourier scalar-product weight 2 pi / df (Fourier.py:152-167), the
-  // caller's division by the Fourier mass, the 1/n1 of the forward transform
+  // Fourier scalar-product weight 2 pi / df (Fourier.py:152-167) and the
+  // caller's division by the Fourier mass
   const double Ly = td->cfg.l[0];
   const double df = std::fabs(Ly - 2.0 * M_PI) < 1e-12 ? 1.0 : 2.0 * M_PI / Ly;
-  h.scale = (2.0 * M_PI / df) / fourier_mass / M;
+  h.scale = (2.0 * M_PI / df) / fourier_mass;
   h.f = (const c64*)f_hat;
   h.u = (c64*)u;
-  static bool attr = false;
-  if (!attr) {
-    JFB_CHECK_CUDA(cudaFuncSetAttribute((const void*)helmholtz2d_kernel,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-    attr = true;
-  }
-  helmholtz2d_kernel<<<kHelmCTAs, kHelmThreads, smem, (cudaStream_t)stream>>>(h);
+  cudaStream_t cs = (cudaStream_t)stream;
+  helmholtz2d_kernel<<<M, kHelmThreads,
+                       (size_t)(N + 2 * nb + kHelmThreads) * sizeof(c64) + (size_t)2 * nb * sizeof(double), cs>>>(h);
   JFB_CHECK_LAUNCH();
-  return JFB_OK;
+  // y: inverse transform of the rows, in place
+  return tps_lines(td->f1n, td->tw1n, +1, N, M, M, h.u, h.u, cs);
 }

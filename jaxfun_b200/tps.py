@@ -208,8 +208,8 @@ class Helmholtz2D:
         self.solver = tpmats_wavenumber_factor(A)
         # the Fourier mass 2 pi / df = L of the scalar product is not in A
         self._fourier_mass = domain[1][1] - domain[1][0]
-        # one-launch path (jfb_helmholtz2d_solve) while the problem fits the
-        # shared memory of one CTA cluster; the separate launches otherwise
+        # fused path (jfb_helmholtz2d_solve) in its size range; the separate
+        # launches otherwise
         L, U = self.solver.runtime_args()
         self._L, self._U = L.contiguous(), U.contiguous()
         self._offs = (_lib.int64_array(self.solver.L_offsets),
@@ -217,7 +217,7 @@ class Helmholtz2D:
         props = torch.cuda.get_device_properties(self.device)
         optin = getattr(props, "shared_memory_per_block_optin", 0)
         n, m, nb = self.TD.N[0], self.TD.N[1], self.TD.num_dofs[0]
-        kc, jr = -(-m // 8), -(-n // 8)  # columns / rows per CTA of the 8-CTA cluster
+        kc, jr = -(-m // 8), -(-n // 8)  # an eighth of the columns / rows
         qs = kc + (5 - kc % 4) % 4  # padded row of the solve vectors
         need = 16 * (2 * n * kc + n * qs + 2 * m * jr) + 8 * n * nb
         self.fused = need <= optin
@@ -245,8 +245,8 @@ class Helmholtz2D:
     def __call__(self, f_hat: torch.Tensor) -> torch.Tensor:
         """f given by orthogonal Chebyshev x Fourier coefficients: backward,
         scalar products, per-mode solves, backward; returns u on the mesh.
-        One launch (the whole problem in the shared memory of one 8-CTA
-        cluster) when it fits, else the separate transforms and the
+        Two launches (a CTA per Fourier mode, then the y transform) in the
+        fused path's size range, else the separate transforms and the
         wavenumber solve."""
         if not self.fused:
             return self.separate(f_hat)
