@@ -267,7 +267,8 @@ int jfb_kmm_energy_gradient(jfb_kmm_plan* plan, const jfb_kmm_state* state,
 
 /* Kernel choices of a flow plan (no counterpart in the reference, whose XLA
  * compiler picks its own kernels): pencil 1 = the FP64 tensor-core pencil
- * stage (folded operators, needs nx <= 65), 0 = one warp per pencil;
+ * stage (folded operators; one kernel for nx <= 65, two kernels above in the
+ * FP64 form), 0 = the warp stage (two warps per pencil);
  * transforms 1 = the fused plane transforms (one launch per step, padded
  * sizes 64 or 96), 0 = three launches; tc_velocity 1 = the mixed form's
  * velocity products on tcgen05 (split BF16, FP32 accumulation); pdl 1 =

@@ -94,6 +94,30 @@ __device__ __forceinline__ void pdl_trigger() {
 }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+__device__ __forceinline__ uint32_t smem_u32(const void* p) {
+  return (uint32_t)__cvta_generic_to_shared(p);
+}
+// L2 prefetch of [ptr, ptr + bytes) in whole 16-byte units.
+__device__ __forceinline__ void prefetch_l2(const void* ptr, size_t bytes) {
+  uintptr_t a = reinterpret_cast<uintptr_t>(ptr);
+  const uintptr_t lo = a & ~(uintptr_t)15, hi = (a + bytes + 15) & ~(uintptr_t)15;
+  for (uintptr_t x = lo; x < hi; x += 32768) {
+    const uint32_t n = (uint32_t)min((uintptr_t)32768, hi - x);
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(x), "r"(n) : "memory");
+  }
+}
+// Asynchronous copies to shared memory (16 bytes: L2 only), and their completion.
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem)), "l"(gmem)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(smem)), "l"(gmem)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+
 // Phase stamps (off by default; built into libjfb200_stamps.so by
 // jaxfun_b200.build with stamps=True): thread 0 of every CTA writes the
 // global timer at the phase boundaries of the step kernels into

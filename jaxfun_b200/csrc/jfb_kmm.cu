@@ -554,7 +554,7 @@ static int launch_pencil(jfb_kmm_plan* pl, const StageArgs& a0, cudaStream_t s) 
   auto* k = pl->split ? (pl->d.grad ? pencil_stage_kernel<2, 1, true> : pencil_stage_kernel<2, 0, true>)
             : pl->d.nD <= 64 ? (pl->d.grad ? pencil_stage_kernel<1, 1> : pencil_stage_kernel<1, 0>)
                              : (pl->d.grad ? pencil_stage_kernel<2, 1> : pencil_stage_kernel<2, 0>);
-  k<<<blocks, kNW * 32, pl->smem_pencil, s>>>(pl->ops, pl->d, a);
+  k<<<blocks, kPencilThreads, pl->smem_pencil, s>>>(pl->ops, pl->d, a);
   JFB_CHECK_LAUNCH();
   return JFB_OK;
 }
@@ -1284,7 +1284,8 @@ static int create_plan(const jfb_kmm_config* cfg, const jfb_mhd_params* mhd,
   while ((size_t)2 * d.My * pl->KC * sizeof(c64) > 100 * 1024 && pl->KC % 2 == 0) pl->KC /= 2;
   pl->smem_y = (size_t)2 * d.My * pl->KC * sizeof(c64);
   pl->smem_z = (size_t)2 * d.Mz * kZRows * 3 * sizeof(c64);
-  pl->smem_pencil = (size_t)(6 * d.Nx * kLDW + kNW * 6 * d.Nx + d.Nx) * sizeof(c64);
+  pl->smem_pencil = (size_t)(6 * d.Nx * kLDW + kNW * 6 * d.Nx + d.Nx) * sizeof(c64) +
+                    (size_t)kPencilTables * d.Nx * sizeof(double);
   pl->smem_zf = (size_t)2 * d.Nz * (kZRows / 2) * 3 * sizeof(c64);
   // warp-shuffle FFT paths (lengths 32 P, P in {2, 3, 4, 6}; Kz <= 64)
   pl->qk = ceil_div(d.Kz, 32);

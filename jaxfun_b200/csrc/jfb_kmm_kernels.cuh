@@ -21,15 +21,16 @@
 
 namespace jfb {
 
-constexpr int kNW = 8;         // pencils (warps) per pencil_stage block
+constexpr int kNW = 8;         // pencils per pencil_stage block
+constexpr int kPencilThreads = 2 * kNW * 32;  // two warps per pencil
+constexpr int kPencilTables = 7;              // per-row tables in shared memory
 constexpr int kLDW = kNW + 1;  // padded pencil stride in shared memory
 constexpr int kMaxNR = 2;      // rows per lane in the register solves (n <= 128)
-constexpr int kSolveChunk = 16;  // back-substitution columns per prefetch
 constexpr int kLoadBatch = 4;    // staged loads per thread in flight
 // Mixed form, warp-per-pencil stage: the FP64 base-flow terms in a separate
 // branch-free pass over the sample points (1) or per loaded H value (0).
 // The pass took the 97x96x96 stage from 474 to 458 us, 129x128x128 from
-// 1173 to 1132 us (events around the launch, steady SBDF3 step).
+// 1173 to 1132 us (before the second warp per pencil).
 #ifndef JFB_WARP_XLIN_PASS
 #define JFB_WARP_XLIN_PASS 1
 #endif
@@ -131,35 +132,32 @@ __host__ __device__ inline int packed_rec_size(int n, bool blocks) {
 // Chebyshev (fam 0): d_n = sum_{m > n, m - n odd} 2 m c_m, d_0 halved
 // (Chebyshev.py:319-353); Legendre (fam 1): d_n = (2n + 1) sum_{m > n, m - n
 // odd} c_m (Legendre.py:195-227).
-// Warp-level helpers of the warp-per-pencil stage: inlined, or (with
-// JFB_WARP_HELPERS_NOINLINE) one shared copy each, for a smaller kernel.
-#ifndef JFB_WARP_HELPERS_NOINLINE
-#define JFB_WARP_HELPERS_NOINLINE 0
-#endif
-#if JFB_WARP_HELPERS_NOINLINE
-#define JFB_WARP_HELPER __noinline__
-#else
-#define JFB_WARP_HELPER __forceinline__
-#endif
-// chebder_warp has one shared copy (sixteen call sites): the smaller
-// warp-per-pencil kernel took 474 instead of 514 us per launch at 97x96x96
-// (the other helpers not inlined as well: 527 us)
-#ifndef JFB_CHEBDER_NOINLINE
-#define JFB_CHEBDER_NOINLINE 1
-#endif
-#if JFB_CHEBDER_NOINLINE
-__device__ __noinline__
-#else
-__device__
-#endif
-void chebder_warp(const c64* c, c64* d, int L, double scale, int lane, int fam) {
+// A lane holds the K <= 5 consecutive coefficients of its share in registers
+// (L <= 129: the host limits Nx) and the weights 2 m, 2 m + 1 as running
+// doubles; a loop over shared memory with an integer conversion per term took
+// several times as long (the order of the sums is unchanged).  One shared copy
+// (sixteen call sites) keeps the kernel small.
+constexpr int kChebPer = 5;
+__device__ __noinline__ void chebder_warp(const c64* c, c64* d, int L, double scale, int lane,
+                                          int fam) {
   const int K = (L + 31) / 32;
-  const int lo = lane * K, hi = min(L, lo + K);
-  c64 se = cmk(0.0, 0.0), so = cmk(0.0, 0.0);
-  for (int m = lo; m < hi; ++m) {
-    const c64 e = (fam ? 1.0 : 2.0 * m) * c[m];
-    if (m & 1) so = so + e; else se = se + e;
+  const int lo = lane * K, n = min(L, lo + K) - lo;
+  const double w0 = fam ? 1.0 : 2.0 * lo, dw = fam ? 0.0 : 2.0;
+  c64 e[kChebPer];
+#pragma unroll
+  for (int q = 0; q < kChebPer; ++q) e[q] = q < n ? c[lo + q] : cmk(0.0, 0.0);
+  // sums over this lane's coefficients, by parity relative to lo
+  c64 sa = cmk(0.0, 0.0), sb = cmk(0.0, 0.0);
+#pragma unroll
+  for (int q = 0; q < kChebPer; ++q) {
+    e[q] = (w0 + q * dw) * e[q];
+    if (q < n) {
+      if (q & 1) sb = sb + e[q];
+      else sa = sa + e[q];
+    }
   }
+  const bool odd = lo & 1;
+  const c64 se = odd ? sb : sa, so = odd ? sa : sb;
   // inclusive suffix sums over lanes >= lane
   c64 ie = se, io = so;
 #pragma unroll
@@ -173,22 +171,24 @@ void chebder_warp(const c64* c, c64* d, int L, double scale, int lane, int fam) 
       io = io + cmk(orr, oi);
     }
   }
-  c64 run_e = ie - se, run_o = io - so;  // sums over lanes > lane
+  const c64 re = ie - se, ro = io - so;  // sums over lanes > lane
+  c64 ra = odd ? ro : re, rb = odd ? re : ro;
   __syncwarp();
-  for (int n = hi - 1; n >= lo; --n) {
-    const c64 cn = c[n];
-    c64 dn = (n & 1) ? run_e : run_o;
-    if (fam) dn = (2.0 * n + 1.0) * dn;
-    else if (n == 0) dn = 0.5 * dn;
-    d[n] = scale * dn;
-    const c64 e = (fam ? 1.0 : 2.0 * n) * cn;
-    if (n & 1) run_o = run_o + e; else run_e = run_e + e;
-  }
+#pragma unroll
+  for (int q = kChebPer - 1; q >= 0; --q)
+    if (q < n) {
+      c64 dn = (q & 1) ? ra : rb;
+      if (fam) dn = (2.0 * lo + (2 * q + 1)) * dn;
+      else if (lo + q == 0) dn = 0.5 * dn;
+      d[lo + q] = scale * dn;
+      if (q & 1) rb = rb + e[q];
+      else ra = ra + e[q];
+    }
   __syncwarp();
 }
 
 // out = S_B^T a  (length Nx from nB)
-__device__ JFB_WARP_HELPER void apply_SBT(const DevOps& o, const Dims& d, const c64* a,
+__device__ __forceinline__ void apply_SBT(const DevOps& o, const Dims& d, const c64* a,
                                           c64* out, int lane) {
   for (int n = lane; n < d.Nx; n += 32) {
     c64 v = cmk(0.0, 0.0);
@@ -200,7 +200,7 @@ __device__ JFB_WARP_HELPER void apply_SBT(const DevOps& o, const Dims& d, const 
   __syncwarp();
 }
 // out = S_D^T a  (length Nx from nD)
-__device__ JFB_WARP_HELPER void apply_SDT(const Dims& d, const c64* a, c64* out, int lane) {
+__device__ __forceinline__ void apply_SDT(const Dims& d, const c64* a, c64* out, int lane) {
   for (int n = lane; n < d.Nx; n += 32) {
     c64 v = cmk(0.0, 0.0);
     if (n < d.nD) v = a[n];
@@ -210,7 +210,7 @@ __device__ JFB_WARP_HELPER void apply_SDT(const Dims& d, const c64* a, c64* out,
   __syncwarp();
 }
 // out[i] = scale * (S_B (ns .* c))[i]   (length nB)
-__device__ JFB_WARP_HELPER void apply_SB_ns(const DevOps& o, const Dims& d, const c64* c,
+__device__ __forceinline__ void apply_SB_ns(const DevOps& o, const Dims& d, const c64* c,
                                             c64* out, double scale, int lane) {
   for (int i = lane; i < d.nB; i += 32) {
     c64 v = (o.sB0[i] * o.ns[i]) * c[i];
@@ -221,7 +221,7 @@ __device__ JFB_WARP_HELPER void apply_SB_ns(const DevOps& o, const Dims& d, cons
   __syncwarp();
 }
 // out[i] = scale * (S_D (ns .* c))[i]   (length nD)
-__device__ JFB_WARP_HELPER void apply_SD_ns(const DevOps& o, const Dims& d, const c64* c,
+__device__ __forceinline__ void apply_SD_ns(const DevOps& o, const Dims& d, const c64* c,
                                             c64* out, double scale, int lane) {
   for (int i = lane; i < d.nD; i += 32) {
     const c64 v = o.ns[i] * c[i] - o.ns[i + 2] * c[i + 2];
@@ -231,18 +231,56 @@ __device__ JFB_WARP_HELPER void apply_SD_ns(const DevOps& o, const Dims& d, cons
 }
 
 // Tri-band (offsets -2, 0, 2) no-pivot LU solve of the Dirichlet mass matrix,
-// in place on `b` (length nD).  Two lanes (one per parity) per vector; `which`
-// selects the lane pair so several vectors can be solved concurrently.
-__device__ __forceinline__ void mass_solve_lane(const DevOps& o, const Dims& d, c64* b,
-                                                int par) {
-  for (int i = par + 2; i < d.nD; i += 2) b[i] = b[i] - o.lul[i] * b[i - 2];
-  int last = d.nD - 1;
-  if ((last & 1) != par) last -= 1;
-  for (int i = last; i >= 0; i -= 2) {
-    c64 v = b[i];
-    if (i + 2 < d.nD) v = v - o.mhi[i] * b[i + 2];
-    b[i] = o.luu[i] * v;
+// in place on one lane's values: rows par, par + 2, ... of one real component
+// (y: row par; rows 4 doubles apart).  The recurrence runs in a register, with
+// kMassBatch rows and factors loaded at once: 27 cycles a row and pass (8 per
+// dependent FP64 operation) against 75 with each load on the chain.
+constexpr int kMassBatch = 8;
+__device__ __forceinline__ void mass_solve_lane(const DevOps& o, int n, double* y, int par) {
+  constexpr int B = kMassBatch;
+  const int m = (n - par + 1) / 2;
+  const double *L = o.lul + par, *H = o.mhi + par, *G = o.luu + par;
+  double v[B], l[B], g[B], prev = 0.0;
+  int r = 0;
+  for (; r + B <= m; r += B) {
+#pragma unroll
+    for (int q = 0; q < B; ++q) {
+      v[q] = y[4 * (r + q)];
+      l[q] = r + q > 0 ? L[2 * (r + q)] : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < B; ++q) prev = v[q] = v[q] - l[q] * prev;
+#pragma unroll
+    for (int q = 0; q < B; ++q) y[4 * (r + q)] = v[q];
   }
+  for (; r < m; ++r) {
+    prev = y[4 * r] - (r > 0 ? L[2 * r] : 0.0) * prev;
+    y[4 * r] = prev;
+  }
+  r = m - 1;
+  prev = G[2 * r] * prev;
+  y[4 * r--] = prev;
+  for (; r >= B - 1; r -= B) {
+#pragma unroll
+    for (int q = 0; q < B; ++q) {
+      v[q] = y[4 * (r - q)];
+      l[q] = H[2 * (r - q)];
+      g[q] = G[2 * (r - q)];
+    }
+#pragma unroll
+    for (int q = 0; q < B; ++q) prev = v[q] = g[q] * (v[q] - l[q] * prev);
+#pragma unroll
+    for (int q = 0; q < B; ++q) y[4 * (r - q)] = v[q];
+  }
+  for (; r >= 0; --r) {
+    const double x = y[4 * r] - H[2 * r] * prev;
+    prev = G[2 * r] * x;
+    y[4 * r] = prev;
+  }
+}
+// The same for a whole vector by four lanes (parity, re/im) of a warp.
+__device__ __forceinline__ void mass_solve_quad(const DevOps& o, int n, c64* b, int q) {
+  mass_solve_lane(o, n, reinterpret_cast<double*>(b) + q, q >> 1);
 }
 
 // No-pivot LU solve of the biharmonic mass matrix (offsets -4..4), in place,
@@ -265,96 +303,127 @@ __device__ __forceinline__ void bmass_solve_lane(const DevOps& o, const Dims& d,
   }
 }
 
-// Solve one parity class of a packed record in registers.  Lane r holds
-// row 2r + par (and 2(r+32) + par when m > 32).  Forward elimination with
-// the unit-lower factor (L[i, i-2], L[i, i-4]) passes the solved rows down
-// the lanes with shuffles; then x = U^-1 y with the record's explicit inverse
-// of the parity's upper factor: y_c is broadcast and every lane r <= c accumulates
-// U^-1[r, c] y_c, kSolveChunk columns of the inverse loaded at a time.  Not
-// inlined: the call sites (Su, Sg, S00, two parities each) share one copy in
-// the instruction cache.
-template <int NR, bool blocks>
-__device__ __noinline__ void parity_solve_regs(const double* __restrict__ rec, int n, c64* y,
-                                               int par, int lane) {
-  const int m0 = (n + 1) / 2;
-  const int m = par ? n / 2 : m0;
-  const double* __restrict__ Ui = rec + 2 * n + (par ? inv_class_size(m0, blocks) : 0);
-  c64 yr[NR];
-  double l1[NR], l2[NR];
-#pragma unroll
-  for (int s = 0; s < NR; ++s) {
-    const int r = lane + 32 * s;
-    const int i = 2 * r + par;
-    const bool ok = r < m;
-    yr[s] = ok ? y[i] : cmk(0.0, 0.0);
-    l1[s] = ok ? __ldg(rec + 2 * i) : 0.0;
-    l2[s] = ok ? __ldg(rec + 2 * i + 1) : 0.0;
-  }
-  // forward elimination: y_r -= l1_r y_{r-1} + l2_r y_{r-2}
-  c64 ym1 = cmk(0.0, 0.0), ym2 = cmk(0.0, 0.0);
-#pragma unroll
-  for (int s = 0; s < NR; ++s) {
-    for (int r0 = 0; r0 < 32; ++r0) {
-      const int r = r0 + 32 * s;
-      if (r >= m) break;
-      if (lane == r0) yr[s] = yr[s] - l1[s] * ym1 - l2[s] * ym2;
-      c64 t;
-      t.re = __shfl_sync(0xffffffffu, yr[s].re, r0);
-      t.im = __shfl_sync(0xffffffffu, yr[s].im, r0);
-      ym2 = ym1;
-      ym1 = t;
-    }
-  }
-  // x = U^-1 y
-  c64 acc[NR];
-#pragma unroll
-  for (int s = 0; s < NR; ++s) acc[s] = cmk(0.0, 0.0);
-  for (int ch = 0; ch * kSolveChunk < m; ++ch) {
-    double u[NR][kSolveChunk];
-#pragma unroll
-    for (int s = 0; s < NR; ++s)
-#pragma unroll
-      for (int cc = 0; cc < kSolveChunk; ++cc) {
-        const int c = cc + kSolveChunk * ch;
-        const int r = lane + 32 * s;
-        u[s][cc] = (c < m && r <= c) ? __ldg(Ui + inv_entry(r, c, blocks)) : 0.0;
-      }
-#pragma unroll
-    for (int cc = 0; cc < kSolveChunk; ++cc) {
-      const int c = cc + kSolveChunk * ch;
-      if (c >= m) break;
-      const int own = c & 31, os = c >> 5;  // lane and slot of row c
-      c64 v = yr[0];
-#pragma unroll
-      for (int s = 1; s < NR; ++s)
-        if (s == os) v = yr[s];
-      c64 yc;
-      yc.re = __shfl_sync(0xffffffffu, v.re, own);
-      yc.im = __shfl_sync(0xffffffffu, v.im, own);
-#pragma unroll
-      for (int s = 0; s < NR; ++s) acc[s] = acc[s] + u[s][cc] * yc;
-    }
-  }
-#pragma unroll
-  for (int s = 0; s < NR; ++s) {
-    const int r = lane + 32 * s;
-    if (r < m) y[2 * r + par] = acc[s];
-  }
-  __syncwarp();
+// Start copying a record's unit-lower multipliers (2 n doubles) to shared memory.
+__device__ __forceinline__ void fetch_lower(double* Ls, const double* __restrict__ rec, int n,
+                                            int lane) {
+  for (int e = lane; e < 2 * n; e += 32) cp_async8(Ls + e, rec + e);
+  cp_async_commit();
 }
 
-// Solve a packed system of size n <= 64 * NR in place on y (both parities).
+// Forward elimination of a packed system with the unit-lower factor (L[i, i-2],
+// L[i, i-4] in Ls): rows par, par + 2, ... of one real component on one lane
+// (q = 2 par + re/im), rows and multipliers loaded a batch at once.
+__device__ __forceinline__ void eliminate_lane(const double* Ls, int n, c64* y, int q) {
+  constexpr int B = 8;
+  const int m = (n + 1 - (q >> 1)) / 2;
+  double* yd = reinterpret_cast<double*>(y) + q;  // row r at 4 r
+  const double* L = Ls + 2 * (q >> 1);            // row r at 4 r
+  double p1 = 0.0, p2 = 0.0;
+  int r = 0;
+  for (; r + B <= m; r += B) {
+    double v[B], a[B], b[B];
+#pragma unroll
+    for (int k = 0; k < B; ++k) {
+      v[k] = yd[4 * (r + k)];
+      a[k] = L[4 * (r + k)];
+      b[k] = L[4 * (r + k) + 1];
+    }
+#pragma unroll
+    for (int k = 0; k < B; ++k) {
+      v[k] = v[k] - a[k] * p1 - b[k] * p2;
+      p2 = p1;
+      p1 = v[k];
+    }
+#pragma unroll
+    for (int k = 0; k < B; ++k) yd[4 * (r + k)] = v[k];
+  }
+  for (; r < m; ++r) {
+    const double v = yd[4 * r] - L[4 * r] * p1 - L[4 * r + 1] * p2;
+    yd[4 * r] = v;
+    p2 = p1;
+    p1 = v;
+  }
+}
+
+// x = U^-1 y in place, with the record's explicit inverse of each parity's
+// upper factor (system of n <= 64 NR rows, one warp): y_c is read by all lanes
+// and every lane r <= c (rows lane, lane + 32) accumulates U^-1[r, c] y_c in
+// order of c; the inverse's columns are loaded 16 or 8 ahead of their use, at
+// constant offsets from one pointer (instruction issue bounds this part).
+// (Eliminations by shuffles inside the warp and columns loaded where they are
+// used took 49 us of a 165 us block at 129 points.)  Not inlined: the call
+// sites (Su, Sg, S00) share one copy.
 template <int NR, bool blocks>
-__device__ __forceinline__ void packed_solve_warp(const double* __restrict__ rec, int n,
-                                                  c64* y, int lane) {
-  parity_solve_regs<NR, blocks>(rec, n, y, 0, lane);
-  parity_solve_regs<NR, blocks>(rec, n, y, 1, lane);
+__device__ __noinline__ void inverse_product_warp(const double* __restrict__ rec, int n, c64* y,
+                                                  int lane) {
+  const int m0 = (n + 1) / 2;
+  // lane part of an entry's offset; the column's part is a constant
+  const int lo = blocks ? (lane >> 3) * 64 + (lane & 7) * 8 : lane;
+  const double* U0 = rec + 2 * n + lo;
+  // columns [C, C + 16) of slot 0, or [C, C + 8) of both slots (C >= 32)
+  auto load = [&]<int C>(const double* U, int m, double (&v)[16]) {
+#pragma unroll
+    for (int q = 0; q < 16; ++q) {
+      const int c = C < 32 ? C + q : C + (q >> 1), s = C < 32 ? 0 : q & 1;
+      const int off = blocks ? (c >> 3) * ((c >> 3) + 1) / 2 * 64 + (c & 3) * 2 + ((c >> 2) & 1) + 256 * s
+                             : c * (c + 1) / 2 + 32 * s;
+      v[q] = c < m && lane + 32 * s <= c ? __ldg(U + off) : 0.0;
+    }
+  };
+  c64 acc[NR];
+  auto use = [&]<int C>(const c64* yp, int m, const double (&v)[16]) {
+#pragma unroll
+    for (int q = 0; q < (C < 32 ? 16 : 8); ++q) {
+      const int c = C + q;
+      if (c >= m) continue;
+      const double2 t = *reinterpret_cast<const double2*>(yp + 2 * c);
+      const c64 yc = cmk(t.x, t.y);
+      acc[0] = acc[0] + v[C < 32 ? q : 2 * q] * yc;
+      if (C >= 32) acc[NR - 1] = acc[NR - 1] + v[2 * q + 1 < 16 ? 2 * q + 1 : 0] * yc;
+    }
+  };
+  double a[16], b[16];
+  load.template operator()<0>(U0, m0, a);
+#pragma unroll 1
+  for (int par = 0; par < 2; ++par) {
+    const int m = par ? n / 2 : m0;
+    const double* U = U0 + (par ? inv_class_size(m0, blocks) : 0);
+    const double* Un = U0 + inv_class_size(m0, blocks);
+    const int mn = par ? 0 : n / 2;  // rows of the next class
+    const c64* yp = y + par;
+#pragma unroll
+    for (int s = 0; s < NR; ++s) acc[s] = cmk(0.0, 0.0);
+    load.template operator()<16>(U, m, b);
+    use.template operator()<0>(yp, m, a);
+    if constexpr (NR > 1) {
+      load.template operator()<32>(U, m, a);
+      use.template operator()<16>(yp, m, b);
+      load.template operator()<40>(U, m, b);
+      use.template operator()<32>(yp, m, a);
+      load.template operator()<48>(U, m, a);
+      use.template operator()<40>(yp, m, b);
+      load.template operator()<56>(U, m, b);
+      use.template operator()<48>(yp, m, a);
+      load.template operator()<0>(Un, mn, a);
+      use.template operator()<56>(yp, m, b);
+    } else {
+      load.template operator()<0>(Un, mn, a);
+      use.template operator()<16>(yp, m, b);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int s = 0; s < NR; ++s) {
+      const int r = lane + 32 * s;
+      if (r < m) y[2 * r + par] = acc[s];
+    }
+  }
+  __syncwarp();
 }
 
 // Rows i = lane + 32 t of one pencil (n <= 128: the host limits Nx to 129),
 // all global loads of the warp issued before the arithmetic.
 // out[i] = c0 x[i] + c1 y[i] + c2 z[i]  (the y, z terms only when c1, c2 != 0)
-__device__ JFB_WARP_HELPER void comb_rows(c64* out, const c64* x, const c64* y, const c64* z,
+__device__ __forceinline__ void comb_rows(c64* out, const c64* x, const c64* y, const c64* z,
                                           double c0, double c1, double c2, int n, size_t P,
                                           int p, int lane) {
   c64 vx[4], vy[4], vz[4];
@@ -381,7 +450,7 @@ __device__ JFB_WARP_HELPER void comb_rows(c64* out, const c64* x, const c64* y, 
   }
 }
 // acc[i] = mass[i] + dt (d0 acc[i] + d1 q1[i] + d2 q2[i])  (q terms when d1, d2 != 0)
-__device__ JFB_WARP_HELPER void rhs_rows(c64* acc, const c64* mass, const c64* q1,
+__device__ __forceinline__ void rhs_rows(c64* acc, const c64* mass, const c64* q1,
                                          const c64* q2, double d0, double d1, double d2,
                                          double dt, int n, size_t P, int p, int lane) {
   c64 v1[4], v2[4];
@@ -407,39 +476,31 @@ __device__ JFB_WARP_HELPER void rhs_rows(c64* acc, const c64* mass, const c64* q
   }
 }
 
+// Barrier of the two warps of pencil w (ids 1 .. kNW; 0 is the block's).
+__device__ __forceinline__ void pair_sync(int w) {
+  asm volatile("bar.sync %0, 64;" ::"r"(w + 1) : "memory");
+}
+
 // Velocity reconstruction (channelflow_kmm.py:855-870): from u0 (TB, in A3)
-// and g (TD, in A4) form uo0 = S_B^T u0 (-> A5), f = P_TD(d/dx uo0),
+// and g (TD, in G) form uo0 = S_B^T u0 (-> A5), f = P_TD(d/dx uo0),
 // u1 = i(ky f + kz g)/k^2 (-> A0), u2 = i(kz f - ky g)/k^2 (-> A1); the
 // ky = kz = 0 pencil takes the real mean-flow vectors (v00, w00) from vw.
-#ifndef JFB_CTA_DMMA_NOINLINE
-#define JFB_CTA_DMMA_NOINLINE 0
-#endif
-#if JFB_CTA_DMMA_NOINLINE
-#define JFB_CTA_DMMA_INLINE __noinline__
-#else
-#define JFB_CTA_DMMA_INLINE __forceinline__
-#endif
-#ifndef JFB_RECON_NOINLINE
-#define JFB_RECON_NOINLINE 0
-#endif
-#if JFB_RECON_NOINLINE
-__device__ __noinline__
-#else
-__device__
-#endif
-void reconstruct_warp(const DevOps& o, const Dims& d, const c64* A3,
-                                 const c64* A4, const c64* vw, bool mean_pencil,
-                                 double kyp, double kzp, c64* A0, c64* A1, c64* A2,
-                                 c64* A5, int lane) {
-  apply_SBT(o, d, A3, A5, lane);            // A5 = uo0 = S_B^T u0
-  chebder_warp(A5, A0, d.Nx, d.dfx, lane, d.family);   // A0 = d/dx uo0
-  apply_SD_ns(o, d, A0, A2, 1.0, lane);      // A2 = S_D(ns du)
-  if (lane < 2) mass_solve_lane(o, d, A2, lane);  // f = projection into TD
-  __syncwarp();
+// Called by both warps of the pencil (role 0 owns A3, role 1 G and vw).
+__device__ __forceinline__ void reconstruct_pair(const DevOps& o, const Dims& d, const c64* A3,
+                                                 const c64* G, const c64* vw, bool mean_pencil,
+                                                 double kyp, double kzp, c64* A0, c64* A1, c64* A2,
+                                                 c64* A5, int w, int role, int lane) {
+  if (role == 0) {
+    apply_SBT(o, d, A3, A5, lane);            // A5 = uo0 = S_B^T u0
+    chebder_warp(A5, A0, d.Nx, d.dfx, lane, d.family);   // A0 = d/dx uo0
+    apply_SD_ns(o, d, A0, A2, 1.0, lane);      // A2 = S_D(ns du)
+    if (lane < 4) mass_solve_quad(o, d.nD, A2, lane);  // f = projection into TD
+  }
+  pair_sync(w);
   const double k2 = kyp * kyp + kzp * kzp;
   const double inv = (k2 == 0.0) ? 1.0 : 1.0 / k2;
-  for (int i = lane; i < d.nD; i += 32) {
-    const c64 f = A2[i], g = A4[i];
+  for (int i = lane + 32 * role; i < d.nD; i += 64) {
+    const c64 f = A2[i], g = G[i];
     c64 u1 = mul_i((kyp * inv) * f + (kzp * inv) * g);
     c64 u2 = mul_i((kzp * inv) * f - (kyp * inv) * g);
     if (mean_pencil) {
@@ -449,147 +510,13 @@ void reconstruct_warp(const DevOps& o, const Dims& d, const c64* A3,
     A0[i] = u1;
     A1[i] = u2;
   }
-  __syncwarp();
+  pair_sync(w);
 }
 
-// ---------------------------------------------------------------------------
-// CTA-level small GEMMs against the x-transform matrices.
-// out[(f * R + r) * kLDW + w] = sum_k A[r * K + k] * in(f, k, w)
-// ---------------------------------------------------------------------------
-template <typename InFn>
-__device__ __forceinline__ void cta_gemm(const double* __restrict__ A, int R, int K, int NF,
-                                         InFn in, c64* out) {
-  const int C = NF * kNW;
-  const int G = blockDim.x / C;
-  const int t = threadIdx.x;
-  const int col = t % C, g = t / C;
-  if (g < G) {
-    const int f = col / kNW, w = col % kNW;
-    for (int r0 = g; r0 < R; r0 += 8 * G) {
-      c64 acc[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) acc[q] = cmk(0.0, 0.0);
-      for (int k = 0; k < K; ++k) {
-        const c64 x = in(f, k, w);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const int r = r0 + q * G;
-          if (r < R) {
-            const double a = __ldg(A + (size_t)r * K + k);
-            acc[q] = cmk(acc[q].re + a * x.re, acc[q].im + a * x.im);
-          }
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int r = r0 + q * G;
-        if (r < R) out[(f * R + r) * kLDW + w] = acc[q];
-      }
-    }
-  }
-}
-
-// Parity-split x-backward: with x_{N-1-j} = -x_j and T_n(-x) = (-1)^n T_n(x),
-// u(x_j) = E_j + O_j and u(x_{N-1-j}) = E_j - O_j, where E (O) sums the even
-// (odd) coefficients.  Halves the Vandermonde work.
-// out[(f * N + j) * kLDW + w] for the NF fields of in(f, n, w).
-template <typename InFn>
-__device__ __forceinline__ void cta_backward_parity(const double* __restrict__ VE,
-                                                    const double* __restrict__ VO, int N,
-                                                    int NF, InFn in, c64* out) {
-  const int C = NF * kNW;
-  const int G = blockDim.x / C;
-  const int t = threadIdx.x;
-  const int col = t % C, g = t / C;
-  const int Jh = (N + 1) / 2, Ne = (N + 1) / 2, No = N / 2;
-  if (g >= G) return;
-  const int f = col / kNW, w = col % kNW;
-  for (int j0 = g; j0 < Jh; j0 += 4 * G) {
-    c64 E[4], O[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) E[q] = O[q] = cmk(0.0, 0.0);
-    for (int m = 0; m < Ne; ++m) {
-      const c64 x = in(f, 2 * m, w);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int j = j0 + q * G;
-        if (j < Jh) {
-          const double a = __ldg(VE + (size_t)j * Ne + m);
-          E[q] = cmk(E[q].re + a * x.re, E[q].im + a * x.im);
-        }
-      }
-    }
-    for (int m = 0; m < No; ++m) {
-      const c64 x = in(f, 2 * m + 1, w);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int j = j0 + q * G;
-        if (j < Jh) {
-          const double a = __ldg(VO + (size_t)j * No + m);
-          O[q] = cmk(O[q].re + a * x.re, O[q].im + a * x.im);
-        }
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int j = j0 + q * G;
-      if (j < Jh) {
-        out[(f * N + j) * kLDW + w] = E[q] + O[q];
-        if (N - 1 - j != j) out[(f * N + N - 1 - j) * kLDW + w] = E[q] - O[q];
-      }
-    }
-  }
-}
-
-// Parity-split x-forward scalar products: sp[2m] = sum_j QE[m][j] (u_j +
-// u_{N-1-j}) (middle node once), sp[2m+1] = sum_j QO[m][j] (u_j - u_{N-1-j}).
-// Input phys(f, j, w); output out[(f * N + n) * kLDW + w].
-template <typename InFn>
-__device__ __forceinline__ void cta_forward_parity(const double* __restrict__ QE,
-                                                   const double* __restrict__ QO, int N,
-                                                   int NF, InFn phys, c64* out) {
-  const int C = NF * kNW;
-  const int G = blockDim.x / C;
-  const int t = threadIdx.x;
-  const int col = t % C, g = t / C;
-  const int Jh = (N + 1) / 2, Jl = N / 2, Ne = (N + 1) / 2, No = N / 2;
-  if (g >= G) return;
-  const int f = col / kNW, w = col % kNW;
-  // virtual rows: [0, Ne) even outputs, [Ne, Ne + No) odd outputs
-  const int R = Ne + No;
-  for (int r0 = g; r0 < R; r0 += 4 * G) {
-    c64 acc[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) acc[q] = cmk(0.0, 0.0);
-    for (int j = 0; j < Jh; ++j) {
-      const c64 a = phys(f, j, w);
-      const c64 b = (N - 1 - j != j) ? phys(f, N - 1 - j, w) : cmk(0.0, 0.0);
-      const c64 sum = a + b, dif = a - b;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int r = r0 + q * G;
-        if (r < Ne) {
-          const double c = __ldg(QE + (size_t)r * Jh + j);
-          acc[q] = cmk(acc[q].re + c * sum.re, acc[q].im + c * sum.im);
-        } else if (r < R && j < Jl) {
-          const double c = __ldg(QO + (size_t)(r - Ne) * Jl + j);
-          acc[q] = cmk(acc[q].re + c * dif.re, acc[q].im + c * dif.im);
-        }
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int r = r0 + q * G;
-      if (r < R) {
-        const int n = (r < Ne) ? 2 * r : 2 * (r - Ne) + 1;
-        out[(f * N + n) * kLDW + w] = acc[q];
-      }
-    }
-  }
-}
-
-constexpr int kDmmaChunk = 8;  // k steps whose operands are loaded together
-constexpr int kDmmaGroup = 6;  // column tiles sharing one operator fragment load
+constexpr int kDmmaChunk = 8;  // k tiles of the operator loaded ahead
+// column tiles sharing one operator fragment load: units that spread evenly
+// over 16 warps (9 x 3 and 17 x 2 at 129 points)
+constexpr int kBwdGroup = 4, kFwdGroup = 3;
 // doubles per B-operand row of the x-backward: 6 fields x kNW pencils x re/im,
 // + 4 so that the four rows of a fragment fall in distinct bank halves
 constexpr int kLDB = 2 * 6 * kNW + 4;
@@ -607,6 +534,36 @@ __device__ __forceinline__ void dmma_8x8x4(double& d0, double& d1, double a, dou
       : "d"(a), "d"(b));
 }
 
+// d[q] += A B over K columns of one 8-row operator tile and nq <= G column
+// tiles, in order of k.  A points at this lane's element of k tile 0 (row
+// valid: ok), B at its element of k tile 0 and column tile 0 (k tiles bstep
+// doubles apart, rows bld).  The operator elements (from L2) are kDmmaChunk k
+// tiles ahead of their use; the rows past K in the last tile count as zero.
+template <int G>
+__device__ __forceinline__ void dmma_stream(const double* __restrict__ A, bool ok, int K, int t4,
+                                            const double* B, int bstep, int bld, int nq,
+                                            double (&d0)[G], double (&d1)[G]) {
+  const int KT = (K + 3) / 4;
+  double a[kDmmaChunk];
+  auto ld = [&](int kt) { return ok && 4 * kt + t4 < K ? __ldg(A + 4 * kt) : 0.0; };
+#pragma unroll
+  for (int u = 0; u < kDmmaChunk; ++u) a[u] = ld(u);
+#pragma unroll 1
+  for (int k0 = 0; k0 < KT; k0 += kDmmaChunk) {
+#pragma unroll
+    for (int u = 0; u < kDmmaChunk; ++u) {
+      const int kt = k0 + u;
+      if (kt >= KT) break;
+      // the last tile's rows past K: any row below K against a zero
+      const double* b = B + (size_t)kt * bstep - max(0, 4 * kt + t4 - (K - 1)) * bld;
+#pragma unroll
+      for (int q = 0; q < G; ++q)
+        if (q < nq) dmma_8x8x4(d0[q], d1[q], a[u], b[8 * q]);
+      a[u] = ld(kt + kDmmaChunk);
+    }
+  }
+}
+
 // Parity-split x-backward on the FP64 tensor cores.  Columns of the product
 // are (pencil w, field f, re/im) with re/im the lowest bit, so each lane's
 // accumulator pair is one complex output value.  E (even coefficients) and O
@@ -615,57 +572,35 @@ __device__ __forceinline__ void dmma_8x8x4(double& d0, double& d1, double a, dou
 // orthogonal coefficient, c = (w NF + f) 2 + re/im, so the fragment of a
 // k step is one 8-byte load per lane from four rows (two wavefronts).
 // Output: out[(f N + j) ldo + w].  A warp's unit of work is one 8-row tile of
-// the operator against up to kDmmaGroup column tiles: each operator fragment
+// the operator against up to kBwdGroup column tiles: each operator fragment
 // (read from L2, shared by all CTAs) is loaded once per unit.
-__device__ JFB_CTA_DMMA_INLINE void cta_backward_dmma(const double* __restrict__ VE,
+__device__ __forceinline__ void cta_backward_dmma(const double* __restrict__ VE,
                                                   const double* __restrict__ VO, int N,
                                                   int NF, const double* Bs, c64* out,
                                                   int ldo) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   const int Jh = (N + 1) / 2, Ne = (N + 1) / 2, No = N / 2;
   const int mt = (Jh + 7) / 8, nt = (NF * kNW * 2) / 8;
-  const int ng = (nt + kDmmaGroup - 1) / kDmmaGroup;
+  const int ng = (nt + kBwdGroup - 1) / kBwdGroup;
   const int g = lane >> 2, t4 = lane & 3;
   for (int unit = warp; unit < mt * ng; unit += nwarps) {
-    const int m0 = (unit / ng) * 8, nb = (unit % ng) * kDmmaGroup;
-    const int nq = min(kDmmaGroup, nt - nb);
+    const int m0 = (unit / ng) * 8, nb = (unit % ng) * kBwdGroup;
+    const int nq = min(kBwdGroup, nt - nb);
     const int ja = m0 + g;  // A row of the a fragment
-    double e0[kDmmaGroup], e1[kDmmaGroup], o0[kDmmaGroup], o1[kDmmaGroup];
+    double e0[kBwdGroup], e1[kBwdGroup], o0[kBwdGroup], o1[kBwdGroup];
 #pragma unroll
-    for (int q = 0; q < kDmmaGroup; ++q) e0[q] = e1[q] = o0[q] = o1[q] = 0.0;
+    for (int q = 0; q < kBwdGroup; ++q) e0[q] = e1[q] = o0[q] = o1[q] = 0.0;
 #pragma unroll
     for (int par = 0; par < 2; ++par) {
       const int K = par ? No : Ne;
-      const double* A = par ? VO : VE;
-      for (int kb = 0; kb < K; kb += 4 * kDmmaChunk) {
-        double av[kDmmaChunk];
-#pragma unroll
-        for (int u = 0; u < kDmmaChunk; ++u) {
-          const int k = kb + 4 * u + t4;
-          av[u] = (ja < Jh && k < K) ? __ldg(A + (size_t)ja * K + k) : 0.0;
-        }
-#pragma unroll
-        for (int q = 0; q < kDmmaGroup; ++q) {
-          if (q >= nq) break;
-          const double* brow = Bs + (nb + q) * 8 + g + par * kLDB;  // + 2 k kLDB
-          double bv[kDmmaChunk];
-#pragma unroll
-          for (int u = 0; u < kDmmaChunk; ++u) {
-            const int k = kb + 4 * u + t4;
-            bv[u] = (k < K) ? brow[2 * k * kLDB] : 0.0;
-          }
-#pragma unroll
-          for (int u = 0; u < kDmmaChunk; ++u)
-            if (kb + 4 * u < K) {
-              if (par) dmma_8x8x4(o0[q], o1[q], av[u], bv[u]);
-              else dmma_8x8x4(e0[q], e1[q], av[u], bv[u]);
-            }
-        }
-      }
+      const double* A = (par ? VO : VE) + (size_t)min(ja, Jh - 1) * K + t4;
+      const double* brow = Bs + nb * 8 + g + (2 * t4 + par) * kLDB;  // + 8 kt kLDB: k = 4 kt + t4
+      dmma_stream<kBwdGroup>(A, ja < Jh, K, t4, brow, 8 * kLDB, 2 * kLDB, nq, par ? o0 : e0,
+                             par ? o1 : e1);
     }
     const int j = m0 + g;
 #pragma unroll
-    for (int q = 0; q < kDmmaGroup; ++q) {
+    for (int q = 0; q < kBwdGroup; ++q) {
       if (q >= nq) break;
       const int colc = (nb + q) * 8 + 2 * t4;  // even column: re, next: im
       const int wc = colc / (2 * NF), fc = (colc / 2) % NF;
@@ -683,51 +618,31 @@ __device__ JFB_CTA_DMMA_INLINE void cta_backward_dmma(const double* __restrict__
 // floor(N/2) rows) sit in shared memory as rows of kLDF doubles, column
 // c = (w NF + f) 2 + re/im.  Output: out[(f N + n) kLDW + w].  Units of
 // work as in cta_backward_dmma.
-__device__ JFB_CTA_DMMA_INLINE void cta_forward_dmma(const double* __restrict__ QE,
+__device__ __forceinline__ void cta_forward_dmma(const double* __restrict__ QE,
                                                  const double* __restrict__ QO, int N, int NF,
                                                  const double* Se, const double* So, c64* out) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   const int Jh = (N + 1) / 2, Jl = N / 2, Ne = (N + 1) / 2, No = N / 2;
   const int mte = (Ne + 7) / 8, mto = (No + 7) / 8, nt = (NF * kNW * 2) / 8;
-  const int ng = (nt + kDmmaGroup - 1) / kDmmaGroup;
+  const int ng = (nt + kFwdGroup - 1) / kFwdGroup;
   const int g = lane >> 2, t4 = lane & 3;
   for (int unit = warp; unit < (mte + mto) * ng; unit += nwarps) {
-    const int mi = unit / ng, nb = (unit % ng) * kDmmaGroup;
-    const int nq = min(kDmmaGroup, nt - nb);
+    const int mi = unit / ng, nb = (unit % ng) * kFwdGroup;
+    const int nq = min(kFwdGroup, nt - nb);
     const bool odd = mi >= mte;
     const int m0 = (odd ? mi - mte : mi) * 8;
     const int M = odd ? No : Ne, K = odd ? Jl : Jh;
     const double* A = odd ? QO : QE;
     const double* B = odd ? So : Se;
     const int ma = m0 + g;
-    double d0[kDmmaGroup], d1[kDmmaGroup];
+    double d0[kFwdGroup], d1[kFwdGroup];
 #pragma unroll
-    for (int q = 0; q < kDmmaGroup; ++q) d0[q] = d1[q] = 0.0;
-    for (int kb = 0; kb < K; kb += 4 * kDmmaChunk) {
-      double av[kDmmaChunk];
-#pragma unroll
-      for (int u = 0; u < kDmmaChunk; ++u) {
-        const int k = kb + 4 * u + t4;
-        av[u] = (ma < M && k < K) ? __ldg(A + (size_t)ma * K + k) : 0.0;
-      }
-#pragma unroll
-      for (int q = 0; q < kDmmaGroup; ++q) {
-        if (q >= nq) break;
-        const double* brow = B + (nb + q) * 8 + g;
-        double bv[kDmmaChunk];
-#pragma unroll
-        for (int u = 0; u < kDmmaChunk; ++u) {
-          const int k = kb + 4 * u + t4;
-          bv[u] = (k < K) ? brow[k * kLDF] : 0.0;
-        }
-#pragma unroll
-        for (int u = 0; u < kDmmaChunk; ++u)
-          if (kb + 4 * u < K) dmma_8x8x4(d0[q], d1[q], av[u], bv[u]);
-      }
-    }
+    for (int q = 0; q < kFwdGroup; ++q) d0[q] = d1[q] = 0.0;
+    dmma_stream<kFwdGroup>(A + (size_t)min(ma, M - 1) * K + t4, ma < M, K, t4,
+                           B + nb * 8 + g + t4 * kLDF, 4 * kLDF, kLDF, nq, d0, d1);
     const int m = m0 + g;
 #pragma unroll
-    for (int q = 0; q < kDmmaGroup; ++q) {
+    for (int q = 0; q < kFwdGroup; ++q) {
       if (q >= nq) break;
       const int colc = (nb + q) * 8 + 2 * t4;
       const int wc = colc / (2 * NF), fc = (colc / 2) % NF;
@@ -740,20 +655,50 @@ __device__ JFB_CTA_DMMA_INLINE void cta_forward_dmma(const double* __restrict__ 
 }
 
 // ---------------------------------------------------------------------------
-// pencil_stage: see file header.  Block = kNW warps, one pencil per warp.
+// pencil_stage: see file header.  A block takes kNW pencils with two warps
+// each: role 0 the u system and the reconstruction, role 1 the g system and
+// the mean flow, with scratch arrays of their own (role 1 in R1, which holds
+// nothing between the scalar products and the x-backward).  Bound by the
+// serial chains of the recurrences and by shared memory (one block per SM), so
+// a second warp per pencil shortens the chains and fills their gaps.  With the
+// recurrences of all pencils on one lane per value (masses: 12 lanes a pencil,
+// eliminations: 4 a system), the per-row tables in shared memory and the
+// inverse read at constant offsets, the mixed 129x128x128 stage went from 972
+// to 700 us and the 65x64x64 prologue from 32 to 27 us, every sum in the order
+// it had (the mixed form's FP64 -> FP32 roundings depend on it).  What is left:
+// the inverse's 520 KB a block from L2 (28 of 107 us), the x products (22).
 // ---------------------------------------------------------------------------
 // kForm: 0 rotational, 1 gradient (each compiled without the other's code);
 // kBlocks: the layout of the factor records (inv_entry; a runtime flag cost 10 %).
 template <int NR, int kForm, bool kBlocks = false>
-__global__ void __launch_bounds__(256, 1) pencil_stage_kernel(DevOps o, Dims d, StageArgs a) {
+__global__ void __launch_bounds__(kPencilThreads, 1) pencil_stage_kernel(DevOps o, Dims d, StageArgs a) {
   const bool grad = kForm == 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   c64* R1 = reinterpret_cast<c64*>(smem_raw);  // 6 * Nx * kLDW
   c64* ARR = R1 + 6 * d.Nx * kLDW;              // kNW * 6 * Nx
   c64* sVW = ARR + kNW * 6 * d.Nx;              // Nx
+  // the per-row tables of the recurrences and stencils
+  double* tab = reinterpret_cast<double*>(sVW + d.Nx);
+  {
+    auto stage = [&](const double* src, int n, int q) {
+      for (int i = threadIdx.x; i < n; i += kPencilThreads) tab[q * d.Nx + i] = src[i];
+      return tab + q * d.Nx;
+    };
+    o.lul = stage(o.lul, d.nD, 0);
+    o.mhi = stage(o.mhi, d.nD, 1);
+    o.luu = stage(o.luu, d.nD, 2);
+    o.ns = stage(o.ns, d.Nx, 3);
+    o.sB0 = stage(o.sB0, d.nB, 4);
+    o.sB2 = stage(o.sB2, d.nB, 5);
+    o.sB4 = stage(o.sB4, d.nB, 6);
+    __syncthreads();
+  }
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kyi = blockIdx.x / d.nKb;
+  const int warp = (threadIdx.x >> 5) % kNW, role = (threadIdx.x >> 5) / kNW;
+  const int lane = threadIdx.x & 31;
+  // ky, -ky, ky + 1, ...: the blocks that share factor records run together
+  const int yq = blockIdx.x / d.nKb;
+  const int kyi = (yq & 1) ? (yq + 1) / 2 : (d.Ny - yq / 2) % d.Ny;
   const int kz0 = (blockIdx.x % d.nKb) * kNW;
   const int p0 = kyi * d.Kz + kz0;
   const int nvalid = min(kNW, d.Kz - kz0);
@@ -772,24 +717,32 @@ __global__ void __launch_bounds__(256, 1) pencil_stage_kernel(DevOps o, Dims d, 
   c64* A3 = A2 + d.Nx;
   c64* A4 = A3 + d.Nx;
   c64* A5 = A4 + d.Nx;
+  c64* B0 = R1 + (warp * 6 + 0) * d.Nx;  // role 1's arrays
+  c64* B1 = B0 + d.Nx;
+  c64* B2 = B1 + d.Nx;
+  c64* B4 = B2 + 2 * d.Nx;
+  c64* B5 = B4 + d.Nx;
   const size_t P = (size_t)d.P;
 
   // ---------------- reconstruction only (u1, u2 of a stored state) --------
   if (a.mode == kReconstruct) {
     if (active) {
-      for (int i = lane; i < d.nB; i += 32) A3[i] = a.u0a[(size_t)i * P + p];
-      for (int i = lane; i < d.nD; i += 32) {
-        A4[i] = a.ga[(size_t)i * P + p];
-        if (mean_pencil) sVW[i] = a.vwa[i];
+      if (role == 0) {
+        for (int i = lane; i < d.nB; i += 32) A3[i] = a.u0a[(size_t)i * P + p];
+      } else {
+        for (int i = lane; i < d.nD; i += 32) {
+          B4[i] = a.ga[(size_t)i * P + p];
+          if (mean_pencil) sVW[i] = a.vwa[i];
+        }
       }
       __syncwarp();
-      reconstruct_warp(o, d, A3, A4, sVW, mean_pencil, kyp, kzp, A0, A1, A2, A5, lane);
-      for (int i = lane; i < d.nD; i += 32) {
+      reconstruct_pair(o, d, A3, B4, sVW, mean_pencil, kyp, kzp, A0, A1, A2, A5, warp, role, lane);
+      for (int i = lane + 32 * role; i < d.nD; i += 64) {
         a.X[(size_t)i * P + p] = A0[i];
         a.Hd_out[(size_t)i * P + p] = A1[i];
       }
     } else if (warp < nvalid) {
-      for (int i = lane; i < d.nD; i += 32) {
+      for (int i = lane + 32 * role; i < d.nD; i += 64) {
         a.X[(size_t)i * P + p] = cmk(0.0, 0.0);
         a.Hd_out[(size_t)i * P + p] = cmk(0.0, 0.0);
       }
@@ -799,6 +752,12 @@ __global__ void __launch_bounds__(256, 1) pencil_stage_kernel(DevOps o, Dims d, 
 
   // ---------------- phase A: nonlinear term of the current state ----------
   if (a.mode != kPrologue) {
+    double* Ls = reinterpret_cast<double*>(role ? R1 + (warp * 6 + 3) * d.Nx : A4);
+    const double* rec = role ? a.fac.sg + (size_t)mode_idx * a.fac.sg_rec
+                             : a.fac.su + (size_t)mode_idx * a.fac.su_rec;
+    // the factor records are needed after two thirds of the block's time
+    if (active && a.mode == kImplicit && lane == 0)
+      prefetch_l2(rec, packed_rec_size(role ? d.nD : d.nB, kBlocks) * sizeof(double));
     // cooperative load of the x-physical H fields into R1[0..2], kLoadBatch
     // values per thread in flight
     auto load_h = [&](int idx) {
@@ -933,22 +892,26 @@ __global__ void __launch_bounds__(256, 1) pencil_stage_kernel(DevOps o, Dims d, 
       // TB.forward(u0), TD.forward(u1), TD.forward(u2), mask, g = i ky u2 - i kz u1
       // (channelflow_kmm.py:677-683)
       if (active) {
-        for (int i = lane; i < d.nB; i += 32) {
-          const c64* t = sT + warp;
-          A0[i] = o.sB0[i] * t[i * kLDW] + o.sB2[i] * t[(i + 2) * kLDW] +
-                  o.sB4[i] * t[(i + 4) * kLDW];
+        if (role == 0) {
+          for (int i = lane; i < d.nB; i += 32) {
+            const c64* t = sT + warp;
+            A0[i] = o.sB0[i] * t[i * kLDW] + o.sB2[i] * t[(i + 2) * kLDW] +
+                    o.sB4[i] * t[(i + 4) * kLDW];
+          }
+          __syncwarp();
+          if (lane < 2) bmass_solve_lane(o, d, A0, lane);
+        } else {
+          for (int f = 1; f < 3; ++f) {
+            c64* out = (f == 1) ? A1 : A2;
+            for (int i = lane; i < d.nD; i += 32)
+              out[i] = sT[(f * d.Nx + i) * kLDW + warp] - sT[(f * d.Nx + i + 2) * kLDW + warp];
+          }
+          __syncwarp();
+          if (lane < 8) mass_solve_quad(o, d.nD, (lane < 4) ? A1 : A2, lane & 3);
         }
-        for (int f = 1; f < 3; ++f) {
-          c64* out = (f == 1) ? A1 : A2;
-          for (int i = lane; i < d.nD; i += 32)
-            out[i] = sT[(f * d.Nx + i) * kLDW + warp] - sT[(f * d.Nx + i + 2) * kLDW + warp];
-        }
-        __syncwarp();
-        if (lane < 2) bmass_solve_lane(o, d, A0, lane);
-        else if (lane < 6) mass_solve_lane(o, d, (lane < 4) ? A1 : A2, lane & 1);
-        __syncwarp();
-        for (int i = lane; i < d.nB; i += 32) a.u0_out[(size_t)i * P + p] = A0[i];
-        for (int i = lane; i < d.nD; i += 32) {
+        pair_sync(warp);
+        for (int i = lane + 32 * role; i < d.nB; i += 64) a.u0_out[(size_t)i * P + p] = A0[i];
+        for (int i = lane + 32 * role; i < d.nD; i += 64) {
           const c64 u1 = A1[i], u2 = A2[i];
           a.u1_out[(size_t)i * P + p] = u1;
           a.u2_out[(size_t)i * P + p] = u2;
@@ -956,7 +919,7 @@ __global__ void __launch_bounds__(256, 1) pencil_stage_kernel(DevOps o, Dims d, 
           if (mean_pencil) a.vw_out[i] = cmk(u1.re, u2.re);
         }
       } else if (warp < nvalid) {
-        for (int i = lane; i < d.nD; i += 32) {
+        for (int i = lane + 32 * role; i < d.nD; i += 64) {
           if (i < d.nB) a.u0_out[(size_t)i * P + p] = cmk(0.0, 0.0);
           a.u1_out[(size_t)i * P + p] = cmk(0.0, 0.0);
           a.u2_out[(size_t)i * P + p] = cmk(0.0, 0.0);
@@ -969,31 +932,34 @@ __global__ void __launch_bounds__(256, 1) pencil_stage_kernel(DevOps o, Dims d, 
       // S_D (T_n, H)_w -> A0..A2, then Dirichlet mass solves
       for (int f = 0; f < 3; ++f) {
         c64* out = (f == 0) ? A0 : (f == 1) ? A1 : A2;
-        for (int i = lane; i < d.nD; i += 32)
+        for (int i = lane + 32 * role; i < d.nD; i += 64)
           out[i] = sT[(f * d.Nx + i) * kLDW + warp] - sT[(f * d.Nx + i + 2) * kLDW + warp];
       }
-      __syncwarp();
-      if (lane < 6) {
-        c64* b = (lane >> 1) == 0 ? A0 : (lane >> 1) == 1 ? A1 : A2;
-        mass_solve_lane(o, d, b, lane & 1);
-      }
-      __syncwarp();
     }
+    __syncthreads();
+    // (vector, parity, re/im) of all pencils over the first lanes of the block
+    // (masked pencils' arrays hold finite leftovers and are not read)
+    if (threadIdx.x < kNW * 12) {
+      const int q = threadIdx.x % 12, w = threadIdx.x / 12;
+      if (w < nvalid && !nyq) mass_solve_quad(o, d.nD, ARR + (w * 6 + q / 4) * d.Nx, q & 3);
+    }
+    __syncthreads();  // R1 becomes role 1's scratch
+    if (active && a.mode == kImplicit) fetch_lower(Ls, rec, role ? d.nD : d.nB, lane);
     if (a.mode == kHOnly) {
       if (active)
         for (int f = 0; f < 3; ++f) {
           const c64* src = (f == 0) ? A0 : (f == 1) ? A1 : A2;
-          for (int i = lane; i < d.nD; i += 32) a.Hd_out[((size_t)f * d.nD + i) * P + p] = src[i];
+          for (int i = lane + 32 * role; i < d.nD; i += 64) a.Hd_out[((size_t)f * d.nD + i) * P + p] = src[i];
         }
       else if (warp < nvalid)
         for (int f = 0; f < 3; ++f)
-          for (int i = lane; i < d.nD; i += 32)
+          for (int i = lane + 32 * role; i < d.nD; i += 64)
             a.Hd_out[((size_t)f * d.nD + i) * P + p] = cmk(0.0, 0.0);
       return;
     }
     if (active) {
       // mean-flow nonlinear rows: -(M00 Re H1), -(M00 Re H2)  packed as re/im
-      if (mean_pencil) {
+      if (mean_pencil && role == 1) {
         for (int i = lane; i < d.nD; i += 32) {
           double v = o.mdi[i] * A1[i].re, w = o.mdi[i] * A2[i].re;
           if (i >= 2) {
@@ -1009,161 +975,190 @@ __global__ void __launch_bounds__(256, 1) pencil_stage_kernel(DevOps o, Dims d, 
         }
         __syncwarp();
       }
-      // orthogonal coefficients Ho_f = S_D^T H_f : A3 <- Ho0, A4 <- Ho1, A5 <- Ho2
-      apply_SDT(d, A0, A3, lane);
-      apply_SDT(d, A1, A4, lane);
-      apply_SDT(d, A2, A5, lane);
-      // t = i ky Ho1 + i kz Ho2  -> A0 ;  Hg = i kz Ho1 - i ky Ho2 -> A1
+      // orthogonal coefficients Ho_f = S_D^T H_f of the projected rows in A0..A2
+      auto ho = [&](const c64* Hf, int n) {
+        c64 v = cmk(0.0, 0.0);
+        if (n < d.nD) v = Hf[n];
+        if (n >= 2 && n - 2 < d.nD) v = v - Hf[n - 2];
+        return v;
+      };
+      // t = i ky Ho1 + i kz Ho2  -> A3 ;  Hg = i kz Ho1 - i ky Ho2 -> B1
       for (int n = lane; n < d.Nx; n += 32) {
-        const c64 h1 = A4[n], h2 = A5[n];
-        A0[n] = mul_i(kyp * h1 + kzp * h2);
-        A1[n] = mul_i(kzp * h1 - kyp * h2);
+        const c64 h1 = ho(A1, n), h2 = ho(A2, n);
+        if (role == 0) A3[n] = mul_i(kyp * h1 + kzp * h2);
+        else B1[n] = mul_i(kzp * h1 - kyp * h2);
       }
-      __syncwarp();
-      chebder_warp(A0, A2, d.Nx, d.dfx, lane, d.family);  // A2 = d/dx t
-      for (int n = lane; n < d.Nx; n += 32) A2[n] = A2[n] + k2 * A3[n];  // Hu
-      __syncwarp();
-      // Nu = Myz S_B(ns Hu) -> A3 ; Ng = Myz S_D(ns Hg) -> A4
-      apply_SB_ns(o, d, A2, A3, d.Myz, lane);
-      apply_SD_ns(o, d, A1, A4, d.Myz, lane);
-      if (a.Nu_out)
-        for (int i = lane; i < d.nB; i += 32) a.Nu_out[(size_t)i * P + p] = A3[i];
-      if (a.Ng_out)
-        for (int i = lane; i < d.nD; i += 32) a.Ng_out[(size_t)i * P + p] = A4[i];
+      pair_sync(warp);  // A1, A2 are role 0's from here
+      if (role == 0) {
+        chebder_warp(A3, A2, d.Nx, d.dfx, lane, d.family);  // A2 = d/dx t
+        for (int n = lane; n < d.Nx; n += 32) A2[n] = A2[n] + k2 * ho(A0, n);  // Hu
+        __syncwarp();
+        apply_SB_ns(o, d, A2, A3, d.Myz, lane);  // Nu = Myz S_B(ns Hu)
+        if (a.Nu_out)
+          for (int i = lane; i < d.nB; i += 32) a.Nu_out[(size_t)i * P + p] = A3[i];
 
-      // ---- right-hand side of Su: Mu (c0 ua + c1 ub + c2 uc) + cL Lu ua + dt N ----
-      comb_rows(A0, a.u0a, a.u0b, a.u0c, a.c0, a.c1, a.c2, d.nB, P, p, lane);
-      __syncwarp();
-      apply_SBT(o, d, A0, A2, lane);            // A2 = S_B^T comb
-      chebder_warp(A2, A5, d.Nx, d.dfx, lane, d.family);   // A5 = D comb
-      chebder_warp(A5, A0, d.Nx, d.dfx, lane, d.family);   // A0 = D^2 comb
-      for (int n = lane; n < d.Nx; n += 32) A2[n] = A0[n] - k2 * A2[n];
-      __syncwarp();
-      if (a.cL != 0.0) {
-        // + cL nu (D^4 - 2 k2 D^2 + k2^2) S_B^T ua
-        for (int i = lane; i < d.nB; i += 32) A1[i] = a.u0a[(size_t)i * P + p];
+        // ---- right-hand side of Su: Mu (c0 ua + c1 ub + c2 uc) + cL Lu ua + dt N ----
+        comb_rows(A0, a.u0a, a.u0b, a.u0c, a.c0, a.c1, a.c2, d.nB, P, p, lane);
         __syncwarp();
-        apply_SBT(o, d, A1, A0, lane);           // A0 = w
-        chebder_warp(A0, A5, d.Nx, d.dfx, lane, d.family);
-        chebder_warp(A5, A1, d.Nx, d.dfx, lane, d.family);  // A1 = D^2 w
-        const double s = a.cL * d.nu;
-        for (int n = lane; n < d.Nx; n += 32)
-          A2[n] = A2[n] + s * (k2 * k2 * A0[n] - (2.0 * k2) * A1[n]);
+        apply_SBT(o, d, A0, A2, lane);            // A2 = S_B^T comb
+        chebder_warp(A2, A5, d.Nx, d.dfx, lane, d.family);   // A5 = D comb
+        chebder_warp(A5, A0, d.Nx, d.dfx, lane, d.family);   // A0 = D^2 comb
+        for (int n = lane; n < d.Nx; n += 32) A2[n] = A0[n] - k2 * A2[n];
         __syncwarp();
-        chebder_warp(A1, A5, d.Nx, d.dfx, lane, d.family);
-        chebder_warp(A5, A0, d.Nx, d.dfx, lane, d.family);  // A0 = D^4 w
-        for (int n = lane; n < d.Nx; n += 32) A2[n] = A2[n] + s * A0[n];
-        __syncwarp();
-      }
-      apply_SB_ns(o, d, A2, A0, d.Myz, lane);  // A0 = mass rows (nB)
-      rhs_rows(A3, A0, a.Nup, a.Nuq, a.d0, a.d1, a.d2, d.dt, d.nB, P, p, lane);  // rhs_u
-      __syncwarp();
-
-      // ---- right-hand side of Sg: Mg comb_g + cL Lg ga + dt N ----
-      comb_rows(A0, a.ga, a.gb, a.gc, a.c0, a.c1, a.c2, d.nD, P, p, lane);
-      __syncwarp();
-      apply_SDT(d, A0, A2, lane);  // A2 = S_D^T comb
-      if (a.cL != 0.0) {
-        for (int i = lane; i < d.nD; i += 32) A1[i] = a.ga[(size_t)i * P + p];
-        __syncwarp();
-        apply_SDT(d, A1, A0, lane);  // A0 = w
-        chebder_warp(A0, A5, d.Nx, d.dfx, lane, d.family);
-        chebder_warp(A5, A1, d.Nx, d.dfx, lane, d.family);  // A1 = D^2 w
-        const double s = a.cL * d.nu;
-        for (int n = lane; n < d.Nx; n += 32) A2[n] = A2[n] + s * (A1[n] - k2 * A0[n]);
-        __syncwarp();
-      }
-      apply_SD_ns(o, d, A2, A0, d.Myz, lane);
-      rhs_rows(A4, A0, a.Ngp, a.Ngq, a.d0, a.d1, a.d2, d.dt, d.nD, P, p, lane);  // rhs_g
-      __syncwarp();
-
-      // ---- mean flow (ky = kz = 0): M00 comb + cL L00 + dt N  -> sVW ----
-      if (mean_pencil) {
-        for (int i = lane; i < d.nD; i += 32) {
-          c64 v = a.c0 * a.vwa[i];
-          if (a.c1 != 0.0) v = v + a.c1 * a.vwb[i];
-          if (a.c2 != 0.0) v = v + a.c2 * a.vwc[i];
-          A0[i] = v;
-        }
-        __syncwarp();
-        apply_SDT(d, A0, A2, lane);
         if (a.cL != 0.0) {
-          for (int i = lane; i < d.nD; i += 32) A1[i] = a.vwa[i];
+          // + cL nu (D^4 - 2 k2 D^2 + k2^2) S_B^T ua
+          for (int i = lane; i < d.nB; i += 32) A1[i] = a.u0a[(size_t)i * P + p];
           __syncwarp();
-          apply_SDT(d, A1, A0, lane);
+          apply_SBT(o, d, A1, A0, lane);           // A0 = w
           chebder_warp(A0, A5, d.Nx, d.dfx, lane, d.family);
-          chebder_warp(A5, A1, d.Nx, d.dfx, lane, d.family);
-          for (int n = lane; n < d.Nx; n += 32) A2[n] = A2[n] + (a.cL * d.nu) * A1[n];
+          chebder_warp(A5, A1, d.Nx, d.dfx, lane, d.family);  // A1 = D^2 w
+          const double s = a.cL * d.nu;
+          for (int n = lane; n < d.Nx; n += 32)
+            A2[n] = A2[n] + s * (k2 * k2 * A0[n] - (2.0 * k2) * A1[n]);
+          __syncwarp();
+          chebder_warp(A1, A5, d.Nx, d.dfx, lane, d.family);
+          chebder_warp(A5, A0, d.Nx, d.dfx, lane, d.family);  // A0 = D^4 w
+          for (int n = lane; n < d.Nx; n += 32) A2[n] = A2[n] + s * A0[n];
           __syncwarp();
         }
-        apply_SD_ns(o, d, A2, A0, 1.0, lane);
-        for (int i = lane; i < d.nD; i += 32) {
-          c64 nl = a.d0 * sVW[i];
-          if (a.d1 != 0.0) nl = nl + a.d1 * a.NVWp[i];
-          if (a.d2 != 0.0) nl = nl + a.d2 * a.NVWq[i];
-          sVW[i] = A0[i] + d.dt * nl;
+        apply_SB_ns(o, d, A2, A0, d.Myz, lane);  // A0 = mass rows (nB)
+        rhs_rows(A3, A0, a.Nup, a.Nuq, a.d0, a.d1, a.d2, d.dt, d.nB, P, p, lane);  // rhs_u
+        __syncwarp();
+
+      } else {
+        apply_SD_ns(o, d, B1, B4, d.Myz, lane);  // Ng = Myz S_D(ns Hg)
+        if (a.Ng_out)
+          for (int i = lane; i < d.nD; i += 32) a.Ng_out[(size_t)i * P + p] = B4[i];
+
+        // ---- right-hand side of Sg: Mg comb_g + cL Lg ga + dt N ----
+        comb_rows(B0, a.ga, a.gb, a.gc, a.c0, a.c1, a.c2, d.nD, P, p, lane);
+        __syncwarp();
+        apply_SDT(d, B0, B2, lane);  // B2 = S_D^T comb
+        if (a.cL != 0.0) {
+          for (int i = lane; i < d.nD; i += 32) B1[i] = a.ga[(size_t)i * P + p];
+          __syncwarp();
+          apply_SDT(d, B1, B0, lane);  // B0 = w
+          chebder_warp(B0, B5, d.Nx, d.dfx, lane, d.family);
+          chebder_warp(B5, B1, d.Nx, d.dfx, lane, d.family);  // B1 = D^2 w
+          const double s = a.cL * d.nu;
+          for (int n = lane; n < d.Nx; n += 32) B2[n] = B2[n] + s * (B1[n] - k2 * B0[n]);
+          __syncwarp();
         }
+        apply_SD_ns(o, d, B2, B0, d.Myz, lane);
+        rhs_rows(B4, B0, a.Ngp, a.Ngq, a.d0, a.d1, a.d2, d.dt, d.nD, P, p, lane);  // rhs_g
         __syncwarp();
-      }
 
-      // ---- solves ----
-      const double* rec_u = a.fac.su + (size_t)mode_idx * a.fac.su_rec;
-      const double* rec_g = a.fac.sg + (size_t)mode_idx * a.fac.sg_rec;
-      packed_solve_warp<NR, kBlocks>(rec_u, d.nB, A3, lane);
-      packed_solve_warp<NR, kBlocks>(rec_g, d.nD, A4, lane);
-      if (mean_pencil) {
-        packed_solve_warp<NR, kBlocks>(a.fac.s00, d.nD, sVW, lane);
-        for (int i = lane; i < d.nD; i += 32) a.vw_out[i] = sVW[i];
-        __syncwarp();
-      }
-      bool bad = false;
-      for (int i = lane; i < d.nB; i += 32) {
-        bad |= !finite_c(A3[i]);
-        a.u0_out[(size_t)i * P + p] = A3[i];
-      }
-      for (int i = lane; i < d.nD; i += 32) {
-        bad |= !finite_c(A4[i]);
-        a.g_out[(size_t)i * P + p] = A4[i];
-      }
-      flag_nonfinite(a.status, bad);
+        // ---- mean flow (ky = kz = 0): M00 comb + cL L00 + dt N  -> sVW ----
+        if (mean_pencil) {
+          for (int i = lane; i < d.nD; i += 32) {
+            c64 v = a.c0 * a.vwa[i];
+            if (a.c1 != 0.0) v = v + a.c1 * a.vwb[i];
+            if (a.c2 != 0.0) v = v + a.c2 * a.vwc[i];
+            B0[i] = v;
+          }
+          __syncwarp();
+          apply_SDT(d, B0, B2, lane);
+          if (a.cL != 0.0) {
+            for (int i = lane; i < d.nD; i += 32) B1[i] = a.vwa[i];
+            __syncwarp();
+            apply_SDT(d, B1, B0, lane);
+            chebder_warp(B0, B5, d.Nx, d.dfx, lane, d.family);
+            chebder_warp(B5, B1, d.Nx, d.dfx, lane, d.family);
+            for (int n = lane; n < d.Nx; n += 32) B2[n] = B2[n] + (a.cL * d.nu) * B1[n];
+            __syncwarp();
+          }
+          apply_SD_ns(o, d, B2, B0, 1.0, lane);
+          for (int i = lane; i < d.nD; i += 32) {
+            c64 nl = a.d0 * sVW[i];
+            if (a.d1 != 0.0) nl = nl + a.d1 * a.NVWp[i];
+            if (a.d2 != 0.0) nl = nl + a.d2 * a.NVWq[i];
+            sVW[i] = B0[i] + d.dt * nl;
+          }
+          __syncwarp();
+        }
 
-      reconstruct_warp(o, d, A3, A4, sVW, mean_pencil, kyp, kzp, A0, A1, A2, A5, lane);
+      }
+    }
+    cp_async_wait_all();
+    __syncthreads();
+    // eliminations of all pencils: warp 0 the u systems, warp 1 the g systems
+    if (threadIdx.x < 64 && lane / 4 < nvalid && !nyq) {
+      const int w = lane / 4;
+      const bool u = threadIdx.x < 32;
+      c64* arr = (u ? ARR : R1) + w * 6 * d.Nx;
+      eliminate_lane(reinterpret_cast<const double*>(arr + (u ? 4 : 3) * d.Nx), u ? d.nB : d.nD,
+                     arr + (u ? 3 : 4) * d.Nx, lane & 3);
+    }
+    __syncthreads();
+    if (active) {
+      if (role == 0) {
+        inverse_product_warp<NR, kBlocks>(rec, d.nB, A3, lane);
+        bool bad = false;
+        for (int i = lane; i < d.nB; i += 32) {
+          bad |= !finite_c(A3[i]);
+          a.u0_out[(size_t)i * P + p] = A3[i];
+        }
+        flag_nonfinite(a.status, bad);
+      } else {
+        inverse_product_warp<NR, kBlocks>(rec, d.nD, B4, lane);
+        if (mean_pencil) {
+          fetch_lower(Ls, a.fac.s00, d.nD, lane);
+          cp_async_wait_all();
+          __syncwarp();
+          if (lane < 4) eliminate_lane(Ls, d.nD, sVW, lane);
+          __syncwarp();
+          inverse_product_warp<NR, kBlocks>(a.fac.s00, d.nD, sVW, lane);
+          for (int i = lane; i < d.nD; i += 32) a.vw_out[i] = sVW[i];
+          __syncwarp();
+        }
+        bool bad = false;
+        for (int i = lane; i < d.nD; i += 32) {
+          bad |= !finite_c(B4[i]);
+          a.g_out[(size_t)i * P + p] = B4[i];
+        }
+        flag_nonfinite(a.status, bad);
+      }
+      reconstruct_pair(o, d, A3, B4, sVW, mean_pencil, kyp, kzp, A0, A1, A2, A5, warp, role, lane);
     }
   } else if (active) {
     // prologue: explicit u0, u1, u2
-    for (int i = lane; i < d.nB; i += 32) A3[i] = a.pu0[(size_t)i * P + p];
-    for (int i = lane; i < d.nD; i += 32) {
-      A0[i] = a.pu1[(size_t)i * P + p];
-      A1[i] = a.pu2[(size_t)i * P + p];
+    if (role == 0) {
+      for (int i = lane; i < d.nB; i += 32) A3[i] = a.pu0[(size_t)i * P + p];
+      for (int i = lane; i < d.nD; i += 32) A0[i] = a.pu1[(size_t)i * P + p];
+      __syncwarp();
+      apply_SBT(o, d, A3, A5, lane);
+    } else {
+      for (int i = lane; i < d.nD; i += 32) A1[i] = a.pu2[(size_t)i * P + p];
     }
-    __syncwarp();
-    apply_SBT(o, d, A3, A5, lane);
+    pair_sync(warp);
   }
 
   // ---------------- phase B: u and omega in orthogonal coefficients -------
   if (active) {
     // A5 = uo0 (already); uo1 = S_D^T u1 -> A2, uo2 = S_D^T u2 -> A3
-    apply_SDT(d, A0, A2, lane);
-    apply_SDT(d, A1, A3, lane);
-    chebder_warp(A3, A4, d.Nx, d.dfx, lane, d.family);  // A4 = D uo2
-    chebder_warp(A2, A0, d.Nx, d.dfx, lane, d.family);  // A0 = D uo1
+    if (role == 0) {
+      apply_SDT(d, A0, A2, lane);
+      chebder_warp(A2, A0, d.Nx, d.dfx, lane, d.family);  // A0 = D uo1
+    } else {
+      apply_SDT(d, A1, A3, lane);
+      chebder_warp(A3, A4, d.Nx, d.dfx, lane, d.family);  // A4 = D uo2
+    }
+    pair_sync(warp);
     if (grad) {
       // gradient form: the x-derivatives of the three components
       // (channelflow_kmm.py:716-740); the y / z derivatives are wavenumber
       // weights applied on the way to the periodic transforms
-      chebder_warp(A5, A1, d.Nx, d.dfx, lane, d.family);  // A1 = D uo0
+      if (role == 0) chebder_warp(A5, A1, d.Nx, d.dfx, lane, d.family);  // A1 = D uo0
     } else {
-      for (int n = lane; n < d.Nx; n += 32) {
+      for (int n = lane + 32 * role; n < d.Nx; n += 64) {
         const c64 u0 = A5[n], u1 = A2[n], u2 = A3[n];
         A1[n] = mul_i(kyp * u2 - kzp * u1);        // omega_0
         A4[n] = mul_i(kzp * u0) - A4[n];           // omega_1
         A0[n] = A0[n] - mul_i(kyp * u0);           // omega_2
       }
     }
-    __syncwarp();
-  } else {
+  } else if (role == 0) {
     for (int n = lane; n < 6 * d.Nx; n += 32) A0[n] = cmk(0.0, 0.0);
-    __syncwarp();
   }
   __syncthreads();
   // x-backward of the six fields: field order (u0, u1, u2, w0, w1, w2) lives
