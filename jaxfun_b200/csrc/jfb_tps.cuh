@@ -53,9 +53,17 @@ __global__ void __launch_bounds__(kXThreads)
   const int64_t M = (int64_t)fw.n1 * fw.n2, m0 = (int64_t)blockIdx.x * kGW;
   const int c = tid & 15, nc = (int)min((int64_t)kGW, M - m0);
   const int KT = (cols + 3) / 4;
+  const bool wide = (reinterpret_cast<uintptr_t>(in) & 15) == 0;
   if (c < nc)
-    for (int k = tid >> 4; k < cols; k += kXThreads / 16)
-      cp_async16(sat(sm, k, c), in + (size_t)k * M + m0 + c);
+    for (int k = tid >> 4; k < cols; k += kXThreads / 16) {
+      if (wide) {
+        cp_async16(sat(sm, k, c), in + (size_t)k * M + m0 + c);
+      } else {  // a caller's field on an 8-byte boundary
+        const double* v = &in[(size_t)k * M + m0 + c].re;
+        cp_async8(sat(sm, k, c), v);
+        cp_async8(&sat(sm, k, c)->im, v + 1);
+      }
+    }
   else
     for (int k = tid >> 4; k < cols; k += kXThreads / 16) *sat(sm, k, c) = cmk(0.0, 0.0);
   for (int e = tid; e < (4 * KT - cols) * kSLd; e += kXThreads) sm[(size_t)cols * kSLd + e] = 0.0;
