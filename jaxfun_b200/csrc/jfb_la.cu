@@ -367,7 +367,7 @@ __global__ void wavenumber_solve_narrow_kernel(const __grid_constant__ StagedSol
   const int step = q.even ? 2 : 1;
   const int v = tid / step, cls = tid - v * step;
   const int m = v % q.M, r = v / q.M;
-  if (v < nv && m < mv && r < rv) {
+  if (v < nv && m < mv && r < rv && cls < n) {  // (n = 1: class 1 has no rows)
     V* x = xs + (size_t)v * q.ldx;
     const double* fm = fac + (size_t)m * q.rec;
     for (int i = cls; i < n; i += step) {
