@@ -2360,13 +2360,17 @@ static int adj_prepare(jfb_kmm_plan* pl) {
   }
   JFB_CHECK_CUDA(allow_smem((const void*)z_adjoint_kernel));
   JFB_CHECK_CUDA(allow_smem((const void*)adj_stage_kernel));
+  // the uploads run on the default stream, the kernels on the caller's
+  JFB_CHECK_CUDA(cudaStreamSynchronize(nullptr));
   pl->adj_ready = true;
   return JFB_OK;
 }
 
 // The run's buffers for T steps in segments of K (zeroed once: the Nyquist
-// rows of the spectra are never written).
-static int adj_buffers(jfb_kmm_plan* pl, int64_t K, int64_t nck) {
+// rows of the spectra are never written).  The fills run on the caller's
+// stream, in order with the run: on the default stream a fill could still be
+// queued when a run on a non-blocking stream has written its buffer.
+static int adj_buffers(jfb_kmm_plan* pl, int64_t K, int64_t nck, cudaStream_t s) {
   AdjRun& R = pl->adj;
   if (R.K == K && R.nck == nck) return JFB_OK;
   R.release();
@@ -2378,7 +2382,7 @@ static int adj_buffers(jfb_kmm_plan* pl, int64_t K, int64_t nck) {
     JFB_CHECK_CUDA(cudaMalloc((void**)p, bytes));
     R.mem.push_back(*p);
     R.bytes += bytes;
-    JFB_CHECK_CUDA(cudaMemset(*p, 0, bytes));
+    JFB_CHECK_CUDA(cudaMemsetAsync(*p, 0, bytes, s));
     return JFB_OK;
   };
   auto all = [&]() -> int {
@@ -2664,7 +2668,7 @@ extern "C" int jfb_kmm_gain_gradient(jfb_kmm_plan* pl, const jfb_kmm_state* init
   for (int k = 0; k < 4; ++k)
     z.nonlinear_old[k] = z.nonlinear_older[k] = z.solution_old[k] = z.solution_older[k] = nullptr;
   if ((st = jfb_kmm_set_state(pl, &z, stream))) return st;
-  if ((st = adj_buffers(pl, K, nck))) return st;
+  if ((st = adj_buffers(pl, K, nck, s))) return st;
   AdjRun& R = pl->adj;
   struct Keep {  // large buffers are given back at the end of the call
     AdjRun& R;
