@@ -530,6 +530,7 @@ static void add_pair(LayoutJobs& J, const void* a, const void* b, int64_t stride
   J.pair[J.np++] = PairJob{(double*)a, (double*)b, stride, vw};
 }
 static int run_layout(const LayoutJobs& J, bool to_half, cudaStream_t s) {
+  if (J.nj + J.np == 0) return JFB_OK;  // every output left out
   size_t most = 1;
   for (int k = 0; k < J.nj; ++k)
     most = std::max(most, (size_t)J.job[k].n * J.Ny * (J.Nz / 2));
