@@ -337,7 +337,8 @@ __global__ void wavenumber_solve_narrow_kernel(const __grid_constant__ StagedSol
   const int64_t f0 = (int64_t)blockIdx.x * q.M, r0 = (int64_t)blockIdx.y * q.RB;
   const int mv = (int)min((int64_t)q.M, q.n_F - f0), rv = (int)min((int64_t)q.RB, q.n_rhs - r0);
   const int warp = tid >> 5, lane = tid & 31, nw = nt >> 5;
-  // factors: one warp per (mode, diagonal), lanes over its columns
+  // factors: one warp per (mode, diagonal), lanes over its columns, all copies
+  // in flight together
   for (int u = warp; u < mv * (q.L.n + q.U.n); u += nw) {
     const int m = u / (q.L.n + q.U.n), dd = u - m * (q.L.n + q.U.n);
     const bool up = dd >= q.L.n;
@@ -345,7 +346,7 @@ __global__ void wavenumber_solve_narrow_kernel(const __grid_constant__ StagedSol
     const int s = up ? q.U.off[d] : -q.L.off[d];
     const double* src = up ? U + ((f0 + m) * q.U.n + d) * n + s : L + ((f0 + m) * q.L.n + d) * n;
     double* dst = fac + (size_t)m * q.rec + (up ? q.U.start[d] : q.L.start[d]);
-    for (int c = lane; c < n - s; c += 32) dst[c] = src[c];
+    for (int c = lane; c < n - s; c += 32) cp_async8(dst + c, src + c);
   }
   auto each = [&](auto&& fn) {  // all elements, the contiguous index fastest
     for (int e = tid; e < nv * n; e += nt) {
@@ -362,7 +363,14 @@ __global__ void wavenumber_solve_narrow_kernel(const __grid_constant__ StagedSol
       if (m < mv && r < rv) fn(staged_addr(q, (unsigned)f0 + m, r0 + r, i), (r * q.M + m) * q.ldx + i);
     }
   };
-  each([&](size_t g, int k) { xs[k] = rhs[g]; });
+  each([&](size_t g, int k) {
+    const double* v = reinterpret_cast<const double*>(rhs + g);
+    double* w = reinterpret_cast<double*>(xs + k);
+    cp_async8(w, v);
+    if constexpr (kCplx) cp_async8(w + 1, v + 1);
+  });
+  cp_async_commit();
+  cp_async_wait_all();
   __syncthreads();
   const int step = q.even ? 2 : 1;
   const int v = tid / step, cls = tid - v * step;
@@ -548,9 +556,34 @@ __global__ void wavenumber_solve_tri_kernel(const __grid_constant__ StagedSolve 
     }
 }
 
+// Whether the staged form is the faster one, `waves` being its blocks over
+// those resident at once.  A block lasts as long as its chains, so the staged
+// time is that of a chain times the waves, while the unstaged kernels keep
+// every vector in flight until memory bounds them.  Measured (complex, n
+// unknowns, F modes, r right-hand sides; unstaged -> staged, us):
+//   narrow, two classes: n = 129, F = 4096: r = 1 (0.9 waves) 179 -> 70, r = 3
+//     (1.4) 228 -> 138, r = 8 (2.8) 323 -> 230; n = 255, F = 4096, r = 8 (5.5)
+//     684 -> 782; n = 2000, F = 4096, r = 3 (28) 3736 -> 21431.  Short chains
+//     keep their lead over more waves: n = 48, F = 4096, r = 64 (9.2) 499 ->
+//     392, n = 63 (11) 638 -> 590, (25) 951 -> 1314, n = 97 (18) 1005 -> 1270.  The smallest pay
+//     only by sharing factors: n = 16, F = 64: r = 2 21 -> 25, r = 8 22 -> 18;
+//     n = 8 14 -> 19.
+//   narrow, one class (a chain twice as long): n = 129, F = 4096: r = 1 (0.7)
+//     130 -> 93, r = 2 (1.2) 134 -> 191; n = 48, F = 64, r = 2 42 -> 50, n = 63
+//     59 -> 62, n = 97 92 -> 74.
+//   wide: F = 4096: n = 97, r = 1 (2.8) 117 -> 126; n = 160 (6.9): r = 1 324 ->
+//     446, r = 2 633 -> 592; n = 255 (28): r = 2 1714 -> 2916, r = 3 2556 ->
+//     2919, r = 8 6754 -> 2648.
+static bool staged_pays(bool narrow, bool even, int n, int64_t n_rhs, double waves) {
+  if (!narrow) return n_rhs >= 4 || waves <= 2.5 * (double)(n_rhs * n_rhs);
+  if (!even) return n >= 64 && waves <= 1.0;
+  if (n < 24) return n >= 12 && n_rhs >= 8;
+  return n <= 48 || waves <= (n <= 64 ? 12.0 : 3.0);
+}
+
 // Launch of the staged solve, or false when one mode's factors and vector do
-// not fit a CTA's shared memory (or, wide, more than four rows per lane): the
-// unstaged kernels take those.
+// not fit a CTA's shared memory (or, wide, more than four rows per lane), or
+// the unstaged kernels are faster: those take it then.
 template <typename V>
 static bool staged_solve(const double* L, const OffsetTable& lt, const double* U,
                          const OffsetTable& ut, int main_idx, int n, int64_t outer, int64_t inner,
@@ -616,6 +649,10 @@ static bool staged_solve(const double* L, const OffsetTable& lt, const double* U
                              : std::max(2, vecs) * 32;
   const int64_t gx = (q.n_F + q.M - 1) / q.M, gy = (n_rhs + q.RB - 1) / q.RB;
   if (gy > 65535) return false;
+  const int64_t resident = std::min<int64_t>(
+      {228 * 1024 / (int64_t)(bytes(q.M, q.RB) + 1024), 2048 / threads, 32});
+  if (!staged_pays(narrow, q.even, n, n_rhs, (double)gx * gy / (148.0 * resident)))
+    return false;
   auto* k = wavenumber_solve_narrow_kernel<V>;
   switch (10 * S + R) {
 #define JFB_TRI(SS, RR) \
