@@ -249,8 +249,12 @@ int jfb_kmm_timed_steps(jfb_kmm_plan* plan, int64_t steps, void* flush_buf,
  * grad->u0, u1, u2, g (full-spectrum reference layout; the Hermitian
  * representative) and zeros to any history pointers given.  The gradient is
  * the hand-written discrete adjoint of the FP64 step (transposed transforms,
- * transposed banded solves, linearised rotational product) over a reverse
- * sweep that recomputes `checkpoint` steps at a time from stored states.
+ * x-operators and solves, linearised rotational product) over a reverse sweep
+ * that recomputes `checkpoint` steps at a time from stored states.  A segment
+ * keeps the six x-physical fields of each of its steps, 96 nx ny nz / 2 bytes a
+ * step (longer ones are cut at 8 GiB).  The plan keeps the sweep's buffers for the
+ * next gradient while they are at most 4 GiB (counted in jfb_kmm_info's
+ * device_bytes); without grad none are needed.
  * FP64 flow plans only.  The plan's loaded state is consumed. */
 int jfb_kmm_gain_gradient(jfb_kmm_plan* plan, const jfb_kmm_state* init, int64_t steps,
                           int64_t checkpoint, double* gain_out, const jfb_kmm_state* grad,

@@ -219,8 +219,9 @@ struct AdjOps {
   double *F = nullptr, *GB = nullptr, *GD = nullptr;
 };
 
-// Device buffers of a gain-gradient run (kept by the plan while they are at
-// most kAdjKeep bytes, so that an ascent's repeated calls do not allocate).
+// Device buffers of a gradient's reverse sweep (kept by the plan while they are
+// at most kAdjKeep bytes, so that an ascent's repeated calls do not allocate; a
+// run for the gain alone needs none of them).
 constexpr size_t kAdjKeep = (size_t)4 << 30;
 struct AdjRun {
   struct Mu {
@@ -228,7 +229,7 @@ struct AdjRun {
   };
   std::vector<void*> mem;
   size_t bytes = 0;
-  int64_t K = 0, nck = 0;
+  int64_t K = 0, nck = 0;  // capacity: states of a segment, checkpoints
   c64 *YF, *AH, *AW, *HZ6, *AX, *EU[3];
   Mu M[4], Q[2][3], S;      // steady ring, the startup stages' solutions, an adjoint state
   c64* TX = nullptr;        // x-physical fields of the segment's states, K slots
@@ -236,7 +237,6 @@ struct AdjRun {
   c64* X0;                  // and of the explicit initial velocity
   c64 *IU0, *IU1, *IU2;     // explicit initial leaves
   std::vector<c64*> ck;     // checkpoints: rings + HX
-  double* dev8 = nullptr;
   void release() {
     for (void* p : mem) cudaFree(p);
     mem.clear();
@@ -307,6 +307,7 @@ struct jfb_kmm_plan {
   double* mdiag_partial = nullptr;
   // adjoint: operators and kept factor bands, built on first use
   bool adj_ready = false;
+  double* energies = nullptr;  // diagnostics of the state a run is at
   jfb::AdjOps aops;
   jfb::AdjRun adj;
   size_t smem_za = 0;
@@ -1784,7 +1785,7 @@ extern "C" int jfb_kmm_get_info(const jfb_kmm_plan* pl, jfb_kmm_info* info) {
   JFB_REQUIRE(pl && info, "null pointer");
   const Dims& d = pl->d;
   info->n_pencils = d.P;
-  info->device_bytes = pl->device_bytes;
+  info->device_bytes = pl->device_bytes + (int64_t)pl->adj.bytes;
   info->launches_per_step = (pl->mhd ? 5 : pl->plane ? 2 : 4) + (pl->gemm && pl->split ? 1 : 0);
   // stage model: 43 E_s + 18 E_m complex values, E_s = Nx Ny (Nz/2+1), E_m = Nx My (Nz/2+1)
   const int64_t H = d.Nz / 2 + 1;
@@ -2354,6 +2355,7 @@ static int adj_prepare(jfb_kmm_plan* pl) {
   if ((st = upload(pl, &A.F, gh.F))) return st;
   if ((st = upload(pl, &A.GB, gh.GB))) return st;
   if ((st = upload(pl, &A.GD, gh.GD))) return st;
+  if ((st = dalloc(pl, (void**)&pl->energies, 10 * sizeof(double)))) return st;
   pl->smem_za = (size_t)2 * d.Mz * kZRows * 5 * sizeof(c64);
   if (pl->smem_za > 227 * 1024) {
     set_error("grid too large for the adjoint z stage");
@@ -2367,13 +2369,14 @@ static int adj_prepare(jfb_kmm_plan* pl) {
   return JFB_OK;
 }
 
-// The run's buffers for T steps in segments of K (zeroed once: the Nyquist
-// rows of the spectra are never written).  The fills run on the caller's
-// stream, in order with the run: on the default stream a fill could still be
-// queued when a run on a non-blocking stream has written its buffer.
+// The sweep's buffers for segments of K steps and nck checkpoints, kept ones
+// where they are enough (zeroed once: the Nyquist rows of the spectra are never
+// written).  The fills run on the caller's stream, in order with the run: on the
+// default stream a fill could still be queued when a run on a non-blocking
+// stream has written its buffer.
 static int adj_buffers(jfb_kmm_plan* pl, int64_t K, int64_t nck, cudaStream_t s) {
   AdjRun& R = pl->adj;
-  if (R.K == K && R.nck == nck) return JFB_OK;
+  if (R.K >= K && R.nck >= nck) return JFB_OK;
   R.release();
   const Dims& d = pl->d;
   const size_t P = d.P, nBP = (size_t)d.nB * P, nDP = (size_t)d.nD * P;
@@ -2416,9 +2419,6 @@ static int adj_buffers(jfb_kmm_plan* pl, int64_t K, int64_t nck, cudaStream_t s)
     AL(R.IU2, nDP);
     R.ck.assign(nck, nullptr);
     for (auto& c : R.ck) AL(c, checkpoint_elems(pl));
-    c64* dv;
-    AL(dv, 5);
-    R.dev8 = (double*)dv;
 #undef AL
     return JFB_OK;
   };
@@ -2594,10 +2594,10 @@ static int adj_energy(jfb_kmm_plan* pl, AdjRun& R, const c64* u0, const c64* u1,
   return JFB_OK;
 }
 
-static int perturbation_energy(jfb_kmm_plan* pl, double* dev8, cudaStream_t s, double* out) {
-  int st = jfb_kmm_diagnostics(pl, dev8, s);
+static int perturbation_energy(jfb_kmm_plan* pl, cudaStream_t s, double* out) {
+  int st = jfb_kmm_diagnostics(pl, pl->energies, s);
   if (st) return st;
-  JFB_CHECK_CUDA(cudaMemcpyAsync(out, dev8, sizeof(double), cudaMemcpyDeviceToHost, s));
+  JFB_CHECK_CUDA(cudaMemcpyAsync(out, pl->energies, sizeof(double), cudaMemcpyDeviceToHost, s));
   JFB_CHECK_CUDA(cudaStreamSynchronize(s));
   return JFB_OK;
 }
@@ -2669,7 +2669,8 @@ extern "C" int jfb_kmm_gain_gradient(jfb_kmm_plan* pl, const jfb_kmm_state* init
   for (int k = 0; k < 4; ++k)
     z.nonlinear_old[k] = z.nonlinear_older[k] = z.solution_old[k] = z.solution_older[k] = nullptr;
   if ((st = jfb_kmm_set_state(pl, &z, stream))) return st;
-  if ((st = adj_buffers(pl, K, nck, s))) return st;
+  // (the last segment starts from no checkpoint: it is recorded on the way)
+  if (grad && (st = adj_buffers(pl, K, nck - 1, s))) return st;
   AdjRun& R = pl->adj;
   struct Keep {  // large buffers are given back at the end of the call
     AdjRun& R;
@@ -2677,17 +2678,19 @@ extern "C" int jfb_kmm_gain_gradient(jfb_kmm_plan* pl, const jfb_kmm_state* init
       if (R.bytes > kAdjKeep) R.release();
     }
   } keep{R};
-  double* dev8 = R.dev8;
 
   // explicit initial leaves and E(0)
-  JFB_CHECK_CUDA(cudaMemcpyAsync(R.IU0, pl->U0[slot(0)], nBP * sizeof(c64), cudaMemcpyDeviceToDevice, s));
-  JFB_CHECK_CUDA(cudaMemcpyAsync(R.IU1, pl->U1S, nDP * sizeof(c64), cudaMemcpyDeviceToDevice, s));
-  JFB_CHECK_CUDA(cudaMemcpyAsync(R.IU2, pl->U2S, nDP * sizeof(c64), cudaMemcpyDeviceToDevice, s));
+  if (grad) {
+    JFB_CHECK_CUDA(cudaMemcpyAsync(R.IU0, pl->U0[slot(0)], nBP * sizeof(c64), cudaMemcpyDeviceToDevice, s));
+    JFB_CHECK_CUDA(cudaMemcpyAsync(R.IU1, pl->U1S, nDP * sizeof(c64), cudaMemcpyDeviceToDevice, s));
+    JFB_CHECK_CUDA(cudaMemcpyAsync(R.IU2, pl->U2S, nDP * sizeof(c64), cudaMemcpyDeviceToDevice, s));
+  }
   double E0 = 0.0, ET = 0.0;
-  if ((st = perturbation_energy(pl, dev8, s, &E0))) return st;
+  if ((st = perturbation_energy(pl, s, &E0))) return st;
   JFB_REQUIRE(std::isfinite(E0) && E0 > 0.0, "initial energy must be positive");
   if ((st = ensure_H(pl, s))) return st;
-  JFB_CHECK_CUDA(cudaMemcpyAsync(R.X0, pl->X, 6 * f * sizeof(c64), cudaMemcpyDeviceToDevice, s));
+  if (grad)
+    JFB_CHECK_CUDA(cudaMemcpyAsync(R.X0, pl->X, 6 * f * sizeof(c64), cudaMemcpyDeviceToDevice, s));
 
   // forward sweep with checkpoints; the last segment's fields are recorded on
   // the way, so that it is not recomputed
@@ -2707,7 +2710,7 @@ extern "C" int jfb_kmm_gain_gradient(jfb_kmm_plan* pl, const jfb_kmm_state* init
     if ((st = grad && m >= a_last ? step_recorded(m, a_last) : forward_step(pl, s, nullptr)))
       return st;
   }
-  if ((st = perturbation_energy(pl, dev8, s, &ET))) return st;
+  if ((st = perturbation_energy(pl, s, &ET))) return st;
   const double gain = ET / E0;
   *gain_out = gain;
   if (!grad) return JFB_OK;
