@@ -360,7 +360,7 @@ class KMM:
         """Time every kernel variant this plan accepts on copies of ``state``
         (default: the loaded state), select the fastest and return
         ``{"variant": ..., "ms_per_step": ...}``.  With ``cache`` the choice
-        is remembered per (device, grid, precision) in the file named by
+        is remembered per (device, grid, form, library build) in the file named by
         JFB200_AUTOTUNE_CACHE (default ~/.cache/jaxfun_b200/autotune.json)
         and reused without timing."""
         from . import autotune as at
