@@ -510,6 +510,8 @@ __global__ void __launch_bounds__(kSThreads, 2)
       }
     }
   } else if (mean_cta) {
+    // mean_flow's named barrier counts kMeanThreads threads
+    static_assert(kSThreads - 4 * kGW == kMeanThreads);
     mean_flow(d, o, G, a, mean, m_nvw, m_vw, m_x, tid - 4 * kGW);
   }
   __syncthreads();
