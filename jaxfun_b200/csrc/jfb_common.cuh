@@ -118,6 +118,13 @@ __device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
+// x / d from r = 1 / d: the product corrected by its residual (Markstein, IBM J.
+// Res. Dev. 34, 1990), for finite results.
+__device__ __forceinline__ double quotient(double x, double d, double r) {
+  const double p = x * r;
+  return fma(fma(-p, d, x), r, p);
+}
+
 // Phase stamps (off by default; built into libjfb200_stamps.so by
 // jaxfun_b200.build with stamps=True): thread 0 of every CTA writes the
 // global timer at the phase boundaries of the step kernels into

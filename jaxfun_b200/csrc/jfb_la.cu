@@ -293,13 +293,17 @@ __global__ void wavenumber_solve_warp_kernel(const double* __restrict__ L, Offse
 //                   unknowns in registers, lane = row of a class; U (and L,
 //                   when it has more than kTriFewL diagonals) as packed dense
 //                   triangles, so a column update is one shared-memory read
-//                   and one multiply-add per row.  y_c stays in place and is
-//                   scaled by 1 / U[c, c] on output.  Up to four right-hand
-//                   sides share a warp and its factor reads.  Bound by issue.
+//                   and one multiply-add per row.  A column of U is divided by
+//                   U[c, c] as it is read, off the chain of the y_c, and x_c =
+//                   y_c / U[c, c] on output: the roundings of a division per
+//                   column (products with 1 / U[c, c] have one more, 6 % more
+//                   error).
+//                   Up to four right-hand sides share a warp and its factor
+//                   reads.  Bound by issue.
 //   narrow factors  (wavenumber_solve_narrow_kernel) a thread per vector and
 //                   class, rows in order, vectors in shared memory.
 // n_P = 63, 4096 modes, three complex right-hand sides (one class of 32 and
-// one of 31 rows): 76 us.  A warp per system reading strided vectors and the
+// one of 31 rows): 80 us.  A warp per system reading strided vectors and the
 // factors once per right-hand side took 201 us; with the vectors in shared
 // memory instead of registers 279 us (two read-modify-writes of 16 bytes per
 // lane and column); one right-hand side per warp 84 us.
@@ -471,9 +475,11 @@ __global__ void wavenumber_solve_tri_kernel(const __grid_constant__ StagedSolve 
   }
   asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
   __syncthreads();
+  // reciprocal diagonals in the triangles' own diagonal entries
   for (int e = tid; e < mv * n; e += nt) {
-    double* dg = fac + (size_t)(e / n) * q.rec + q.oD + e % n;
-    *dg = 1.0 / *dg;
+    double* Fm = fac + (size_t)(e / n) * q.rec;
+    const int i = e % n, c = i >> sh;
+    Fm[(sh && (i & 1) ? tri1 : 0) + c * (c + 1) / 2 + c] = 1.0 / Fm[q.oD + i];
   }
   __syncthreads();
   if (!live) return;  // no barrier below
@@ -530,16 +536,17 @@ __global__ void wavenumber_solve_tri_kernel(const __grid_constant__ StagedSolve 
     for (int cl = 0; cl < 2; ++cl) {
       if (c >= mc[cl]) continue;
       const double* T = F + (cl ? tri1 : 0) + c * (c + 1) / 2;
-      const double rd = F[q.oD + (c << sh) + cl];
+      const double dg = F[q.oD + (c << sh) + cl], rd = T[c];
       double u[S];
 #pragma unroll
-      for (int s = 0; s < S; ++s) u[s] = lane + 32 * s < c ? T[lane + 32 * s] : 0.0;
+      for (int s = 0; s < S; ++s)
+        u[s] = lane + 32 * s < c ? quotient(T[lane + 32 * s], dg, rd) : 0.0;
 #pragma unroll
       for (int k = 0; k < R; ++k) {
-        const V xc = rd * bcast(y[k][cl], c);
+        const V yc = bcast(y[k][cl], c);
 #pragma unroll
         for (int s = 0; s < S; ++s)
-          if (lane + 32 * s < c) y[k][cl][s] = y[k][cl][s] - u[s] * xc;
+          if (lane + 32 * s < c) y[k][cl][s] = y[k][cl][s] - u[s] * yc;
       }
     }
   }
@@ -549,10 +556,21 @@ __global__ void wavenumber_solve_tri_kernel(const __grid_constant__ StagedSolve 
     for (int s = 0; s < S; ++s) {
       const int i = ((lane + 32 * s) << sh) + cl;
       if (cl >= ncls || i >= n) continue;
-      const double rd = F[q.oD + i];
+      const int c = lane + 32 * s;
+      const double dg = F[q.oD + i], rd = F[(cl ? tri1 : 0) + c * (c + 1) / 2 + c];
 #pragma unroll
-      for (int k = 0; k < R; ++k)
-        if (k < rv) out[staged_addr(q, (unsigned)f0 + m, rw + k, i)] = rd * y[k][cl][s];
+      for (int k = 0; k < R; ++k) {
+        if (k >= rv) continue;
+        // (infinities and NaN: the product alone)
+        auto result = [&](double v) {
+          const double x = quotient(v, dg, rd);
+          return isfinite(x) ? x : v * rd;
+        };
+        V x = y[k][cl][s];
+        if constexpr (kCplx) x = cmk(result(x.re), result(x.im));
+        else x = result(x);
+        out[staged_addr(q, (unsigned)f0 + m, rw + k, i)] = x;
+      }
     }
 }
 
@@ -571,11 +589,14 @@ __global__ void wavenumber_solve_tri_kernel(const __grid_constant__ StagedSolve 
 //   narrow, one class (a chain twice as long): n = 129, F = 4096: r = 1 (0.7)
 //     130 -> 93, r = 2 (1.2) 134 -> 191; n = 48, F = 64, r = 2 42 -> 50, n = 63
 //     59 -> 62, n = 97 92 -> 74.
-//   wide: F = 4096: n = 97, r = 1 (2.8) 117 -> 126; n = 160 (6.9): r = 1 324 ->
-//     446, r = 2 633 -> 592; n = 255 (28): r = 2 1714 -> 2916, r = 3 2556 ->
-//     2919, r = 8 6754 -> 2648.
+//   wide, F = 4096: n = 129, r = 1 (4.6) 210 -> 312, r = 3 600 -> 432; n = 255
+//     (28): r = 1 866 -> 2441, r = 3 2556 -> 2919, r = 8 6754 -> 2648.  With a
+//     smooth field's coefficients, whose smallest underflow, the unstaged
+//     divisions take their slow path: n = 95, r = 1 (2.8) 173 -> 130, n = 127
+//     (4.6) 275 -> 235, against 111 and 200 for random numbers.
 static bool staged_pays(bool narrow, bool even, int n, int64_t n_rhs, double waves) {
-  if (!narrow) return n_rhs >= 4 || waves <= 2.5 * (double)(n_rhs * n_rhs);
+  const int rows = even ? (n + 1) / 2 : n;  // of a class
+  if (!narrow) return n_rhs >= 4 || waves <= (rows <= 64 ? 8.0 : 2.5) * n_rhs;
   if (!even) return n >= 64 && waves <= 1.0;
   if (n < 24) return n >= 12 && n_rhs >= 8;
   return n <= 48 || waves <= (n <= 64 ? 12.0 : 3.0);
