@@ -220,7 +220,9 @@ def _fused_sum(tpmats: Sequence[TPMatrix], u: torch.Tensor) -> torch.Tensor | No
     n = u.shape[poly]
     cplx = u.is_complex()
     diags_total = sum(len(tp.mats[poly].offsets) for tp in tpmats)
-    if diags_total > 512 or n > 4096 or n * 17 * (16 if cplx else 8) > 200 * 1024:
+    modes = u.numel() // n
+    if (diags_total > 512 or n > 4096 or n * 17 * (16 if cplx else 8) > 200 * 1024
+            or modes > 2**31 - 1):
         return None
     fourier = [a for a in range(nd) if a != poly]
     x = u.to(torch.complex128 if cplx else torch.float64).contiguous()
