@@ -224,6 +224,12 @@ def _fused_sum(tpmats: Sequence[TPMatrix], u: torch.Tensor) -> torch.Tensor | No
     if (diags_total > 512 or n > 4096 or n * 17 * (16 if cplx else 8) > 200 * 1024
             or modes > 2**31 - 1):
         return None
+    # Long dense operators on few modes: too few blocks read the operators, each
+    # all of them.  257 rows, 129 diagonals, 4096 modes: one term 157 us by
+    # factors, 219 us fused (129 rows, 65 diagonals: 61 and 65; three terms 197
+    # and 181); at 16384 modes 129 rows take 194 and 134.
+    if n * diags_total > 16000 * len(tpmats) and modes <= 8192:
+        return None
     fourier = [a for a in range(nd) if a != poly]
     x = u.to(torch.complex128 if cplx else torch.float64).contiguous()
     y = torch.empty_like(x)

@@ -14,6 +14,8 @@ def _dia(n, offsets):
 
 @pytest.mark.parametrize("shape, diagonals, terms", [
     ((3, 1 << 16, 1 << 16), 2, 1),     # more modes than a 32-bit index holds
+    ((257, 64, 64), 129, 1),           # long dense operators on few modes
+    ((64, 257, 64), 129, 3),
     ((800, 4, 4), 3, 1),               # a column block beyond shared memory
 ])
 def test_left_to_the_general_path(shape, diagonals, terms):
