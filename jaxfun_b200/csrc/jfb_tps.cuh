@@ -43,8 +43,9 @@ __device__ __forceinline__ c64 ipow_times(c64 w, int idx, int n, int k, double d
 // periodic axes).  A block stages 16 columns of the field as B-operand rows
 // (swizzled as in gemm_sw) and its warps take the row tiles of A: the field is
 // read once, where one thread per output read every column once per row from
-// L2 (23 -> 7 us for 65 x 63 on 4096 columns).  Bound by memory.
-constexpr int kXThreads = 256;
+// L2 (23 -> 7 us for 65 x 63 on 4096 columns).  Bound by latency: load, product
+// and store of a block follow one another.
+constexpr int kXThreads = 256;  // at most: a warp per row tile
 __global__ void __launch_bounds__(kXThreads)
     x_apply_kernel(const double* __restrict__ frag, int rows, int cols, const c64* __restrict__ in,
                    c64* __restrict__ out, const __grid_constant__ FourierWeight fw) {
@@ -55,7 +56,7 @@ __global__ void __launch_bounds__(kXThreads)
   const int KT = (cols + 3) / 4;
   const bool wide = (reinterpret_cast<uintptr_t>(in) & 15) == 0;
   if (c < nc)
-    for (int k = tid >> 4; k < cols; k += kXThreads / 16) {
+    for (int k = tid >> 4; k < cols; k += blockDim.x / 16) {
       if (wide) {
         cp_async16(sat(sm, k, c), in + (size_t)k * M + m0 + c);
       } else {  // a caller's field on an 8-byte boundary
@@ -65,8 +66,8 @@ __global__ void __launch_bounds__(kXThreads)
       }
     }
   else
-    for (int k = tid >> 4; k < cols; k += kXThreads / 16) *sat(sm, k, c) = cmk(0.0, 0.0);
-  for (int e = tid; e < (4 * KT - cols) * kSLd; e += kXThreads) sm[(size_t)cols * kSLd + e] = 0.0;
+    for (int k = tid >> 4; k < cols; k += blockDim.x / 16) *sat(sm, k, c) = cmk(0.0, 0.0);
+  for (int e = tid; e < (4 * KT - cols) * kSLd; e += blockDim.x) sm[(size_t)cols * kSLd + e] = 0.0;
   cp_async_commit();
   cp_async_wait_all();
   __syncthreads();
@@ -76,13 +77,13 @@ __global__ void __launch_bounds__(kXThreads)
   for (int nt = 0; nt < 4; ++nt) {
     const int64_t m = m0 + nt * 4 + t4;
     w[nt] = cmk(fw.scale, 0.0);
-    if (m < M) {
-      w[nt] = ipow_times(w[nt], (int)(m / fw.n2), fw.n1, fw.k1, fw.df1);
-      w[nt] = ipow_times(w[nt], (int)(m % fw.n2), fw.n2, fw.k2, fw.df2);
+    if (m < M && fw.k1 + fw.k2) {
+      w[nt] = ipow_times(w[nt], (int)m / fw.n2, fw.n1, fw.k1, fw.df1);
+      w[nt] = ipow_times(w[nt], (int)m % fw.n2, fw.n2, fw.k2, fw.df2);
     }
   }
-  for (int mt = warp + blockIdx.y * (kXThreads / 32); mt * 8 < rows;
-       mt += gridDim.y * (kXThreads / 32)) {
+  for (int mt = warp + blockIdx.y * (blockDim.x / 32); mt * 8 < rows;
+       mt += gridDim.y * (blockDim.x / 32)) {
     double acc[4][2];
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt) acc[nt][0] = acc[nt][1] = 0.0;
@@ -523,7 +524,9 @@ static int tps_x(const double* A, int rows, int cols, const c64* in, c64* out,
   // few columns (2-D spaces): the row tiles over several blocks
   const unsigned gx = (unsigned)((M + kGW - 1) / kGW);
   const unsigned gy = gx >= 148 ? 1 : std::min<unsigned>(148 / gx + 1, (rows + 63) / 64);
-  x_apply_kernel<<<dim3(gx, gy), kXThreads, (size_t)(cols + 3) / 4 * 4 * kSLd * sizeof(double), s>>>(
+  // few rows: fewer warps a block, so that more blocks load at once
+  const int threads = std::min(kXThreads, 32 * std::max(2, (rows + 7) / 8));
+  x_apply_kernel<<<dim3(gx, gy), threads, (size_t)(cols + 3) / 4 * 4 * kSLd * sizeof(double), s>>>(
       A, rows, cols, in, out, fw);
   JFB_CHECK_LAUNCH();
   return JFB_OK;
