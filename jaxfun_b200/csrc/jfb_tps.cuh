@@ -230,6 +230,7 @@ struct Helm2DArgs {
   int nL, nU, umain;
   int l2, l4;  // indices of the L offsets -2 / -4 (-1: absent) when those are all of L
   int loff[kHelmMaxDiag], uoff[kHelmMaxDiag];
+  int staged;  // general form: the mode's factors in shared memory, rows of nb | 1
   int N, nb, M;
   double scale;  // Fourier scalar-product weight / fourier_mass
   const c64* f;
@@ -245,18 +246,36 @@ __global__ void __launch_bounds__(kHelmThreads)
   c64* x = F + N;                             // nb: right-hand side, then y
   c64* z = x + nb;                            // nb: solution
   c64* part = z + nb;                         // kHelmThreads: partial sums
-  double* l2s = reinterpret_cast<double*>(part + kHelmThreads);  // nb: L[r, r-2], L[r, r-4]
+  // nb each: L[r, r-2], L[r, r-4], or U[r, r] and its reciprocal
+  double* l2s = reinterpret_cast<double*>(part + kHelmThreads);
   double* l4s = l2s + nb;
   const double* Lk = h.L + (size_t)k * h.nL * nb;
   const double* Uk = h.U + (size_t)k * h.nU * nb;
   const bool fast = h.Uinv && h.l2 + h.l4 > -2;
   const int row = tid & (kHelmRows - 1), grp = tid / kHelmRows;
   for (int n = tid; n < N; n += kHelmThreads) F[n] = h.f[(size_t)n * M + k];
-  if (fast)
-    for (int r = tid; r < nb; r += kHelmThreads) {
+  for (int r = tid; r < nb; r += kHelmThreads) {
+    if (fast) {
       l2s[r] = (h.l2 >= 0 && r >= 2) ? __ldg(Lk + (size_t)h.l2 * nb + r - 2) : 0.0;
       l4s[r] = (h.l4 >= 0 && r >= 4) ? __ldg(Lk + (size_t)h.l4 * nb + r - 4) : 0.0;
+    } else {
+      l2s[r] = __ldg(Uk + (size_t)h.umain * nb + r);
+      l4s[r] = 1.0 / l2s[r];
     }
+  }
+  __shared__ int offs[2 * kHelmMaxDiag];
+  double *Ls = l4s + nb, *Us = Ls + (size_t)h.nL * (nb | 1);
+  if (!fast)
+    for (int d = tid; d < h.nL + h.nU; d += kHelmThreads)
+      offs[d] = d < h.nL ? h.loff[d] : h.uoff[d - h.nL];
+  if (h.staged) {
+    for (int e = tid; e < (h.nL + h.nU) * nb; e += kHelmThreads) {
+      const int d = e / nb, c = e - d * nb;
+      cp_async8(Ls + (size_t)d * (nb | 1) + c, d < h.nL ? Lk + e : Uk + e - h.nL * nb);
+    }
+    cp_async_commit();
+    cp_async_wait_all();
+  }
   // the matrix entries of the two products do not depend on f: on their way
   // while the right-hand side and the recurrence run
   const double* Ui = h.Uinv + (size_t)k * nb * nb + row;
@@ -308,22 +327,30 @@ __global__ void __launch_bounds__(kHelmThreads)
     if (tid < nb) z[tid] = total(tid);
   } else if (tid < 32) {
     // column-oriented substitution: once x_c is final each lane applies its
-    // diagonals' entries of column c to their rows (distinct per diagonal)
+    // diagonals' entries of column c to their rows (distinct per diagonal), from
+    // shared memory (a lane's diagonals are lines apart in memory, and argument
+    // words indexed by lane are read one by one).
+    // Called without explicit inverses, 62 / 98 / 148 unknowns on 64 / 16 / 16
+    // modes: 62 / 112 / 191 -> 36 / 58 / 91 us.
+    const int ld = h.staged ? nb | 1 : nb;
+    const double *Lf = h.staged ? Ls : Lk, *Uf = h.staged ? Us : Uk;
     for (int c = 0; c < nb; ++c) {
       const c64 y = x[c];
       for (int d = lane; d < h.nL; d += 32) {
-        const int r = c - h.loff[d];
-        if (r < nb) x[r] = x[r] - __ldg(Lk + (size_t)d * nb + c) * y;
+        const int r = c - offs[d];
+        if (r < nb) x[r] = x[r] - Lf[(size_t)d * ld + c] * y;
       }
       __syncwarp();
     }
     for (int c = nb - 1; c >= 0; --c) {
-      const double dg = __ldg(Uk + (size_t)h.umain * nb + c);
-      const c64 v = x[c], xc = cmk(v.re / dg, v.im / dg);
+      const double dg = l2s[c], rd = l4s[c];
+      const c64 y = x[c];
+      c64 xc = cmk(quotient(y.re, dg, rd), quotient(y.im, dg, rd));
+      if (!finite_c(xc)) xc = cmk(y.re / dg, y.im / dg);
       if (lane == 0) z[c] = xc;
       for (int d = lane; d < h.nU; d += 32) {
-        const int sft = h.uoff[d], r = c - sft;
-        if (sft > 0 && r >= 0) x[r] = x[r] - __ldg(Uk + (size_t)d * nb + c) * xc;
+        const int sft = offs[h.nL + d], r = c - sft;
+        if (sft > 0 && r >= 0) x[r] = x[r] - Uf[(size_t)d * ld + c] * xc;
       }
       __syncwarp();
     }
@@ -813,8 +840,12 @@ extern "C" int jfb_helmholtz2d_solve(const jfb_tps* tc, const jfb_tps* td, const
   h.f = (const c64*)f_hat;
   h.u = (c64*)u;
   cudaStream_t cs = (cudaStream_t)stream;
-  helmholtz2d_kernel<<<M, kHelmThreads,
-                       (size_t)(N + 2 * nb + kHelmThreads) * sizeof(c64) + (size_t)2 * nb * sizeof(double), cs>>>(h);
+  size_t sm = (size_t)(N + 2 * nb + kHelmThreads) * sizeof(c64) + (size_t)2 * nb * sizeof(double);
+  const size_t factors = (size_t)(h.nL + h.nU) * (nb | 1) * sizeof(double);
+  h.staged = !(U_inv && h.l2 + h.l4 > -2) && sm + factors <= 200 * 1024;
+  if (h.staged) sm += factors;
+  if (sm > 48 * 1024) JFB_CHECK_CUDA(allow_smem((const void*)helmholtz2d_kernel));
+  helmholtz2d_kernel<<<M, kHelmThreads, sm, cs>>>(h);
   JFB_CHECK_LAUNCH();
   // y: inverse transform of the rows, in place
   return tps_lines(td->f1n, td->tw1n, +1, N, M, M, h.u, h.u, cs);
