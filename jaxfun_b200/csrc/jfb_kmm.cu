@@ -619,8 +619,8 @@ static int launch_implicit(jfb_kmm_plan* pl, const StageArgs& a, cudaStream_t s)
   if (pl->split) {
     const Dims& d = pl->d;
     const size_t sr = split_rhs_smem(d.Nx, d.nB, d.nD, g.slin != 0.0);
-    JFB_CHECK_CUDA(launch_ex(pl->pdl, d.grad ? pencil_rhs_kernel<1> : pencil_rhs_kernel<0>,
-                             dim3(blocks), dim3(kSThreads), sr, s, d, pl->ops, pl->gops, g));
+    JFB_CHECK_CUDA(launch_ex(pl->pdl, pencil_rhs_kernel, dim3(blocks), dim3(kSThreads), sr, s, d,
+                             pl->ops, pl->gops, g));
     JFB_CHECK_CUDA(launch_ex(pl->pdl, d.grad ? pencil_velocity_kernel<1> : pencil_velocity_kernel<0>,
                              dim3(blocks), dim3(kSThreads), split_vel_smem(d.nB, d.nD), s, d,
                              pl->gops, g));
@@ -1552,8 +1552,7 @@ static int create_plan(const jfb_kmm_config* cfg, const jfb_mhd_params* mhd,
       G.kt_mg_lin[0] = ceil_div(nDe, 4);
       G.kt_mg_lin[1] = ceil_div(nDo, 4);
       pl->smem_gemm = smem;
-      for (const void* fn : {(const void*)pencil_rhs_kernel<0>, (const void*)pencil_rhs_kernel<1>,
-                             (const void*)pencil_velocity_kernel<0>,
+      for (const void* fn : {(const void*)pencil_rhs_kernel, (const void*)pencil_velocity_kernel<0>,
                              (const void*)pencil_velocity_kernel<1>})
         JFB_CHECK_CUDA(allow_smem(fn));
       JFB_CHECK_CUDA(allow_smem((const void*)pencil_gemm_kernel<false, 0>));
@@ -2443,8 +2442,7 @@ static PTermList tlist(c64* dst, int rows, bool acc) {
 }
 
 static void term(PTermList& L, const c64* src, const double* mat, int src_rows, int trans,
-                 double cre, double cim, int a = 0, int b = 0, int c = 0, int sel = 0,
-                 int realpart = 0) {
+                 double cre, double cim, int a = 0, int b = 0, int c = 0) {
   if (cre == 0.0 && cim == 0.0) return;
   PTerm& T = L.t[L.n++];
   T.src = src;
@@ -2456,8 +2454,6 @@ static void term(PTermList& L, const c64* src, const double* mat, int src_rows, 
   T.a = a;
   T.b = b;
   T.c = c;
-  T.sel = sel;
-  T.realpart = realpart;
 }
 
 static int run(jfb_kmm_plan* pl, const PTermList& L, cudaStream_t s) {

@@ -41,8 +41,6 @@ struct PTerm {
   int trans;
   double cre, cim;
   int a, b, c;
-  int sel;       // 0: every pencil, 1: all but the mean pencil, 2: the mean pencil only
-  int realpart;  // keep the real part of the term
 };
 
 constexpr int kMaxTerms = 8;
@@ -76,7 +74,6 @@ __global__ void __launch_bounds__(256) pencil_terms_kernel(Dims d, PTermList L) 
     const bool mean = (p == 0);
     for (int t = 0; t < L.n; ++t) {
       const PTerm& T = L.t[t];
-      if ((T.sel == 1 && mean) || (T.sel == 2 && !mean)) continue;
       double s = 1.0;
       for (int e = 0; e < T.a; ++e) s *= ky;
       for (int e = 0; e < T.b; ++e) s *= kz;
@@ -112,7 +109,6 @@ __global__ void __launch_bounds__(256) pencil_terms_kernel(Dims d, PTermList L) 
       const c64 cf = cmk(T.cre * s, T.cim * s);
 #pragma unroll
       for (int q = 0; q < kTermRows; ++q) {
-        if (T.realpart) v[q].im = 0.0;
         acc[q] = acc[q] + cf * v[q];
       }
     }
@@ -199,7 +195,7 @@ __global__ void __launch_bounds__(kSThreads, 1)
   const int nKc = (d.Kz + 7) / 8, bid = blockIdx.x;
   const int kyi = bid / nKc, kz0 = (bid % nKc) * 8;
   const int nkz = min(8, d.Kz - kz0);
-  const int N = d.Nx, Jh = G.Jh, Jl = G.Jl, nB = d.nB, nD = d.nD;
+  const int N = d.Nx, Jh = G.Jh, nB = d.nB, nD = d.nD;
   const size_t P = (size_t)d.P;
   const double* __restrict__ frag = G.frag;
   const bool mean_cta = bid == 0;

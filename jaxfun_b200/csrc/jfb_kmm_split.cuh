@@ -30,10 +30,12 @@
 // differ by up to 1e-7 (seen at 129x128x128 in one of four seeds), so a stage
 // that sums in another order would not reproduce the form's results.
 //
-// Measured (steady SBDF3 stage, both kernels together): 97x96x96 372 -> 131
-// us.  At 129x128x128  Bounds, per CTA at Nx = 129: the
-// inverse factors from memory (35 of 121 us; 300 MB per stage), Nu and Ng on
-// the FP64 tensor pipe (24 us), the level and history rows (15 us).
+// Measured (steady SBDF3 stage, both kernels together, events around the
+// launches): 97x96x96 434 -> 138 us, 129x128x128 1033 -> 331 us against the warp
+// stage with one warp per pencil.  What a CTA spends its time on at 129x128x128:
+// of 118 us in pencil_rhs_kernel the inverse factors from memory 36 (300 MB per
+// stage), Nu and Ng on the FP64 tensor pipe 25, the level and history rows 15, the
+// mass products 11; of 48 in pencil_velocity_kernel the products and stores 40.
 #pragma once
 
 #include "jfb_kmm_gemm.cuh"
@@ -181,11 +183,9 @@ __device__ __forceinline__ void tile_columns(const Dims& d, int kyi, int kz0, Ti
   }
 }
 
-template <int kForm>
 __global__ void __launch_bounds__(kSThreads, 2)
     pencil_rhs_kernel(const __grid_constant__ Dims d, const __grid_constant__ DevOps o,
                       const __grid_constant__ GemmOps G, const __grid_constant__ GemmStageArgs a) {
-  constexpr bool grad = kForm == 1;
   extern __shared__ __align__(128) double sm[];
   __shared__ TileCols tc;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(kSThreads, 2)
   const int kyi = bid / nKc, kz0 = (bid % nKc) * 8;
   const int nkz = min(8, d.Kz - kz0);
   const bool mean_cta = bid == 0;
-  const int N = d.Nx, Jh = G.Jh, Jl = G.Jl, nB = d.nB, nD = d.nD;
+  const int N = d.Nx, Jh = G.Jh, nB = d.nB, nD = d.nD;
   const size_t P = (size_t)d.P;
   const double* __restrict__ frag = G.frag + (size_t)(bid % G.nrep) * G.nfrag;
   const double sl = a.slin;
@@ -221,9 +221,7 @@ __global__ void __launch_bounds__(kSThreads, 2)
   if (col_ok)
     for (int r = hw; r < 3 * N; r += kSThreads / 16) {
       const int f = r >= 2 * N ? 2 : r >= N ? 1 : 0;
-      c64* dst = sat(sm, f * hb + r - f * N, hc);
-      if (a.x32) cp_async8(dst, reinterpret_cast<const c32*>(a.HX) + (size_t)r * P + so);
-      else cp_async16(dst, a.HX + (size_t)r * P + so);
+      cp_async16(sat(sm, f * hb + r - f * N, hc), a.HX + (size_t)r * P + so);
     }
   cp_async_commit();
   // history and level rows of this tile into L2 while H arrives (each row is
@@ -251,34 +249,11 @@ __global__ void __launch_bounds__(kSThreads, 2)
   for (int idx = tid; idx < Jh * kGW; idx += kSThreads) {
     const int j = idx / kGW, w = idx % kGW, jm = N - 1 - j, p = tc.p[w];
     const bool ok = p >= 0;
-    c32 xl[2][4];
-    if (a.Xlin && ok) {
-      const int fs[4] = {0, grad ? 6 : 1, grad ? 7 : 3, grad ? 8 : 5};
-#pragma unroll
-      for (int s = 0; s < 2; ++s)
-#pragma unroll
-        for (int k = 0; k < 4; ++k) xl[s][k] = a.Xlin[((size_t)fs[k] * N + (s ? jm : j)) * P + p];
-    }
     c64 h[2][3];
-    auto value = [&](int row) {
-      const c64* q = sat(sm, row, w);
-      if (!a.x32) return *q;
-      const c32 v = *reinterpret_cast<const c32*>(q);
-      return cmk((double)v.re, (double)v.im);
-    };
 #pragma unroll
     for (int f = 0; f < 3; ++f) {
-      h[0][f] = ok ? value(f * hb + j) : cmk(0.0, 0.0);
-      h[1][f] = (ok && jm != j) ? value(f * hb + jm) : cmk(0.0, 0.0);
-    }
-    if (a.Xlin && ok) {
-      if (grad) {
-        add_base_convection_terms(xl[0], d.uwall * o.xphys[j], d.uwall, h[0]);
-        if (jm != j) add_base_convection_terms(xl[1], d.uwall * o.xphys[jm], d.uwall, h[1]);
-      } else {
-        add_base_flow_terms(xl[0], p == 0, d.uwall * o.xphys[j], d.uwall, h[0]);
-        if (jm != j) add_base_flow_terms(xl[1], p == 0, d.uwall * o.xphys[jm], d.uwall, h[1]);
-      }
+      h[0][f] = ok ? *sat(sm, f * hb + j, w) : cmk(0.0, 0.0);
+      h[1][f] = (ok && jm != j) ? *sat(sm, f * hb + jm, w) : cmk(0.0, 0.0);
     }
     if (mean_cta && w == 0) {
       mean[j] = h[0][1].re;
@@ -600,16 +575,9 @@ __global__ void __launch_bounds__(kSThreads, 2)
     auto cv = [&](const double (&v)[2][2], int nt) { return cmk(v[nt][0], v[nt][1]); };
     auto put = [&](int q, int p, const c64 fe, const c64 fo) {
       const c64 vp = fe + fo, vm = fe - fo;
-      const size_t e = (size_t)q * N * P + p;
-      if (a.x32) {
-        c32* X = reinterpret_cast<c32*>(a.X) + e;
-        X[(size_t)j * P] = cmk((float)vp.re, (float)vp.im);
-        X[(size_t)jm * P] = cmk((float)vm.re, (float)vm.im);
-      } else {
-        c64* X = a.X + e;
-        X[(size_t)j * P] = vp;
-        X[(size_t)jm * P] = vm;
-      }
+      c64* X = a.X + (size_t)q * N * P + p;
+      X[(size_t)j * P] = vp;
+      X[(size_t)jm * P] = vm;
     };
     // even (E) and odd (O) halves of A0 u0, P1 u0, B1 g, then P2 u0, B2 g
     double aE[2][2], aO[2][2], vE[2][2], vO[2][2], wE[2][2], wO[2][2];

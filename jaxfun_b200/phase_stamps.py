@@ -1,4 +1,4 @@
-"""Phase split of the two step kernels from the phase-stamp build.
+"""Phase split of the step kernels from the phase-stamp build.
 
 Usage (profiling only; needs ``libjfb200_stamps.so``, built by
 ``python -m jaxfun_b200.build --stamps``)::
@@ -8,10 +8,11 @@ Usage (profiling only; needs ``libjfb200_stamps.so``, built by
 
 Runs the benchmark workload (seeded Couette perturbation, Re 1000, dt 0.01)
 for a few steps, then one steady step after a 256 MiB L2 flush, and prints
-per-phase durations of ``pencil_gemm_kernel`` (kernel 0) and
-``plane_cross_kernel`` (kernel 1): the median over CTAs of each interval
-between consecutive stamps, and the median CTA's total.  Phase names follow
-the stamp points in the kernels (jfb_kmm_gemm.cuh, jfb_kmm_warpk.cuh).
+per-phase durations of the stamped kernels that ran (``pencil_gemm_kernel``
+and ``plane_cross_kernel``, or above Nx = 65 in FP64 ``pencil_rhs_kernel`` and
+``pencil_velocity_kernel``): the median over CTAs of each interval between
+consecutive stamps, and the median CTA's total.  Phase names follow the stamp
+points in the kernels (jfb_kmm_gemm.cuh, jfb_kmm_warpk.cuh, jfb_kmm_split.cuh).
 """
 
 from __future__ import annotations
@@ -26,6 +27,11 @@ PENCIL = ("launch+prologue", "staging", "mirror+mass inputs", "B products", "C1 
           "C2 U^-1 products", "C3 stores+wait", "D velocity", "middle node")
 PLANE = ("launch+wait", "y staging", "y inverse FFT", "z stage", "y forward FFT",
          "stores", "cluster exit")
+RHS = ("H staging", "mirror sums", "Nu, Ng products", "mass inputs", "mass products",
+       "right-hand sides + multipliers", "elimination + mean flow", "U^-1 products", "stores")
+VELOCITY = ("staging", "products + stores", "middle node")
+KERNELS = (("pencil_gemm", PENCIL), ("plane_cross", PLANE), ("pencil_rhs", RHS),
+           ("pencil_velocity", VELOCITY))
 
 
 def main(argv=None) -> int:
@@ -55,21 +61,21 @@ def main(argv=None) -> int:
     flush = torch.empty(256 << 20, dtype=torch.uint8, device=dev)
     n_cta, n_ph = 1024, 16
     out = {"grid": list(grid), "precision": a.precision, "unit": "us"}
-    runs = {0: [], 1: []}
+    runs = [[] for _ in KERNELS]
     for _ in range(a.repeats):
         flush.fill_(1)
         g.advance_resident(1)
         torch.cuda.synchronize(dev)
         buf = (ctypes.c_ulonglong * (4 * n_cta * n_ph))()
         _lib.check(lib.jfb_debug_read_stamps(buf, 4 * n_cta * n_ph))
-        for k, nph in ((0, len(PENCIL) + 1), (1, len(PLANE) + 1)):
-            ctas = []
+        for k, (_, names) in enumerate(KERNELS):
+            nph, ctas = len(names) + 1, []
             for c in range(n_cta):
                 st = [buf[(k * n_cta + c) * n_ph + i] for i in range(nph)]
                 if all(st) and all(st[i + 1] >= st[i] for i in range(nph - 1)):
                     ctas.append(st)
             runs[k].append(ctas)
-    for k, names in ((0, PENCIL), (1, PLANE)):
+    for k, (kernel, names) in enumerate(KERNELS):
         last = runs[k][-1]
         if not last:
             continue
@@ -94,7 +100,7 @@ def main(argv=None) -> int:
                 rec["tc_subphases_median_cta"] = {
                     n: statistics.median((c[i + 1] - c[i]) / 1e3 for c in sub)
                     for i, n in enumerate(names)}
-        out["pencil_gemm" if k == 0 else "plane_cross"] = rec
+        out[kernel] = rec
     print(json.dumps(out))
     return 0
 
