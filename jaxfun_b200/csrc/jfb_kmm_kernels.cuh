@@ -663,10 +663,11 @@ __device__ __forceinline__ void cta_forward_dmma(const double* __restrict__ QE,
 // a second warp per pencil shortens the chains and fills their gaps.  With the
 // recurrences of all pencils on one lane per value (masses: 12 lanes a pencil,
 // eliminations: 4 a system), the per-row tables in shared memory and the
-// inverse read at constant offsets, the mixed 129x128x128 stage went from 972
-// to 700 us and the 65x64x64 prologue from 32 to 27 us, every sum in the order
-// it had (the mixed form's FP64 -> FP32 roundings depend on it).  What is left:
-// the inverse's 520 KB a block from L2 (28 of 107 us), the x products (22).
+// inverse read at constant offsets, the mixed 129x128x128 stage went from 1124
+// to 808 us, the 97x96x96 one from 458 to 320 (events around the launch) and the
+// 65x64x64 prologue from 32 to 27 us, every sum in the order it had (the mixed
+// form's FP64 -> FP32 roundings depend on it).  What is left: the inverse's 520
+// KB a block from L2 (a quarter of a block's time), the x products (a fifth).
 // ---------------------------------------------------------------------------
 // kForm: 0 rotational, 1 gradient (each compiled without the other's code);
 // kBlocks: the layout of the factor records (inv_entry; a runtime flag cost 10 %).

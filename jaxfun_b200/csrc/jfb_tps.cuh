@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(256) fft_rows_warp_kernel(const c64* __restric
 // quarter of a row (9.4 us with a thread per row and no loads ahead).
 // ---------------------------------------------------------------------------
 constexpr int kHelmMaxDiag = 256;
-constexpr int kHelmCTAs = 8;  // of the size range (jfb_helmholtz2d_solve)
+constexpr int kHelmCTAs = 8;  // parts of the size range's formula (jfb_helmholtz2d_solve)
 constexpr int kHelmRows = 128, kHelmSplit = 4;  // thread = (row, every 4th column)
 constexpr int kHelmThreads = kHelmRows * kHelmSplit;
 constexpr int kHelmCols = 16;  // matrix entries a thread loads ahead
@@ -784,7 +784,9 @@ extern "C" int jfb_helmholtz2d_solve(const jfb_tps* tc, const jfb_tps* td, const
               "too many diagonals");
   const int N = td->N, nb = td->nb, M = td->n1;
   const int KC = (M + kHelmCTAs - 1) / kHelmCTAs, JR = (N + kHelmCTAs - 1) / kHelmCTAs;
-  // the size range of this call: problems that fit one cluster's shared memory
+  // the size range of this call, unchanged since the solve was one cluster's: 2 N c
+  // + N q + 2 n1 ceil(N/8) complex values and the x operator in one CTA's shared
+  // memory.  What it refuses goes through the separate launches.
   const int QS = KC + ((5 - KC % 4) % 4);
   const size_t smem = ((size_t)2 * N * KC + (size_t)N * QS + (size_t)2 * M * JR) * sizeof(c64) +
                       (size_t)nb * N * sizeof(double);
