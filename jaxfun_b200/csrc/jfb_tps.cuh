@@ -846,7 +846,8 @@ extern "C" int jfb_helmholtz2d_solve(const jfb_tps* tc, const jfb_tps* td, const
   const size_t factors = (size_t)(h.nL + h.nU) * (nb | 1) * sizeof(double);
   h.staged = !(U_inv && h.l2 + h.l4 > -2) && sm + factors <= 200 * 1024;
   if (h.staged) sm += factors;
-  if (sm > 48 * 1024) JFB_CHECK_CUDA(allow_smem((const void*)helmholtz2d_kernel));
+  // (the kernel holds 2 KB besides)
+  if (sm > 46 * 1024) JFB_CHECK_CUDA(allow_smem((const void*)helmholtz2d_kernel));
   helmholtz2d_kernel<<<M, kHelmThreads, sm, cs>>>(h);
   JFB_CHECK_LAUNCH();
   // y: inverse transform of the rows, in place

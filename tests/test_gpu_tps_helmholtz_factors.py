@@ -17,6 +17,7 @@ pytestmark = pytest.mark.gpu
     ((16, 8), (-3, -1), (0, 1, 2, 5)),
     ((40, 6), (-4, -2), tuple(range(0, 38, 2))),
     ((67, 12), (-2,), tuple(range(40))),       # several diagonals per lane
+    ((100, 8), (-2,), tuple(range(42))),       # 47 KB with the kernel's own 2 KB: over 48
     ((131, 4), (-6, -4, -2), (0, 2, 128)),
     ((160, 2), (-1,), tuple(range(158))),      # 201 KB of factors: read from memory
 ])
