@@ -506,7 +506,8 @@ extern "C" int jfb_tps_create(const jfb_tps_config* cfg, jfb_tps** out) {
   if (allow_smem((const void*)y_backward_kernel<double>) != cudaSuccess ||
       allow_smem((const void*)y_forward_kernel<double>) != cudaSuccess ||
       allow_smem((const void*)fft_rows_kernel) != cudaSuccess ||
-      allow_smem((const void*)x_apply_kernel) != cudaSuccess) {
+      allow_smem((const void*)x_apply_kernel) != cudaSuccess ||
+      cudaStreamSynchronize(nullptr) != cudaSuccess) {  // the uploads have arrived
     set_error("cannot configure the transform kernels");
     return fail(JFB_ERR_CUDA);
   }
@@ -528,6 +529,8 @@ static int tps_xmap(jfb_tps* t, int map, int k, const double** A, int* rows, int
     double* d = nullptr;
     JFB_CHECK_CUDA(cudaMalloc((void**)&d, h.size() * sizeof(double)));
     cudaError_t e = cudaMemcpy(d, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice);
+    // (a copy from pageable memory may return before it has arrived)
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
     if (e != cudaSuccess) {
       cudaFree(d);
       JFB_CHECK_CUDA(e);
